@@ -1,5 +1,4 @@
 // Sampling kernels: greedy argmax, temperature + top-k / top-p / min-p sampling, grammar bitmask, penalties.
-// One CTA (1024 threads) per batch row; the row stays L2-resident across passes (V = 128 K -> 256 KB bf16).
 //
 // Reference counterparts: python/sglang/srt/layers/sampler.py:98-320 (softmax + FlashInfer
 // top_k_top_p_sampling_from_probs / min_p), kernels/aot/csrc/grammar/apply_token_bitmask_inplace_cuda.cu:157,
@@ -23,18 +22,6 @@ __device__ __forceinline__ float block_reduce_max(float v, float* red) {
   r = warp_max(r);
   r = __shfl_sync(0xffffffffu, r, 0);
   // broadcast from warp 0 to everyone
-  __syncthreads();
-  if (threadIdx.x == 0) red[0] = r;
-  __syncthreads();
-  return red[0];
-}
-__device__ __forceinline__ float block_reduce_sum(float v, float* red) {
-  v = warp_sum(v);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float r = (threadIdx.x < (blockDim.x >> 5)) ? red[threadIdx.x] : 0.f;
-  r = warp_sum(r);
   __syncthreads();
   if (threadIdx.x == 0) red[0] = r;
   __syncthreads();
@@ -70,166 +57,485 @@ struct SampleParams {
   int V, stride;
 };
 
-template <typename T>
-__global__ void __launch_bounds__(SAMP_THREADS) sample_kernel(const T* __restrict__ logits, SampleParams p) {
-  __shared__ float red[32];
-  __shared__ float s_chunk[SAMP_THREADS];
-  __shared__ int s_arg;
-  __shared__ int h_cnt[SAMP_BINS];
-  __shared__ float h_mass[SAMP_BINS];
-  __shared__ int s_bin;
-  __shared__ float s_bc, s_bm;
-  const int row = blockIdx.x;
-  const T* lr = logits + (size_t)row * p.stride;
+// ---------------------------------------------------------------- the sampler: a cluster of eight CTAs per row
+// A row (V = 128 K: 256 KB of bf16) does not fit one SM's shared memory and one SM reads it slowly, so eight CTAs take an eighth each, keep it in
+// shared memory for every later pass, and exchange block results (maximum, sums, histogram segments) through distributed shared memory.  Every
+// thread reads only what it staged itself, 8 consecutive logits at a time, so the passes need no barrier between them.
+//
+// top-k / top-p: two-level histogram over d = (max - logit) / T (r = p / p_max = e^-d): 2048 bins of width 1/64 cover r down to e^-32, a second
+// 2048 bins refine the one that holds the boundary (7.6e-6 in d).  Shared-memory atomics are native for integers only (a float add is a
+// compare-and-swap loop that collapses on the popular bins of a broad tail), so both levels count integers: elements, or r over the bin's largest r
+// in fixed point.  The fixed-point mass only nominates a bin; the masses before and inside it are then summed in fp32 and the nomination is moved
+// until they enclose the target.  Elements beyond d = 32 (masked ones, cold temperatures) meet in the last bin and are added up in registers.
+//
+// Measured (B200, bf16, rows asking in turn for greedy / nucleus / top-k / min-p / plain): 121 x 128256 2594 -> 69 us, 1 x 128256 (greedy) 11 us; the
+// version before kept one CTA per row, scalar loads and float atomics.
+constexpr int SAMP_CL = 8;              // CTAs per row: a portable cluster
+constexpr int SAMP_SEG = SAMP_BINS / SAMP_CL;
+
+__device__ __forceinline__ uint32_t cl_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cl_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cl_map(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cl_st(const void* p, uint32_t rank, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cl_map(p, rank)), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t cl_ld(const void* p, uint32_t rank) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cl_map(p, rank)) : "memory");
+  return v;
+}
+
+template <int NW>
+struct SampShared {
+  uint32_t slot[2][2][SAMP_CL];         // [parity][value][rank]: block results of a reduction
+  uint32_t wred[2][NW];
+  uint32_t hist[SAMP_BINS];
+  float seg_total[SAMP_CL], scan[SAMP_SEG / 32];
+  int hit;
+  uint32_t cand_bin[SAMP_CL], cand_before[SAMP_CL];
+  uint32_t kept[SAMP_CL * NW];          // kept mass of every warp of the row
+  int pick;
+  float pick_run, pick_u;
+};
+
+__device__ __forceinline__ void samp_load8(const __nv_bfloat16* p, float (&v)[8]) {
+  const U4 a = ld128(p);
+  v[0] = bf16_lo(a.x); v[1] = bf16_hi(a.x); v[2] = bf16_lo(a.y); v[3] = bf16_hi(a.y);
+  v[4] = bf16_lo(a.z); v[5] = bf16_hi(a.z); v[6] = bf16_lo(a.w); v[7] = bf16_hi(a.w);
+}
+__device__ __forceinline__ void samp_load8(const float* p, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+// STAGED: the CTA's slice fits shared memory (V up to ~800 K bf16 / 400 K fp32); otherwise every pass reads the row again
+template <typename T, int NT, bool STAGED>
+__global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT) sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
+  constexpr int NW = NT / 32;
+  extern __shared__ __align__(16) uint8_t samp_dyn[];
+  __shared__ SampShared<NW> sh;
+  const int rank = (int)cl_rank(), row = blockIdx.x / SAMP_CL;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int V = p.V;
-  const int tid = threadIdx.x;
-  const int topk = p.top_k[row];
-  // ---- pass 1: max (+ argmax)
-  float mx = -INFINITY; int am = 0x7fffffff;
-  for (int i = tid; i < V; i += SAMP_THREADS) {
-    const float v = to_f<T>(lr[i]);
-    if (v > mx) { mx = v; am = i; }
-  }
-  const float gmax = block_reduce_max(mx, red);
-  if (tid == 0) s_arg = 0x7fffffff;
-  __syncthreads();
-  if (mx == gmax) atomicMin(&s_arg, am);   // smallest index among ties (matches torch.argmax)
-  __syncthreads();
-  const int arg = s_arg;
-  const float temp = fmaxf(p.temperature[row], 1e-6f);
-  const float inv_t = 1.f / temp;
-  // ---- pass 2: partition function at temperature
-  float z = 0.f;
-  for (int i = tid; i < V; i += SAMP_THREADS) z += __expf((to_f<T>(lr[i]) - gmax) * inv_t);
-  const float Z = block_reduce_sum(z, red);
-  int token = arg;
-  if (topk != 1) {
-    const float top_p = p.top_p[row];
-    const float min_p = p.min_p[row];
-    // threshold in "relative probability" space r = p / p_max in (0, 1]; keep {r >= thr}
-    float thr = min_p;   // min-p: p >= min_p * p_max
-    const bool need_k = topk > 0 && topk < V;
-    const bool need_p = top_p < 1.f;
-    // Threshold search by a two-level histogram over d = (max - logit) / T  (r = e^-d): 2048 bins of width 1/64 cover r down to e^-32, a
-    // second 2048-bin histogram refines the one bin that holds the boundary (resolution 7.6e-6 in d).  5 passes over the row instead of
-    // the 2 x 24 bisection passes of the first version (882 us at 256 x 128 K, profiles/microbench_r1.md).
-    float d_max = INFINITY;              // keep { d <= d_max }
-    float base_mass = Z;
-    auto fill_hist = [&](float d_lo, float inv_w, float d_cap) {
-      for (int i = tid; i < SAMP_BINS; i += SAMP_THREADS) { h_cnt[i] = 0; h_mass[i] = 0.f; }
-      __syncthreads();
-      for (int i = tid; i < V; i += SAMP_THREADS) {
-        const float d = (gmax - to_f<T>(lr[i])) * inv_t;
-        if (d >= d_lo && d <= d_cap) {
-          const int b = min(SAMP_BINS - 1, (int)((d - d_lo) * inv_w));
-          atomicAdd(&h_cnt[b], 1);
-          atomicAdd(&h_mass[b], __expf(-d));
-        }
-      }
-      __syncthreads();
-    };
-    // first bin index whose inclusive prefix reaches the target (count or mass); also returns the exclusive prefix before that bin
-    auto find_bin = [&](bool by_count, float target, float& before_cnt, float& before_mass) -> int {
-      // serial scan by one warp over 2048 bins (64 per lane) — 2048 smem reads, negligible next to a pass over V
-      if (tid < 32) {
-        float c = 0.f, m = 0.f;
-        for (int i = tid * (SAMP_BINS / 32); i < (tid + 1) * (SAMP_BINS / 32); ++i) { c += (float)h_cnt[i]; m += h_mass[i]; }
-        float pc = c, pm = m;            // inclusive scan across lanes
+  const T* lr = logits + (size_t)row * p.stride;
+  const int slice = rank * NW * per_warp;                              // first logit of this CTA
+  const int w0 = slice + warp * per_warp, w1 = min(w0 + per_warp, V);  // this warp's contiguous range
+  T* stage = reinterpret_cast<T*>(samp_dyn);
+  const bool vec = (reinterpret_cast<uintptr_t>(lr) & 15) == 0;
+
+  auto get8 = [&](int i, float (&v)[8]) {                              // 8 logits from i; those beyond the row are NaN (every comparison fails)
+    if (STAGED) { samp_load8(stage + (i - slice), v); return; }
+    if (vec && i + 8 <= V) { samp_load8(lr + i, v); return; }
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const float tc = __shfl_up_sync(0xffffffffu, pc, o), tm = __shfl_up_sync(0xffffffffu, pm, o);
-          if (tid >= o) { pc += tc; pm += tm; }
-        }
-        const float ec = pc - c, em = pm - m;          // exclusive prefix of this lane's segment
-        const bool mine = by_count ? (ec <= target && pc >= target) : (em <= target && pm >= target);      // lowest such lane wins below
-        const unsigned ball = __ballot_sync(0xffffffffu, mine);
-        if (ball == 0) {
-          if (tid == 31) { s_bin = SAMP_BINS; s_bc = pc; s_bm = pm; }      // target beyond the histogram: keep everything in range
-        } else if (tid == __ffs(ball) - 1) {
-          float rc = ec, rm = em;
-          int b = tid * (SAMP_BINS / 32);
-          for (;; ++b) {
-            const float nc = rc + (float)h_cnt[b], nm = rm + h_mass[b];
-            if ((by_count ? nc : nm) >= target) break;
-            rc = nc; rm = nm;
-          }
-          s_bin = b; s_bc = rc; s_bm = rm;
-        }
-      }
-      __syncthreads();
-      before_cnt = s_bc; before_mass = s_bm;
-      const int b = s_bin;
-      __syncthreads();
-      return b;
-    };
-    constexpr float W1 = 1.f / 64.f;                   // level-1 bin width (2048 bins -> d in [0, 32))
-    if (need_k || need_p) {
-      fill_hist(0.f, 1.f / W1, INFINITY);
-      float bc, bm;
-      if (need_k) {
-        const int b1 = find_bin(true, (float)topk, bc, bm);
-        if (b1 < SAMP_BINS) {
-          const float lo1 = b1 * W1;
-          float c_before = bc, m_before = bm;
-          fill_hist(lo1, (float)SAMP_BINS / W1, (b1 == SAMP_BINS - 1) ? INFINITY : lo1 + W1);
-          const int b2 = find_bin(true, (float)topk - c_before, bc, bm);
-          d_max = (b2 >= SAMP_BINS - 1 && b1 == SAMP_BINS - 1) ? INFINITY : lo1 + (float)(min(b2, SAMP_BINS - 1) + 1) * (W1 / SAMP_BINS);
-          base_mass = m_before + bm + ((b2 < SAMP_BINS) ? h_mass[min(b2, SAMP_BINS - 1)] : 0.f);
-          __syncthreads();
-          if (need_p) fill_hist(0.f, 1.f / W1, d_max);          // level-1 again, restricted to the top-k set
-        }
-      }
-      if (need_p) {
-        const float target = top_p * base_mass;
-        const int b1 = find_bin(false, target, bc, bm);
-        if (b1 < SAMP_BINS) {
-          const float lo1 = b1 * W1, m_before = bm;
-          fill_hist(lo1, (float)SAMP_BINS / W1, fminf(d_max, (b1 == SAMP_BINS - 1) ? INFINITY : lo1 + W1));
-          const int b2 = find_bin(false, target - m_before, bc, bm);
-          if (!(b2 >= SAMP_BINS - 1 && b1 == SAMP_BINS - 1)) d_max = fminf(d_max, lo1 + (float)(min(b2, SAMP_BINS - 1) + 1) * (W1 / SAMP_BINS));
-        }
-      }
-    }
-    if (d_max < INFINITY) thr = fmaxf(thr, __expf(-d_max));
-    // ---- pass 3: kept mass per contiguous chunk, block scan, pick
-    const int chunk = (V + SAMP_THREADS - 1) / SAMP_THREADS;
-    const int c0 = tid * chunk, c1 = min(V, c0 + chunk);
-    float cm = 0.f;
-    for (int i = c0; i < c1; ++i) {
-      const float r = __expf((to_f<T>(lr[i]) - gmax) * inv_t);
-      if (r >= thr) cm += r;
-    }
-    s_chunk[tid] = cm;
-    const float total = block_reduce_sum(cm, red);
-    // a seeded request draws from (its seed, ITS OWN output position): the stream does not depend on which step / row / batch the scheduler
-    // happened to put it in (the first version mixed the global step counter in, so seeded output changed with scheduling)
-    const bool own = p.seeds && p.seeds[2 * row + 1] >= 0;
-    const long long step = p.step_ptr ? *p.step_ptr : p.step;
-    const float u = (own ? rng_uniform((unsigned long long)p.seeds[2 * row], 0ull, (unsigned long long)p.seeds[2 * row + 1])
-                         : rng_uniform(p.global_seed, (unsigned long long)row, (unsigned long long)step)) * total;
-    if (tid == 0) {
-      float run = 0.f; int pick = SAMP_THREADS - 1;
-      for (int t = 0; t < SAMP_THREADS; ++t) {
-        if (run + s_chunk[t] > u) { pick = t; break; }
-        run += s_chunk[t];
-      }
-      // walk inside the chunk
-      int tok = arg;
-      const int a0 = pick * chunk, a1 = min(V, a0 + chunk);
-      for (int i = a0; i < a1; ++i) {
-        const float r = __expf((to_f<T>(lr[i]) - gmax) * inv_t);
-        if (r >= thr) { run += r; tok = i; if (run > u) break; }
-      }
-      s_arg = tok;
-    }
+    for (int j = 0; j < 8; ++j) v[j] = i + j < V ? to_f<T>(lr[i + j]) : __int_as_float(0x7fffffff);
+  };
+  int par = 0;
+  auto reduce2 = [&](float& a, float& b) {                             // sums over the row, the same bits in every thread
+    a = warp_sum(a); b = warp_sum(b);
+    if (lane == 0) { sh.wred[0][warp] = __float_as_uint(a); sh.wred[1][warp] = __float_as_uint(b); }
     __syncthreads();
-    token = s_arg;
+    if (warp == 0) {
+      a = warp_sum(lane < NW ? __uint_as_float(sh.wred[0][lane]) : 0.f);
+      b = warp_sum(lane < NW ? __uint_as_float(sh.wred[1][lane]) : 0.f);
+      if (lane < SAMP_CL) { cl_st(&sh.slot[par][0][rank], lane, __float_as_uint(a)); cl_st(&sh.slot[par][1][rank], lane, __float_as_uint(b)); }
+    }
+    cl_sync();
+    a = b = 0.f;
+#pragma unroll
+    for (int r = 0; r < SAMP_CL; ++r) { a += __uint_as_float(sh.slot[par][0][r]); b += __uint_as_float(sh.slot[par][1][r]); }
+    par ^= 1;                                                          // (the next writers of this half have passed the next barrier)
+  };
+
+  // ---- stage the slice, maximum and its lowest index (torch.argmax)
+  float mx = -INFINITY;
+  int am = 0x7fffffff;
+  if (STAGED) {
+    if (vec) {
+#pragma unroll 4
+      for (int i = w0 + lane * 8; i < w1; i += 256) {
+        T* dst = stage + (i - slice);
+        if (i + 8 <= V) {
+#pragma unroll
+          for (int k = 0; k < (int)sizeof(T) / 2; ++k) st128(dst + k * (16 / sizeof(T)), ldg128(lr + i + k * (16 / sizeof(T))));
+        } else {
+          for (int j = 0; j < 8; ++j) dst[j] = i + j < V ? lr[i + j] : T(__int_as_float(0x7fffffff));
+        }
+      }
+    } else {
+#pragma unroll 2
+      for (int i = w0 + lane * 8; i < w1; i += 256) {
+        T* dst = stage + (i - slice);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) dst[j] = i + j < V ? lr[i + j] : T(__int_as_float(0x7fffffff));
+      }
+    }
   }
-  if (tid == 0) {
+  for (int i = w0 + lane * 8; i < w1; i += 256) {
+    float v[8];
+    get8(i, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (v[j] > mx) { mx = v[j]; am = i + j; }
+  }
+  const float own_max = mx;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, mx, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, am, o);
+    if (ov > mx || (ov == mx && oi < am)) { mx = ov; am = oi; }
+  }
+  if (lane == 0) { sh.wred[0][warp] = __float_as_uint(mx); sh.wred[1][warp] = (uint32_t)am; }
+  __syncthreads();
+  if (warp == 0) {
+    mx = lane < NW ? __uint_as_float(sh.wred[0][lane]) : -INFINITY;
+    am = lane < NW ? (int)sh.wred[1][lane] : 0x7fffffff;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, mx, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, am, o);
+      if (ov > mx || (ov == mx && oi < am)) { mx = ov; am = oi; }
+    }
+    if (lane < SAMP_CL) { cl_st(&sh.slot[par][0][rank], lane, __float_as_uint(mx)); cl_st(&sh.slot[par][1][rank], lane, (uint32_t)am); }
+  }
+  cl_sync();
+  float gmax = -INFINITY;
+  int arg = 0x7fffffff;
+#pragma unroll
+  for (int r = 0; r < SAMP_CL; ++r) {                                  // ranks in index order: a strict comparison keeps the lowest index
+    const float ov = __uint_as_float(sh.slot[par][0][r]);
+    if (ov > gmax) { gmax = ov; arg = (int)sh.slot[par][1][r]; }
+  }
+  if (arg == 0x7fffffff) arg = 0;                                      // a row without a finite logit
+  par ^= 1;
+
+  const float inv_t = 1.f / fmaxf(p.temperature[row], 1e-6f);
+  const int topk = p.top_k[row];
+  const bool greedy = topk == 1;
+  const float top_p = p.top_p[row];
+  const bool need_k = topk > 0 && topk < V, need_p = top_p < 1.f;
+
+  // f(logit's d, its index offset) over this thread's valid logits
+  auto each = [&](auto&& f) {
+#pragma unroll 2
+    for (int i = w0 + lane * 8; i < w1; i += 256) {
+      float v[8];
+      get8(i, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f((gmax - v[j]) * inv_t);
+    }
+  };
+  float Z = 0.f;
+  if (p.out_logprobs || (!greedy && need_p && !need_k)) {
+    float z = 0.f, unused = 0.f;
+    for (int i = w0 + lane * 8; i < w1; i += 256) {
+      float v[8];
+      get8(i, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (i + j < V) z += __expf((v[j] - gmax) * inv_t);
+    }
+    reduce2(z, unused);
+    Z = z;
+  }
+  auto finish = [&](int token) {
     p.out_tokens[row] = token;
     if (p.next_token_buf && p.out_slots) p.next_token_buf[p.out_slots[row]] = token;
     if (p.out_logprobs) p.out_logprobs[row] = (to_f<T>(lr[token]) - gmax) * inv_t - __logf(Z);
+  };
+  if (greedy) {
+    if (rank == 0 && tid == 0) finish(arg);
+    return;                            // (nobody reads this CTA's shared memory after the barrier above)
   }
+
+  // ---- threshold in d: keep { d <= d_max }
+  constexpr float W1 = 1.f / 64.f;
+  const float scale = fminf(16384.f, 4294967040.f / (float)V);
+  float d_max = INFINITY;
+  auto bin1 = [](float d) { return min(SAMP_BINS - 1, (int)(d * (1.f / W1))); };
+  auto clear = [&]() {
+    for (int i = tid; i < SAMP_BINS; i += NT) sh.hist[i] = 0;
+    __syncthreads();
+  };
+  auto flush_last = [&](uint32_t last) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) last += __shfl_xor_sync(0xffffffffu, last, o);
+    if (lane == 0 && last) atomicAdd(&sh.hist[SAMP_BINS - 1], last);
+  };
+  // first bin whose inclusive prefix reaches the target (SAMP_BINS: none does) and the exclusive prefix before it.  value(bin, sum) weighs a bin
+  auto find_bin = [&](float target, float& before, auto&& value) -> int {
+    if (tid == 0) sh.hit = SAMP_BINS;
+    cl_sync();                                                         // every CTA's histogram is complete
+    float own = 0.f, li = 0.f;
+    const int bin = rank * SAMP_SEG + tid;
+    if (tid < SAMP_SEG) {
+      uint32_t s = 0;
+#pragma unroll
+      for (int r = 0; r < SAMP_CL; ++r) s += cl_ld(&sh.hist[bin], r);
+      own = value(bin, s);
+      li = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, li, o);
+        if (lane >= o) li += t;
+      }
+      if (lane == 31) sh.scan[warp] = li;
+    }
+    __syncthreads();
+    float base = 0.f, total = 0.f;
+#pragma unroll
+    for (int w = 0; w < SAMP_SEG / 32; ++w) {
+      if (w == warp) base = total;
+      total += sh.scan[w];
+    }
+    if (tid < SAMP_CL) cl_st(&sh.seg_total[rank], tid, __float_as_uint(total));
+    cl_sync();
+    float seg = 0.f;
+    for (int r = 0; r < rank; ++r) seg += sh.seg_total[r];
+    float excl = 0.f;
+    if (tid < SAMP_SEG) {
+      const float prev = __shfl_up_sync(0xffffffffu, li, 1);
+      excl = seg + (base + (lane ? prev : 0.f));
+      if (seg + (base + li) >= target && (excl < target || bin == 0)) atomicMin(&sh.hit, bin);
+    }
+    __syncthreads();
+    const int hit = sh.hit;
+    if (hit == SAMP_BINS) {
+      if (tid < SAMP_CL) cl_st(&sh.cand_bin[rank], tid, SAMP_BINS);
+    } else if (bin == hit && tid < SAMP_SEG) {
+      for (int r = 0; r < SAMP_CL; ++r) { cl_st(&sh.cand_before[rank], r, __float_as_uint(excl)); cl_st(&sh.cand_bin[rank], r, (uint32_t)hit); }
+    }
+    cl_sync();
+    int found = SAMP_BINS;
+#pragma unroll
+    for (int r = SAMP_CL - 1; r >= 0; --r)
+      if (sh.cand_bin[r] < SAMP_BINS) { found = (int)sh.cand_bin[r]; before = __uint_as_float(sh.cand_before[r]); }
+    return found;
+  };
+  // refine bin b1: the smallest d edge whose kept count / mass reaches ``target``, given what lies before the bin
+  auto refine = [&](int b1, float target, auto&& weigh) -> float {
+    const float lo = b1 * W1, far = b1 == SAMP_BINS - 1 ? d_max : fminf(d_max, lo + W1);
+    clear();
+    uint32_t last = 0;
+    each([&](float d) {
+      if (d >= lo && d <= far && bin1(d) == b1) {
+        const int b = min(SAMP_BINS - 1, (int)((d - lo) * (SAMP_BINS / W1)));
+        if (b == SAMP_BINS - 1) ++last;
+        else atomicAdd(&sh.hist[b], 1u);
+      }
+    });
+    flush_last(last);
+    float before = 0.f;
+    const int b2 = find_bin(target, before, weigh);
+    if (b1 == SAMP_BINS - 1 && b2 >= SAMP_BINS - 1) return INFINITY;
+    return lo + (float)(min(b2, SAMP_BINS - 1) + 1) * (W1 / SAMP_BINS);
+  };
+  float base_mass = Z;
+  if (need_k) {
+    // The k-th largest of the threads' own maxima bounds the k-th largest logit from below: 2048 of them (or 8192) are histogrammed first, and only
+    // what lies above that bound then meets the atomics, instead of the whole row
+    float dm = INFINITY;
+    const auto count = [](int, uint32_t s) { return (float)s; };
+    if (topk <= SAMP_CL * NT / 2) {
+      clear();
+      const float d = (gmax - own_max) * inv_t;
+      if (d >= 0.f) atomicAdd(&sh.hist[bin1(d)], 1u);
+      float unused = 0.f;
+      const int b = find_bin((float)topk, unused, count);
+      if (b < SAMP_BINS - 1) dm = (b + 1) * W1;
+    }
+    clear();
+    uint32_t last = 0;
+    each([&](float d) {
+      if (d >= 0.f && d <= dm) {
+        const int b = bin1(d);
+        if (b == SAMP_BINS - 1) ++last;
+        else atomicAdd(&sh.hist[b], 1u);
+      }
+    });
+    flush_last(last);
+    float before = 0.f;
+    const int b1 = find_bin((float)topk, before, count);
+    if (b1 < SAMP_BINS) d_max = refine(b1, (float)topk - before, count);
+    if (need_p) {
+      float m = 0.f, unused = 0.f;
+      const float edge = d_max;
+      each([&](float d) { if (d >= 0.f && d <= edge) m += __expf(-d); });
+      reduce2(m, unused);
+      base_mass = m;
+    }
+  }
+  if (need_p) {
+    const float target = top_p * base_mass;
+    const float dm = d_max;
+    // all logits of r below (1 - p) base / V together cannot reach the mass that is cut off: half of that bound keeps the broad tail out of the atomics
+    const float tail = 0.5f * (1.f - top_p) * base_mass / (float)V;
+    const float d_tail = tail > 0.f ? fminf(dm, -__logf(tail)) : dm;
+    clear();
+    uint32_t last = 0;
+    each([&](float d) {
+      if (d >= 0.f && d <= d_tail) {
+        const int b = bin1(d);
+        const uint32_t q = (uint32_t)(__expf(b * W1 - d) * scale + 0.5f);
+        if (b == SAMP_BINS - 1) last += q;
+        else atomicAdd(&sh.hist[b], q);
+      }
+    });
+    flush_last(last);
+    float before = 0.f;
+    const float inv_scale = 1.f / scale;
+    int b1 = find_bin(target, before, [&](int bin, uint32_t s) { return (float)s * inv_scale * __expf(-bin * W1); });
+    b1 = min(b1, SAMP_BINS - 1);
+    float m_before, m_in;
+    int moved = 0;                                                     // one direction only: rounding at an edge cannot make it swing
+    while (true) {                                                     // (the same numbers in every thread of the cluster)
+      m_before = m_in = 0.f;
+      const int b = b1;
+      const float far = b == SAMP_BINS - 1 ? dm : fminf(dm, (b + 1) * W1);
+      each([&](float d) {
+        if (d >= 0.f && d <= far) {
+          const int k = bin1(d);
+          if (k <= b) {
+            const float r = __expf(-d);
+            if (k < b) m_before += r;
+            else m_in += r;
+          }
+        }
+      });
+      reduce2(m_before, m_in);
+      if (m_before >= target && b1 > 0 && moved <= 0) { moved = -1; --b1; continue; }
+      if (m_before + m_in < target && b1 < SAMP_BINS - 1 && moved >= 0) { moved = 1; ++b1; continue; }
+      break;
+    }
+    if (moved < 0 || m_before + m_in >= target)
+      d_max = fminf(d_max, refine(b1, target - m_before, [&](int b, uint32_t s) { return (float)s * __expf(-(b1 * W1 + (b + 0.5f) * (W1 / SAMP_BINS))); }));
+  }
+  // keep { r >= thr }, r = p / p_max
+  const float thr = d_max < INFINITY ? fmaxf(p.min_p[row], __expf(-d_max)) : p.min_p[row];
+  const float d_far = thr > 0.f ? -__logf(thr) + 0.01f : INFINITY;     // beyond it no r can reach thr: saves the exponential
+
+  // ---- kept mass of every warp (index order), the warp that holds the drawn point, then the token inside it
+  float cm = 0.f;
+  each([&](float d) {
+    if (d <= d_far) {
+      const float r = __expf(-d);
+      if (r >= thr) cm += r;
+    }
+  });
+  cm = warp_sum(cm);
+  if (lane < SAMP_CL) cl_st(&sh.kept[rank * NW + warp], lane, __float_as_uint(cm));
+  cl_sync();
+  if (warp == 0) {
+    constexpr int PER = SAMP_CL * NW / 32;
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) s += __uint_as_float(sh.kept[lane * PER + k]);
+    float incl = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const float total = __shfl_sync(0xffffffffu, incl, 31);
+    // a seeded request draws from (its seed, ITS OWN output position): the stream does not depend on which step / row / batch it landed in
+    const bool own = p.seeds && p.seeds[2 * row + 1] >= 0;
+    const long long step = p.step_ptr ? *p.step_ptr : p.step;
+    float u = (own ? rng_uniform((unsigned long long)p.seeds[2 * row], 0ull, (unsigned long long)p.seeds[2 * row + 1])
+                   : rng_uniform(p.global_seed, (unsigned long long)row, (unsigned long long)step)) * total;
+    const float up = __shfl_up_sync(0xffffffffu, incl, 1);
+    unsigned who = __ballot_sync(0xffffffffu, incl > u && s > 0.f);
+    if (who == 0) {                                                    // rounding at the very end: the last kept logit
+      who = __ballot_sync(0xffffffffu, s > 0.f);
+      who = who ? 1u << (31 - __clz(who)) : 0u;
+      u = INFINITY;
+    }
+    if (who == 0) {
+      if (lane == 0) sh.pick = -1;
+    } else if (lane == __ffs(who) - 1) {
+      float run = lane ? up : 0.f;
+      int pick = -1;
+      float pick_run = run;
+      for (int k = 0; k < PER; ++k) {
+        const float m = __uint_as_float(sh.kept[lane * PER + k]);
+        if (m <= 0.f) continue;
+        pick = lane * PER + k;
+        pick_run = run;
+        run += m;
+        if (run > u) break;
+      }
+      sh.pick = pick; sh.pick_run = pick_run; sh.pick_u = u;
+    }
+  }
+  __syncthreads();
+  const int pick = sh.pick;
+  if (pick < 0) {
+    if (rank == 0 && tid == 0) finish(arg);
+    return;
+  }
+  if (pick != rank * NW + warp) return;
+  float run = sh.pick_run;
+  const float u = sh.pick_u;
+  int token = arg;
+  for (int i0 = w0; i0 < w1; i0 += 256) {
+    const int i = i0 + lane * 8;
+    float v[8], r[8], s = 0.f;
+    int mine = -1;                                                     // last kept logit of this lane
+    if (i < w1) get8(i, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float e = i < w1 ? __expf((v[j] - gmax) * inv_t) : 0.f;
+      const bool keep = i < w1 && e >= thr;
+      r[j] = keep ? e : 0.f;
+      s += r[j];
+      if (keep) mine = i + j;
+    }
+    float incl = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const float up = __shfl_up_sync(0xffffffffu, incl, 1);
+    const unsigned who = __ballot_sync(0xffffffffu, run + incl > u && s > 0.f);
+    if (who) {
+      if (lane == __ffs(who) - 1) {
+        float c = run + (lane ? up : 0.f);
+        int tok = mine;
+#pragma unroll
+        for (int j = 7; j >= 0; --j) {                                 // the first kept logit whose running mass passes u (from the back: the lowest stays)
+          float upto = c;
+          for (int k = 0; k <= j; ++k) upto += r[k];
+          if (r[j] > 0.f && upto > u) tok = i + j;
+        }
+        finish(tok);
+      }
+      return;
+    }
+    const int far = __reduce_max_sync(0xffffffffu, mine);
+    if (far >= 0) token = far;
+    run += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) finish(token);
+}
+
+template <typename T, int NT>
+static void launch_sample(const void* logits, const SampleParams& p, int B, cudaStream_t stream) {
+  constexpr int NW = NT / 32;
+  const int per_warp = ((p.V + SAMP_CL * NW - 1) / (SAMP_CL * NW) + 255) / 256 * 256;
+  const size_t bytes = (size_t)per_warp * NW * sizeof(T);
+  if (bytes <= 200 * 1024) {
+    auto kern = sample_kernel<T, NT, true>;
+    if (bytes > 32 * 1024) SGLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    kern<<<B * SAMP_CL, NT, bytes, stream>>>((const T*)logits, p, per_warp);
+  } else {
+    sample_kernel<T, NT, false><<<B * SAMP_CL, NT, 0, stream>>>((const T*)logits, p, per_warp);
+  }
+  SGLB_CUDA_CHECK(cudaGetLastError());
 }
 
 void sample(const void* logits, bool bf16, int B, int V, int stride, const float* temperature, const int* top_k,
@@ -239,9 +545,14 @@ void sample(const void* logits, bool bf16, int B, int V, int stride, const float
   if (B <= 0) return;
   SampleParams p{temperature, top_k, top_p, min_p, seeds, out_slots, next_token_buf, out_tokens, out_logprobs, global_seed,
                  step_ptr, step, V, stride};
-  if (bf16) sample_kernel<__nv_bfloat16><<<B, SAMP_THREADS, 0, stream>>>((const __nv_bfloat16*)logits, p);
-  else sample_kernel<float><<<B, SAMP_THREADS, 0, stream>>>((const float*)logits, p);
-  SGLB_CUDA_CHECK(cudaGetLastError());
+  // few rows: one CTA per SM, so its threads hide the latency alone; many rows: small CTAs, several per SM (the line is where the chip is full)
+  if (B <= 18) {
+    if (bf16) launch_sample<__nv_bfloat16, 1024>(logits, p, B, stream);
+    else launch_sample<float, 1024>(logits, p, B, stream);
+  } else {
+    if (bf16) launch_sample<__nv_bfloat16, 256>(logits, p, B, stream);
+    else launch_sample<float, 256>(logits, p, B, stream);
+  }
 }
 
 // ---------------------------------------------------------------- grammar bitmask: logits[b, v] = -inf where bit == 0

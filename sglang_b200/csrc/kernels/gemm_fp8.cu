@@ -8,9 +8,12 @@
 // Scales change every 128-wide K block, so partial products cannot simply accumulate in TMEM.  Each K block is
 // therefore ONE 128-byte-swizzled smem stage (128 fp8 = 128 B per row) = 4 tcgen05.mma kind::f8f6f4 (K=32 each) into a
 // fresh TMEM accumulator stage; the epilogue warps drain that stage with tcgen05.ld, apply xs*ws and accumulate in fp32
-// registers ("promotion") while the tensor core already fills the next TMEM stage (4 stages x 128 columns = all 512).
+// registers ("promotion") while the tensor core already fills the next TMEM stage.  Two kernels:
 //
-//   warp 0 : TMA producer      warp 1 : MMA issuer      warp 2 : TMEM alloc      warps 4..7 : promotion + epilogue
+//   prompt shapes (gemm_fp8_block_kernel): rows of A are the UMMA M dimension, 256 / 128 / 64 weight rows the N dimension, persistent CTAs.
+//     warp 0 : TMA producer      warp 1 : MMA issuer      warp 2 : TMEM alloc      warps 4.. : promotion + epilogue, 64 columns each at most
+//   decode shapes (gemm_fp8_swap_kernel, up to 128 tokens): 128 weight rows are the M dimension, the tokens the N dimension, so no tensor or TMA
+//     work goes into padding rows; a cluster shares a tile's K blocks and adds its partial sums through distributed shared memory.
 //
 // Reference counterparts: python/sglang/srt/layers/quantization/fp8_kernel.py (per_token_group_quant_fp8,
 // w8a8_block_fp8_matmul), fp8_utils.py:552-808 (DeepGEMM / cutlass / triton dispatch), sgl-kernel fp8_blockwise_gemm.
@@ -23,26 +26,39 @@ namespace sglb {
 
 constexpr int F8_BM = 128;
 constexpr int F8_BK = 128;          // fp8 elements = bytes per swizzled row = one scale group
-constexpr int F8_THREADS = 256;
+// sum pair += s * (a, b): one packed instruction for two fp32 fused multiply-adds, each rounded as fmaf rounds it
+__device__ __forceinline__ void fma_pair(float2& sum, float s, uint32_t a, uint32_t b) {
+  uint64_t acc = *reinterpret_cast<uint64_t*>(&sum), v, m;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(a), "r"(b));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(m) : "r"(__float_as_uint(s)));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(m), "l"(v));
+  sum = *reinterpret_cast<float2*>(&acc);
+}
 
+// Bound by the tensor core once the promotion keeps up: per K block a 128 x 256 tile is 512 cycles of UMMA against, per SM sub-partition, 4 warps x
+// 32 packed multiply-adds and their TMEM loads.  The version before promoted 128 x 128 with one warpgroup (128 scalar multiply-adds behind four
+// exposed TMEM loads per block) and was bound by that chain.  Measured, 3001 tokens, [28672 x 4096] and [4096 x 14336]: 445 -> 318 us a product (together 1.66 PFLOP/s).
 template <int BN>
 struct F8Cfg {
   static constexpr int A_BYTES = F8_BM * F8_BK;
   static constexpr int B_BYTES = BN * F8_BK;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN >= 128) ? 6 : 8;
-  static constexpr int NACC = 512 / BN > 4 ? 4 : 512 / BN;      // TMEM accumulator stages
+  static constexpr int STAGES = BN == 256 ? 4 : BN == 128 ? 6 : 8;
+  static constexpr int NACC = BN == 256 ? 2 : 4;                // TMEM accumulator stages
   static constexpr int TMEM_COLS = NACC * BN;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+  static constexpr int COLS = BN == 64 ? 32 : 64;               // columns of one epilogue warp
+  static constexpr int EPI_WARPS = 4 * (BN / COLS);
+  static constexpr int THREADS = 128 + 32 * EPI_WARPS;
 };
 
 template <int BN>
-__global__ void __launch_bounds__(F8_THREADS, 1)
+__global__ void __launch_bounds__(F8Cfg<BN>::THREADS, 1)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const float* __restrict__ xs, const float* __restrict__ ws, __nv_bfloat16* __restrict__ C, int M, int N, int K,
                       int ldc, int xs_stride, int ws_stride) {
   using Cfg = F8Cfg<BN>;
-  constexpr int STAGES = Cfg::STAGES, NACC = Cfg::NACC;
+  constexpr int STAGES = Cfg::STAGES, NACC = Cfg::NACC, COLS = Cfg::COLS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
@@ -62,7 +78,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   if (warp == 0 && lane == 0) { tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); }
   if (warp == 1 && lane == 0) {
     for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-    for (int i = 0; i < NACC; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], 4); }
+    for (int i = 0; i < NACC; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], Cfg::EPI_WARPS); }
     fence_barrier_init();
   }
   if (warp == 2) { tmem_alloc(tmem_ptr, Cfg::TMEM_COLS); tmem_relinquish(); }
@@ -104,46 +120,46 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
     }
   } else if (warp >= 4) {
-    const int q = warp - 4;
+    const int q = warp & 3, c0 = ((warp - 4) >> 2) * COLS;          // a warp reads the TMEM lanes of its index modulo 4
     int acc = 0; uint32_t acc_phase = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
       const int m_blk = tile % m_tiles, n_blk = tile / m_tiles;
       const int row = m_blk * F8_BM + q * 32 + lane;
       const int row_c = min(row, M - 1);
-      float sum[BN];
+      const int col0 = n_blk * BN + c0;
+      // the warp's columns (64 from a multiple of 64) lie in one 128-wide weight block
+      const float* ws_row = ws + (size_t)(min(col0, N - 1) >> 7) * ws_stride;
+      float2 sum[COLS / 2];
 #pragma unroll
-      for (int i = 0; i < BN; ++i) sum[i] = 0.f;
+      for (int i = 0; i < COLS / 2; ++i) sum[i] = make_float2(0.f, 0.f);
       const float* xs_row = xs + (size_t)row_c * xs_stride;
-      float a_scale = __ldg(xs_row);
+      float a_scale = __ldg(xs_row), w_scale = __ldg(ws_row);
       for (int kb = 0; kb < num_kb; ++kb) {
-        const float a_next = (kb + 1 < num_kb) ? __ldg(xs_row + kb + 1) : 0.f;
+        const float s = a_scale * w_scale;
+        if (kb + 1 < num_kb) { a_scale = __ldg(xs_row + kb + 1); w_scale = __ldg(ws_row + kb + 1); }
         mbar_wait(&tfull[acc], acc_phase);
         tc_fence_after();
-        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
+        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + c0;
 #pragma unroll
-        for (int c = 0; c < BN / 32; ++c) {
-          // weight-block scale of these 32 columns (a 128-column block never straddles a 32-column chunk)
-          const int nb = min(n_blk * BN + c * 32, N - 1) >> 7;
-          const float s = a_scale * __ldg(ws + (size_t)nb * ws_stride + kb);
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(t_row + c * 32, r);
+        for (int c = 0; c < COLS; c += 16) {
+          uint32_t r[16];
+          tmem_ld_32x32b_x16(t_row + c, r);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) sum[c * 32 + i] = fmaf(s, __uint_as_float(r[i]), sum[c * 32 + i]);
+          for (int i = 0; i < 8; ++i) fma_pair(sum[c / 2 + i], s, r[2 * i], r[2 * i + 1]);
         }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty[acc]);
         if (++acc == NACC) { acc = 0; acc_phase ^= 1; }
-        a_scale = a_next;
       }
       if (row < M) {
 #pragma unroll
-        for (int v = 0; v < BN / 8; ++v) {
-          const int col = n_blk * BN + v * 8;
+        for (int v = 0; v < COLS / 8; ++v) {
+          const int col = col0 + v * 8;
           if (col < N) {
-            const U4 o = U4{pack_bf16(sum[v * 8], sum[v * 8 + 1]), pack_bf16(sum[v * 8 + 2], sum[v * 8 + 3]),
-                            pack_bf16(sum[v * 8 + 4], sum[v * 8 + 5]), pack_bf16(sum[v * 8 + 6], sum[v * 8 + 7])};
+            const U4 o = U4{pack_bf16(sum[v * 4].x, sum[v * 4].y), pack_bf16(sum[v * 4 + 1].x, sum[v * 4 + 1].y),
+                            pack_bf16(sum[v * 4 + 2].x, sum[v * 4 + 2].y), pack_bf16(sum[v * 4 + 3].x, sum[v * 4 + 3].y)};
             st128(C + (size_t)row * ldc + col, o);
           }
         }
@@ -172,24 +188,233 @@ static void launch_fp8(const void* A, const float* xs, const void* W, const floa
   }
   const int m_tiles = (M + F8_BM - 1) / F8_BM, n_tiles = (N + BN - 1) / BN;
   const int grid = (int)std::min<long long>((long long)m_tiles * n_tiles, num_sms);
-  kern<<<grid, F8_THREADS, Cfg::SMEM_BYTES, stream>>>(tmA, tmB, xs, ws, (__nv_bfloat16*)C, M, N, K, ldc, xs_stride, ws_stride);
+  kern<<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(tmA, tmB, xs, ws, (__nv_bfloat16*)C, M, N, K, ldc, xs_stride, ws_stride);
   SGLB_CUDA_CHECK(cudaGetLastError());
+}
+
+// ---------------------------------------------------------------- decode shapes: weights as the UMMA M dimension
+// Bound by streaming the weights.  Every CTA owns (128 weight rows) x (a share of the K blocks); the CTAs of a cluster share one tile, park their
+// fp32 partial sums in their own shared memory and each adds up (in rank order) and writes an equal part of the tokens.  Small CTAs (three 16 KB
+// weight stages) so that three or four of them per SM keep ~200 KB in flight and hide one another's start and end.
+// Measured, 9 tokens, [7168 x 8192] and [8192 x 3584]: 43.6 -> 15.1 us a product on average (the version before ran 32-wide tiles of 128 padded rows).
+constexpr int F8S_THREADS = 192;
+template <int NT>
+struct F8SwapCfg {
+  static constexpr int W_BYTES = 128 * F8_BK;
+  static constexpr int STAGE_BYTES = W_BYTES + NT * F8_BK;
+  static constexpr int STAGES = 3;
+  // accumulator stages: the CTAs that shared memory lets onto an SM never want more than its 512 TMEM columns (a cluster must not wait for them)
+  static constexpr int NACC = NT <= 32 ? 4 : 2;
+  static constexpr int TMEM_COLS = NACC * NT;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 8 * NT * 4 + 256 + 1024;
+  static_assert((228 * 1024 / (SMEM_BYTES + 1024)) * TMEM_COLS <= 512, "TMEM columns of the co-resident CTAs");
+  static_assert(NT * 128 * 4 <= STAGES * STAGE_BYTES, "the partial sums reuse the stages");
+};
+
+template <int NT>
+__global__ void __launch_bounds__(F8S_THREADS)
+gemm_fp8_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const float* __restrict__ xs,
+                     const float* __restrict__ ws, __nv_bfloat16* __restrict__ C, int M, int N, int K, int ldc, int xs_stride, int ws_stride, int splits) {
+  using Cfg = F8SwapCfg<NT>;
+  constexpr int STAGES = Cfg::STAGES, NACC = Cfg::NACC;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sW = smem;
+  uint8_t* sX = smem + STAGES * Cfg::W_BYTES;
+  float* s_scale = reinterpret_cast<float*>(smem + STAGES * Cfg::STAGE_BYTES);     // [warp][2][NT] token scales of a K block, a copy per warp
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_scale + 8 * NT);
+  uint64_t* full = bars;
+  uint64_t* empty = bars + STAGES;
+  uint64_t* tfull = bars + 2 * STAGES;
+  uint64_t* tempty = bars + 2 * STAGES + NACC;
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * NACC);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = blockIdx.x / splits, rank = blockIdx.x % splits;
+  const int num_kb = (K + F8_BK - 1) / F8_BK;
+  const int kb0 = num_kb * rank / splits, kb1 = num_kb * (rank + 1) / splits;
+
+  if (warp == 5 && lane == 0) { tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmX); }
+  if (warp == 4 && lane == 0) {
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < NACC; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], 4); }
+    fence_barrier_init();
+  }
+  if (warp == 0) { tmem_alloc(tmem_ptr, Cfg::TMEM_COLS); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_ptr;
+
+  if (warp == 5) {
+    if (lane == 0) {
+      int stage = 0; uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mbar_wait(&empty[stage], phase ^ 1);
+        mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
+        tma_load_2d(sW + stage * Cfg::W_BYTES, &tmW, &full[stage], kb * F8_BK, tile * 128);
+        tma_load_2d(sX + stage * NT * F8_BK, &tmX, &full[stage], kb * F8_BK, 0);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 4) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(UMMA_E4M3, UMMA_E4M3, 128, NT, 0, 0);
+      int stage = 0; uint32_t phase = 0;
+      int acc = 0; uint32_t acc_phase = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mbar_wait(&tempty[acc], acc_phase ^ 1);
+        mbar_wait(&full[stage], phase);
+        tc_fence_after();
+        const uint64_t wdesc = make_smem_desc_sw128(smem_u32(sW + stage * Cfg::W_BYTES), 0, 1024);
+        const uint64_t xdesc = make_smem_desc_sw128(smem_u32(sX + stage * NT * F8_BK), 0, 1024);
+#pragma unroll
+        for (int k = 0; k < F8_BK / 32; ++k) umma_f8_ss(tmem_base + acc * NT, wdesc + 2 * k, xdesc + 2 * k, idesc, k != 0);
+        umma_commit(&empty[stage]);
+        umma_commit(&tfull[acc]);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        if (++acc == NACC) { acc = 0; acc_phase ^= 1; }
+      }
+    }
+    __syncwarp();
+  } else {
+    float sum[NT];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) sum[i] = 0.f;
+    const float* ws_row = ws + (size_t)tile * ws_stride;                // 128 rows from a multiple of 128: one scale per K block
+    float* mine = s_scale + warp * 2 * NT;
+    constexpr int PL = (NT + 31) / 32;
+    float nx[PL];
+    auto fetch = [&](int kb) {
+      const float w = __ldg(ws_row + kb);
+#pragma unroll
+      for (int i = 0; i < PL; ++i) nx[i] = i * 32 + lane < M ? __ldg(xs + (size_t)(i * 32 + lane) * xs_stride + kb) * w : 0.f;
+    };
+    if (kb0 < kb1) fetch(kb0);
+    int acc = 0; uint32_t acc_phase = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      float* sc = mine + (kb & 1) * NT;
+#pragma unroll
+      for (int i = 0; i < PL; ++i)
+        if (i * 32 + lane < NT) sc[i * 32 + lane] = nx[i];
+      if (kb + 1 < kb1) fetch(kb + 1);
+      __syncwarp();                     // (the other half is rewritten only after every lane has passed the next one)
+      mbar_wait(&tfull[acc], acc_phase);
+      tc_fence_after();
+      const uint32_t t_row = tmem_base + ((uint32_t)(warp * 32) << 16) + acc * NT;
+#pragma unroll
+      for (int c = 0; c < NT; c += 16) {
+        uint32_t r[16];
+        tmem_ld_32x32b_x16(t_row + c, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+          const float4 f = *reinterpret_cast<const float4*>(sc + c + i);
+          sum[c + i] = fmaf(f.x, __uint_as_float(r[i]), sum[c + i]);
+          sum[c + i + 1] = fmaf(f.y, __uint_as_float(r[i + 1]), sum[c + i + 1]);
+          sum[c + i + 2] = fmaf(f.z, __uint_as_float(r[i + 2]), sum[c + i + 2]);
+          sum[c + i + 3] = fmaf(f.w, __uint_as_float(r[i + 3]), sum[c + i + 3]);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[acc]);
+      if (++acc == NACC) { acc = 0; acc_phase ^= 1; }
+    }
+    const int n = tile * 128 + threadIdx.x;
+    if (splits == 1) {
+      if (n < N) {
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+          if (j < M) C[(size_t)j * ldc + n] = __float2bfloat16(sum[j]);
+      }
+    } else {
+      // the last block's accumulator is drained, so its multiplications have read the stages: their memory takes the partial sums
+      float* part = reinterpret_cast<float*>(smem);
+#pragma unroll
+      for (int j = 0; j < NT; ++j) part[j * 128 + threadIdx.x] = sum[j];
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+  if (splits > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int n = tile * 128 + threadIdx.x;
+    if (threadIdx.x < 128 && n < N) {
+      const int j1 = min(M, NT * (rank + 1) / splits);
+      const uint32_t base = smem_u32(smem) + threadIdx.x * 4;
+      for (int j = NT * rank / splits; j < j1; ++j) {
+        float v[8], t = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          uint32_t a;
+          v[r] = 0.f;
+          if (r < splits) {
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(base + j * 512), "r"(r));
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[r]) : "r"(a) : "memory");
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) t += v[r];
+        C[(size_t)j * ldc + n] = __float2bfloat16(t);
+      }
+    }
+    // nobody leaves while a peer still reads its partial sums
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+template <int NT>
+static void launch_fp8_swap(const void* A, const float* xs, const void* W, const float* ws, void* C, int M, int N, int K, int lda, int ldw,
+                            int ldc, int xs_stride, int ws_stride, int num_sms, cudaStream_t stream) {
+  using Cfg = F8SwapCfg<NT>;
+  uint64_t dW[2] = {(uint64_t)K, (uint64_t)N}, sWs[1] = {(uint64_t)ldw};
+  uint64_t dX[2] = {(uint64_t)K, (uint64_t)M}, sXs[1] = {(uint64_t)lda};
+  uint32_t bW[2] = {F8_BK, 128}, bX[2] = {F8_BK, (uint32_t)NT};
+  CUtensorMap tmW = make_tmap(W, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, dW, sWs, bW, CU_TENSOR_MAP_SWIZZLE_128B);
+  CUtensorMap tmX = make_tmap(A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, dX, sXs, bX, CU_TENSOR_MAP_SWIZZLE_128B);
+  auto kern = gemm_fp8_swap_kernel<NT>;
+  SGLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+  const int tiles = (N + 127) / 128, num_kb = (K + F8_BK - 1) / F8_BK;
+  // share a tile's K blocks while the CTAs fit the chip at once and each still has two blocks to stream
+  const int slots = num_sms * (228 * 1024 / (Cfg::SMEM_BYTES + 1024));
+  int splits = 1;
+  while (splits < 8 && tiles * splits * 2 <= slots && num_kb >= splits * 4) splits *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(tiles * splits); cfg.blockDim = dim3(F8S_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM_BYTES; cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  SGLB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmW, tmX, xs, ws, (__nv_bfloat16*)C, M, N, K, ldc, xs_stride, ws_stride, splits));
 }
 
 void gemm_fp8_block(const void* A, const float* xs, const void* W, const float* ws, void* C, int M, int N, int K, int lda, int ldw,
                     int ldc, int xs_stride, int ws_stride, int num_sms, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return;
   if (K % 16 || N % 8 || lda % 16 || ldw % 16) throw std::runtime_error("sglb fp8 gemm: K, lda, ldw must be multiples of 16 and N of 8");
+#define SGLB_F8(F) F(A, xs, W, ws, C, M, N, K, lda, ldw, ldc, xs_stride, ws_stride, num_sms, stream)
+  // up to 128 tokens fit one UMMA N dimension beside 128 weight rows; from there on a weight tile would be read once per 128 tokens either way
+  if (M <= 16) { SGLB_F8(launch_fp8_swap<16>); return; }
+  if (M <= 32) { SGLB_F8(launch_fp8_swap<32>); return; }
+  if (M <= 64) { SGLB_F8(launch_fp8_swap<64>); return; }
+  if (M <= 128) { SGLB_F8(launch_fp8_swap<128>); return; }
+  // the width whose waves take the least time: a tile costs its columns plus a start and an end worth about 32 of them
   const int m_tiles = (M + F8_BM - 1) / F8_BM;
-  // small M is weight-bandwidth bound: narrower tiles -> more CTAs streaming W
-  int bn = 128;
-  if (m_tiles * ((N + 127) / 128) < num_sms) bn = 64;
-  if (m_tiles * ((N + 63) / 64) < num_sms) bn = 32;
-  switch (bn) {
-    case 128: launch_fp8<128>(A, xs, W, ws, C, M, N, K, lda, ldw, ldc, xs_stride, ws_stride, num_sms, stream); break;
-    case 64: launch_fp8<64>(A, xs, W, ws, C, M, N, K, lda, ldw, ldc, xs_stride, ws_stride, num_sms, stream); break;
-    default: launch_fp8<32>(A, xs, W, ws, C, M, N, K, lda, ldw, ldc, xs_stride, ws_stride, num_sms, stream); break;
+  int bn = 0;
+  long long best = 0;
+  for (int w : {256, 128, 64}) {
+    const long long tiles = (long long)m_tiles * ((N + w - 1) / w), cost = (tiles + num_sms - 1) / num_sms * (w + 32);
+    if (!bn || cost < best) { bn = w; best = cost; }
   }
+  switch (bn) {
+    case 256: SGLB_F8(launch_fp8<256>); break;
+    case 128: SGLB_F8(launch_fp8<128>); break;
+    default: SGLB_F8(launch_fp8<64>); break;
+  }
+#undef SGLB_F8
 }
 
 // ---------------------------------------------------------------- activation quantiser: one warp per (row, 128-group)

@@ -87,39 +87,54 @@ void rmsnorm(void* x, void* residual, const void* w, void* out, int T, int H, in
 }
 
 // ---------------------------------------------------------------- act(x[:, :I]) * x[:, I:]
+// Bound by memory once the arithmetic is out of its way: a CTA keeps one row (no division per vector) and two vectors of each half in flight per
+// thread, and the SiLU's quotient is a reciprocal and a product (two special-function results per element; the IEEE division sequence alone took
+// longer than the bytes).  [5003, 28672] bf16: 93 -> 66 us, 430 MB.
+__device__ __forceinline__ float silu_f32(float g) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-g)));
+  return g * r;
+}
 template <int ACT>  // 0 silu, 1 gelu(erf), 2 gelu(tanh)
-__global__ void act_and_mul_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out, int T, int I,
-                                   int x_stride) {
-  const int nvec = I >> 3;
-  const size_t total = (size_t)T * nvec;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
-    const int t = idx / nvec, vi = idx % nvec;
-    const __nv_bfloat16* row = x + (size_t)t * x_stride;
-    U4 a = ld128(row + vi * 8), b = ld128(row + I + vi * 8);
-    float g[8] = {bf16_lo(a.x), bf16_hi(a.x), bf16_lo(a.y), bf16_hi(a.y), bf16_lo(a.z), bf16_hi(a.z), bf16_lo(a.w), bf16_hi(a.w)};
-    float u[8] = {bf16_lo(b.x), bf16_hi(b.x), bf16_lo(b.y), bf16_hi(b.y), bf16_lo(b.z), bf16_hi(b.z), bf16_lo(b.w), bf16_hi(b.w)};
-    float o[8];
+__device__ __forceinline__ U4 act_mul8(const U4 a, const U4 b) {
+  const float g[8] = {bf16_lo(a.x), bf16_hi(a.x), bf16_lo(a.y), bf16_hi(a.y), bf16_lo(a.z), bf16_hi(a.z), bf16_lo(a.w), bf16_hi(a.w)};
+  const float u[8] = {bf16_lo(b.x), bf16_hi(b.x), bf16_lo(b.y), bf16_hi(b.y), bf16_lo(b.z), bf16_hi(b.z), bf16_lo(b.w), bf16_hi(b.w)};
+  float o[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      float a_;
-      if (ACT == 0) a_ = g[k] / (1.f + __expf(-g[k]));
-      else if (ACT == 1) a_ = 0.5f * g[k] * (1.f + erff(g[k] * 0.7071067811865476f));
-      else { const float c = 0.7978845608028654f * (g[k] + 0.044715f * g[k] * g[k] * g[k]); a_ = 0.5f * g[k] * (1.f + tanhf(c)); }
-      o[k] = a_ * u[k];
-    }
-    st128(out + (size_t)t * I + vi * 8, U4{pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7])});
+  for (int k = 0; k < 8; ++k) {
+    float a_;
+    if (ACT == 0) a_ = silu_f32(g[k]);
+    else if (ACT == 1) a_ = 0.5f * g[k] * (1.f + erff(g[k] * 0.7071067811865476f));
+    else { const float c = 0.7978845608028654f * (g[k] + 0.044715f * g[k] * g[k] * g[k]); a_ = 0.5f * g[k] * (1.f + tanhf(c)); }
+    o[k] = a_ * u[k];
   }
+  return U4{pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7])};
+}
+
+template <int ACT>
+__global__ void __launch_bounds__(256) act_and_mul_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out, int I, int x_stride) {
+  const __nv_bfloat16* row = x + (size_t)blockIdx.x * x_stride;
+  __nv_bfloat16* dst = out + (size_t)blockIdx.x * I;
+  const int nvec = I >> 3, step = gridDim.y * 256;
+  int v = blockIdx.y * 256 + threadIdx.x;
+  for (; v + step < nvec; v += 2 * step) {
+    const U4 a0 = ld128(row + v * 8), b0 = ld128(row + I + v * 8), a1 = ld128(row + (v + step) * 8), b1 = ld128(row + I + (v + step) * 8);
+    st128(dst + v * 8, act_mul8<ACT>(a0, b0));
+    st128(dst + (v + step) * 8, act_mul8<ACT>(a1, b1));
+  }
+  if (v < nvec) st128(dst + v * 8, act_mul8<ACT>(ld128(row + v * 8), ld128(row + I + v * 8)));
 }
 
 void act_and_mul(const void* x, void* out, int T, int I, int x_stride, int act, cudaStream_t stream) {
   if (T <= 0) return;
   if (I % 8) throw std::runtime_error("sglb act_and_mul: I must be a multiple of 8");
-  const size_t total = (size_t)T * (I / 8);
-  size_t gq = (total + 255) / 256; const int grid = (int)(gq < (size_t)(148 * 16) ? gq : (size_t)(148 * 16));
+  const int chunks = (I / 8 + 255) / 256;
+  // few rows: a CTA per 256 vectors of a row; from a few CTAs per SM on, longer rows per CTA
+  const dim3 grid(T, T * chunks <= 148 * 8 ? chunks : (chunks + 3) / 4);
   auto X = (const __nv_bfloat16*)x; auto O = (__nv_bfloat16*)out;
-  if (act == 0) act_and_mul_kernel<0><<<grid, 256, 0, stream>>>(X, O, T, I, x_stride);
-  else if (act == 1) act_and_mul_kernel<1><<<grid, 256, 0, stream>>>(X, O, T, I, x_stride);
-  else act_and_mul_kernel<2><<<grid, 256, 0, stream>>>(X, O, T, I, x_stride);
+  if (act == 0) act_and_mul_kernel<0><<<grid, 256, 0, stream>>>(X, O, I, x_stride);
+  else if (act == 1) act_and_mul_kernel<1><<<grid, 256, 0, stream>>>(X, O, I, x_stride);
+  else act_and_mul_kernel<2><<<grid, 256, 0, stream>>>(X, O, I, x_stride);
   SGLB_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -227,12 +242,90 @@ __global__ void __launch_bounds__(256) rope_kv_write_kernel(__nv_bfloat16* __res
   }
 }
 
+// The common form (whole head rotated, halves, one slab, 16-byte aligned rows): a CTA per token, a thread per eight rotation pairs, so every access is
+// 16 bytes and the token's sines are read from L1 by all its heads.  5003 tokens, 32 + 8 heads of 128: 51 -> 24 us (it was four bytes a lane).
+template <typename CacheT>
+__device__ __forceinline__ void store_cache8(CacheT* dst, const float (&o)[8], float inv_scale);
+template <>
+__device__ __forceinline__ void store_cache8<__nv_bfloat16>(__nv_bfloat16* dst, const float (&o)[8], float) {
+  st128(dst, U4{pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7])});
+}
+template <>
+__device__ __forceinline__ void store_cache8<__nv_fp8_e4m3>(__nv_fp8_e4m3* dst, const float (&o)[8], float inv_scale) {
+  __align__(8) __nv_fp8_e4m3 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __nv_fp8_e4m3(o[i] * inv_scale);
+  *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(v);
+}
+__device__ __forceinline__ void unpack8(const U4 a, float (&f)[8]) {
+  f[0] = bf16_lo(a.x); f[1] = bf16_hi(a.x); f[2] = bf16_lo(a.y); f[3] = bf16_hi(a.y);
+  f[4] = bf16_lo(a.z); f[5] = bf16_hi(a.z); f[6] = bf16_lo(a.w); f[7] = bf16_hi(a.w);
+}
+
+template <typename CacheT>
+__global__ void __launch_bounds__(384) rope_kv_write_vec_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
+                                                                const __nv_bfloat16* __restrict__ v, const int* __restrict__ positions,
+                                                                const float* __restrict__ cos_sin, CacheT* __restrict__ k_cache,
+                                                                CacheT* __restrict__ v_cache, const int* __restrict__ out_loc, int Hq, int Hkv,
+                                                                int D, int per, int q_stride, int k_stride, int v_stride, float k_inv_scale,
+                                                                float v_inv_scale) {
+  const int t = blockIdx.x, half = D >> 1, items = (Hq + 2 * Hkv) * per;      // per = half / 8 threads a head
+  const float* cs = cos_sin + (size_t)positions[t] * D;
+  const size_t slot = out_loc[t];
+  for (int i = threadIdx.x; i < items; i += blockDim.x) {
+    const int h = i / per, c = (i - h * per) * 8;
+    if (h < Hq + Hkv) {
+      __nv_bfloat16* src = h < Hq ? q + (size_t)t * q_stride + h * D : const_cast<__nv_bfloat16*>(k) + (size_t)t * k_stride + (h - Hq) * D;
+      float x1[8], x2[8], co[8], si[8], o1[8], o2[8];
+      unpack8(ld128(src + c), x1);
+      unpack8(ld128(src + half + c), x2);
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        *reinterpret_cast<float4*>(co + j) = __ldg(reinterpret_cast<const float4*>(cs + c + j));
+        *reinterpret_cast<float4*>(si + j) = __ldg(reinterpret_cast<const float4*>(cs + half + c + j));
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { o1[j] = x1[j] * co[j] - x2[j] * si[j]; o2[j] = x2[j] * co[j] + x1[j] * si[j]; }
+      if (h < Hq) {
+        store_cache8<__nv_bfloat16>(src + c, o1, 1.f);
+        store_cache8<__nv_bfloat16>(src + half + c, o2, 1.f);
+      } else {
+        CacheT* dst = k_cache + (slot * Hkv + (h - Hq)) * D;
+        store_cache8<CacheT>(dst + c, o1, k_inv_scale);
+        store_cache8<CacheT>(dst + half + c, o2, k_inv_scale);
+      }
+    } else {
+      const __nv_bfloat16* src = v + (size_t)t * v_stride + (h - Hq - Hkv) * D;
+      CacheT* dst = v_cache + (slot * Hkv + (h - Hq - Hkv)) * D;
+      float a[8], b[8];
+      unpack8(ld128(src + c), a);
+      unpack8(ld128(src + half + c), b);
+      store_cache8<CacheT>(dst + c, a, v_inv_scale);
+      store_cache8<CacheT>(dst + half + c, b, v_inv_scale);
+    }
+  }
+}
+
 void rope_kv_write(void* q, const void* k, const void* v, const int* positions, const float* cos_sin, void* k_cache,
                    void* v_cache, const int* out_loc, int T, int Hq, int Hkv, int D, int rot, int q_stride, int k_stride,
                    int v_stride, bool neox, bool fp8_cache, float k_scale, float v_scale, int nslabs, long long slab_stride,
                    cudaStream_t stream) {
   if (T <= 0) return;
   if (rot % 4 || D % 2) throw std::runtime_error("sglb rope: rotary_dim must be a multiple of 4");
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (neox && rot == D && D % 16 == 0 && nslabs == 1 && q_stride % 8 == 0 && k_stride % 8 == 0 && v_stride % 8 == 0 && aligned(q) && aligned(k) &&
+      aligned(v) && aligned(cos_sin) && aligned(k_cache) && aligned(v_cache)) {
+    const int per = D / 16, threads = min(384, ((Hq + 2 * Hkv) * per + 31) / 32 * 32);
+#define RV(CT)                                                                                                                              \
+  rope_kv_write_vec_kernel<CT><<<T, threads, 0, stream>>>((__nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, positions, cos_sin, \
+                                                          (CT*)k_cache, (CT*)v_cache, out_loc, Hq, Hkv, D, per, q_stride, k_stride, v_stride,  \
+                                                          1.f / k_scale, 1.f / v_scale)
+    if (fp8_cache) RV(__nv_fp8_e4m3);
+    else RV(__nv_bfloat16);
+#undef RV
+    SGLB_CUDA_CHECK(cudaGetLastError());
+    return;
+  }
   const long warps = (long)T * (Hq + 2 * Hkv);
   const int grid = (int)((warps + 7) / 8);
   auto Q = (__nv_bfloat16*)q; auto K = (const __nv_bfloat16*)k; auto V = (const __nv_bfloat16*)v;

@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(256) per_token_group_quant_fp8_kernel(const __
   const int row = gw / groups, g = gw % groups;
   const int col = g * 128 + lane * 4;
   float v[4] = {0.f, 0.f, 0.f, 0.f};
-  if (col + 3 < K) {
+  if (col + 3 < K && ((x_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 7) == 0)) {      // (rows of another stride are read value by value)
     const uint2 raw = *reinterpret_cast<const uint2*>(x + (size_t)row * x_stride + col);
     v[0] = bf16_lo(raw.x); v[1] = bf16_hi(raw.x); v[2] = bf16_lo(raw.y); v[3] = bf16_hi(raw.y);
   } else {
@@ -454,11 +454,60 @@ __global__ void __launch_bounds__(256) per_token_group_quant_fp8_kernel(const __
   }
 }
 
+// 16-byte rows: a thread takes eight values, half a warp a group, and a warp four groups whose loads are all in flight together.
+// [3001, 4096] and [3001, 14336], on average: 36 -> 20 us (it was one 8-byte load a lane and a warp per group).
+__global__ void __launch_bounds__(256) per_token_group_quant_fp8_vec_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
+                                                                            float* __restrict__ scales, long long total, int K, int x_stride,
+                                                                            int groups, int ue8m0) {
+  const int lane = threadIdx.x & 31, half = lane >> 4, l = lane & 15;
+  const long long g0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4 + half;
+  U4 raw[2];
+  int row[2], col[2], grp[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const long long g = g0 + 2 * i;
+    row[i] = g < total ? (int)((unsigned)g / (unsigned)groups) : -1;
+    grp[i] = row[i] < 0 ? 0 : (int)((unsigned)g - (unsigned)row[i] * (unsigned)groups);
+    col[i] = grp[i] * 128 + l * 8;
+    raw[i] = row[i] >= 0 && col[i] < K ? ldg128(x + (size_t)row[i] * x_stride + col[i]) : U4{0, 0, 0, 0};
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float v[8] = {bf16_lo(raw[i].x), bf16_hi(raw[i].x), bf16_lo(raw[i].y), bf16_hi(raw[i].y),
+                        bf16_lo(raw[i].z), bf16_hi(raw[i].z), bf16_lo(raw[i].w), bf16_hi(raw[i].w)};
+    float amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    float scale = fmaxf(amax, 1e-10f) / 448.f;
+    if (ue8m0) scale = exp2f(ceilf(log2f(scale)));
+    const float inv = 1.f / scale;
+    if (row[i] < 0) continue;
+    if (l == 0) scales[(size_t)row[i] * groups + grp[i]] = scale;
+    if (col[i] >= K) continue;
+    uint32_t w[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j] * inv, v[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+      const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j + 2] * inv, v[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
+      w[j] = lo | hi << 16;
+    }
+    *reinterpret_cast<uint2*>(q + (size_t)row[i] * K + col[i]) = make_uint2(w[0], w[1]);
+  }
+}
+
 void per_token_group_quant_fp8(const void* x, void* q, float* scales, int M, int K, int x_stride, bool ue8m0, cudaStream_t stream) {
   if (M <= 0) return;
   if (K % 4) throw std::runtime_error("sglb fp8 quant: K must be a multiple of 4");
   const int groups = (K + 127) / 128;
   const long long warps = (long long)M * groups;
+  if (K % 8 == 0 && x_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0 && warps < (1ll << 31)) {
+    per_token_group_quant_fp8_vec_kernel<<<(int)((warps + 31) / 32), 256, 0, stream>>>((const __nv_bfloat16*)x, (uint8_t*)q, scales, warps, K, x_stride,
+                                                                                       groups, ue8m0);
+    SGLB_CUDA_CHECK(cudaGetLastError());
+    return;
+  }
   const int grid = (int)((warps * 32 + 255) / 256);
   per_token_group_quant_fp8_kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, (uint8_t*)q, scales, M, K, x_stride, groups, ue8m0);
   SGLB_CUDA_CHECK(cudaGetLastError());

@@ -471,8 +471,8 @@ void mamba2_scan(const at::Tensor& u, c10::optional<at::Tensor> z, c10::optional
   sglb::mamba2_scan(u.data_ptr<float>(), (int)u.stride(0), z.has_value() ? z->data_ptr() : nullptr, z.has_value() ? (int)z->stride(0) : 0,
                     fixed ? nullptr : dt_raw->data_ptr(), fixed ? 0 : (int)dt_raw->stride(0), in_bf16,
                     fixed ? nullptr : dt_bias->data_ptr<float>(), fixed ? nullptr : A_log->data_ptr<float>(), opt_ptr<float>(D),
-                    state.data_ptr<float>(), req_slots.data_ptr<int>(), seq_lens.data_ptr<int>(), opt_ptr<int>(cu_q), B, (int)H, (int)P, (int)N, (int)G,
-                    out.data_ptr<float>(), opt_ptr<float>(decay), opt_ptr<float>(gates), gates.has_value() ? (int)gates->size(2) : 0, cur_stream());
+                    state.data_ptr<float>(), req_slots.data_ptr<int>(), seq_lens.data_ptr<int>(), opt_ptr<int>(cu_q), B, (int)u.size(0), (int)H, (int)P, (int)N,
+                    (int)G, out.data_ptr<float>(), opt_ptr<float>(decay), opt_ptr<float>(gates), gates.has_value() ? (int)gates->size(2) : 0, cur_stream());
   count();
 }
 
@@ -1187,8 +1187,18 @@ void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::
   c10::cuda::CUDAGuard g(x.device());
   auto stream = cur_stream();
   const int pairs = T * K;
-  const int max_tiles = (pairs + 127) / 128 + E;
-  const int cap = max_tiles * 128;
+  // Up to 64 rows an expert on average the block is bound by the weights: rows become the narrow operand (gemm_grouped_decode.cu) in tiles that hold
+  // twice the average, so that few experts need a second one; beyond, 128-row tiles (gemm_tc.cu), whose two token tiles an expert read its weights once.
+  const bool decode = pairs <= 64ll * E;
+  int tile = 128;
+  if (decode)
+    for (int t : {16, 32, 64, 128}) {
+      tile = t;
+      if (2ll * pairs <= (long long)t * E) break;
+    }
+  const int max_tiles = pairs / tile + std::min(E, pairs);
+  const int live_tiles = std::max(1, std::min(max_tiles, std::min(E, pairs)));
+  const int cap = max_tiles * tile;
   auto i32 = x.options().dtype(at::kInt);
   auto meta = at::empty({cap + pairs + max_tiles + 1}, i32);
   int* sorted_row = meta.data_ptr<int>();
@@ -1196,34 +1206,39 @@ void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::
   int* tile_expert = inv_pos + pairs;
   int* num_tiles = tile_expert + max_tiles;
   auto row_w = at::empty({cap}, x.options().dtype(at::kFloat));
-  sglb::moe_align(topk_ids.data_ptr<int>(), topk_w.data_ptr<float>(), pairs, E, (int)expert_offset, sorted_row, inv_pos,
+  sglb::moe_align(topk_ids.data_ptr<int>(), topk_w.data_ptr<float>(), pairs, E, (int)expert_offset, tile, sorted_row, inv_pos,
                   row_w.data_ptr<float>(), tile_expert, num_tiles, max_tiles, stream);
   auto xs = at::empty({cap, H}, x.options());
-  sglb::moe_gather(x.data_ptr(), sorted_row, num_tiles, xs.data_ptr(), H, (int)x.stride(0), K, cap, num_sms(), stream,
+  sglb::moe_gather(x.data_ptr(), sorted_row, num_tiles, xs.data_ptr(), H, (int)x.stride(0), K, cap, tile, stream,
                    weight_input ? row_w.data_ptr<float>() : nullptr);
+  enum { NONE = 0, SILU = 1, ROWSCALE = 2, RELU2 = 3 };
+  auto product = [&](const at::Tensor& a, const at::Tensor& w, at::Tensor& c, int n_out, int k, int epi) {
+    if (decode)
+      sglb::gemm_grouped_decode(a.data_ptr(), w.data_ptr(), c.data_ptr(), row_w.data_ptr<float>(), sorted_row, tile, n_out, k, k, n_out, E, tile_expert,
+                                num_tiles, max_tiles, live_tiles, epi, num_sms(), stream);
+    else
+      sglb::gemm_bf16_tc_grouped(a.data_ptr(), w.data_ptr(), c.data_ptr(), epi == ROWSCALE ? row_w.data_ptr<float>() : nullptr, cap, n_out, k, k, n_out, E,
+                                 tile_expert, num_tiles, epi == SILU, num_sms(), stream, epi == RELU2);
+  };
   auto h = at::empty({cap, I}, x.options());
   if (act == 0) {
-    sglb::gemm_bf16_tc_grouped(xs.data_ptr(), w13.data_ptr(), h.data_ptr(), nullptr, cap, I, H, H, I, E, tile_expert, num_tiles, true,
-                               num_sms(), stream);
+    product(xs, w13, h, I, H, SILU);
   } else if (act == 2) {
-    sglb::gemm_bf16_tc_grouped(xs.data_ptr(), w13.data_ptr(), h.data_ptr(), nullptr, cap, I, H, H, I, E, tile_expert, num_tiles, false, num_sms(), stream,
-                               true);
+    product(xs, w13, h, I, H, RELU2);
   } else {
     // clamped GLU: the gate|up block comes out of the grouped GEMM whole, the activation is its own (vectorised) pass
     auto h2 = at::empty({cap, 2 * I}, x.options());
-    sglb::gemm_bf16_tc_grouped(xs.data_ptr(), w13.data_ptr(), h2.data_ptr(), nullptr, cap, 2 * I, H, H, 2 * I, E, tile_expert, num_tiles, false,
-                               num_sms(), stream);
+    product(xs, w13, h2, 2 * I, H, NONE);
     sglb::clamped_glu(h2.data_ptr(), h.data_ptr(), true, cap, I, act_limit, act_alpha, stream);
     count();
   }
   auto& ys = xs;   // the gathered inputs are dead once the first GEMM has run (same stream): reuse as the [cap, H] output
-  sglb::gemm_bf16_tc_grouped(h.data_ptr(), w2.data_ptr(), ys.data_ptr(), weight_input ? nullptr : row_w.data_ptr<float>(), cap, H, I, I, H, E,
-                             tile_expert, num_tiles, false, num_sms(), stream);
+  product(h, w2, ys, H, I, weight_input ? NONE : ROWSCALE);
   if (peer_slots) {
     sglb::moe_combine_push(ys.data_ptr(), inv_pos, nullptr, T, H, K, peer_slots, peer_flags, rank, world, epoch, done, num_sms(), stream);
   } else {
     TORCH_CHECK(out.has_value() && out->is_contiguous());
-    sglb::moe_combine(ys.data_ptr(), inv_pos, nullptr, out->data_ptr(), T, H, K, num_sms(), stream);
+    sglb::moe_combine(ys.data_ptr(), inv_pos, nullptr, out->data_ptr(), T, H, K, stream);
   }
   count(5);
 }

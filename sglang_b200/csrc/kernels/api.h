@@ -53,6 +53,10 @@ void gemm_bf16_tc_grouped(const void* A, const void* W, void* C, const float* ro
                           int ldc, int num_experts, const int* tile_expert, const int* num_m_tiles, bool split_silu, int num_sms,
                           cudaStream_t stream, bool relu2 = false);
 
+// gemm_grouped_decode.cu
+void gemm_grouped_decode(const void* X, const void* W, void* C, const float* row_scale, const int* sorted_row, int tile, int n_out, int K, int lda, int ldc,
+                         int E, const int* tile_expert, const int* num_tiles, int max_tiles, int live_tiles, int epi, int num_sms, cudaStream_t stream);
+
 // kvio.cu: device pool <-> pinned host pool page movers (HiCache L1 <-> L2), zero-copy over UVA, layer_first / page_first host layouts
 void kv_transfer_pages(void* dev, void* host_devptr, const int* dev_pages, const int* host_pages, int n, int planes, long long dev_plane_stride,
                        long long host_plane_stride, long long host_page_stride, int chunk_bytes, bool to_host, cudaStream_t stream);
@@ -83,12 +87,11 @@ void per_token_group_quant_fp8(const void* x, void* q, float* scales, int M, int
 // moe.cu
 void moe_topk_softmax(const void* logits, bool bf16, float* out_w, int* out_ids, int T, int E, int K, int stride, bool renorm,
                       cudaStream_t stream);
-void moe_align(const int* topk_ids, const float* topk_w, int n_pairs, int E, int expert_offset, int* sorted_row, int* inv_pos,
+void moe_align(const int* topk_ids, const float* topk_w, int n_pairs, int E, int expert_offset, int tile, int* sorted_row, int* inv_pos,
                float* row_w, int* tile_expert, int* num_tiles, int max_tiles, cudaStream_t stream);
 void moe_gather(const void* x, const int* sorted_row, const int* num_tiles, void* xs, int H, int x_stride, int K, int cap_rows,
-                int num_sms, cudaStream_t stream, const float* row_w = nullptr);
-void moe_combine(const void* ys, const int* inv_pos, const float* pair_w, void* out, int T, int H, int K, int num_sms,
-                 cudaStream_t stream);
+                int tile, cudaStream_t stream, const float* row_w = nullptr);
+void moe_combine(const void* ys, const int* inv_pos, const float* pair_w, void* out, int T, int H, int K, cudaStream_t stream);
 void moe_combine_push(const void* ys, const int* inv_pos, const float* pair_w, int T, int H, int K, const int64_t* peer_slot_ptrs,
                       const int64_t* peer_flag_ptrs, int rank, int world, const uint32_t* epoch_ptr, uint32_t* done_ctr, int num_sms,
                       cudaStream_t stream);
@@ -134,7 +137,7 @@ void causal_softmax(const float* scores, void* out, bool out_bf16, int rows, int
 void attention_sink_gate(const void* o, int ldo, const float* lse, const float* sinks, int rows, int H, int Dv, void* out, cudaStream_t stream);
 // mamba.cu (ragged Mamba-2 recurrence), residual_f32.cu (sandwich norms), elementwise.cu (bigram embedding), moe.cu (identity / shared experts)
 void mamba2_scan(const float* u, int ldu, const void* z, int ldz, const void* dt_raw, int lddt, bool bf16, const float* dt_bias, const float* A_log,
-                 const float* D, float* state, const int* req_slots, const int* seq_lens, const int* cu_q, int B, int H, int P, int N, int G, float* out,
+                 const float* D, float* state, const int* req_slots, const int* seq_lens, const int* cu_q, int B, int T, int H, int P, int N, int G, float* out,
                  const float* decay, const float* gates, int gstride, cudaStream_t stream);
 void mlstm_prepare(const void* proj, int ld, bool bf16, const float* raw, int T, int B, int H, int D, int Dv, float cap, float* mstate, const int* req_slots,
                    const int* seq_lens, const int* cu_q, float* u, float* gates, cudaStream_t stream);

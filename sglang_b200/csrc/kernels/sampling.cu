@@ -58,9 +58,8 @@ struct SampleParams {
 };
 
 // ---------------------------------------------------------------- the sampler: a cluster of eight CTAs per row
-// A row (V = 128 K: 256 KB of bf16) does not fit one SM's shared memory and one SM reads it slowly, so eight CTAs take an eighth each, keep it in
-// shared memory for every later pass, and exchange block results (maximum, sums, histogram segments) through distributed shared memory.  Every
-// thread reads only what it staged itself, 8 consecutive logits at a time, so the passes need no barrier between them.
+// Eight CTAs take an eighth of a row each (the batch's logits stay in L2 between passes) and exchange block results (maximum, sums, histogram segments)
+// through distributed shared memory.  A lane always takes 8 consecutive logits, a warp a contiguous range, so that index order survives everywhere.
 //
 // top-k / top-p: two-level histogram over d = (max - logit) / T (r = p / p_max = e^-d): 2048 bins of width 1/64 cover r down to e^-32, a second
 // 2048 bins refine the one that holds the boundary (7.6e-6 in d).  Shared-memory atomics are native for integers only (a float add is a
@@ -68,8 +67,13 @@ struct SampleParams {
 // in fixed point.  The fixed-point mass only nominates a bin; the masses before and inside it are then summed in fp32 and the nomination is moved
 // until they enclose the target.  Elements beyond d = 32 (masked ones, cold temperatures) meet in the last bin and are added up in registers.
 //
-// Measured (B200, bf16, rows asking in turn for greedy / nucleus / top-k / min-p / plain): 121 x 128256 2594 -> 69 us, 1 x 128256 (greedy) 11 us; the
-// version before kept one CTA per row, scalar loads and float atomics.
+// What can be kept is usually a handful of candidates: the threads' own maxima (2048 or 8192 of them) bound the boundary from below, one pass collects
+// what lies above that bound, and the first CTA alone finishes the row on that list without further cluster barriers.  A row whose list would not fit
+// (a broad nucleus, a large k) goes through the same steps on the whole row with all eight.
+//
+// Bound by the two passes over the row and a chain of about eight cluster barriers.  Measured (B200, bf16, rows asking in turn for greedy / nucleus /
+// top-k / min-p / plain): 121 x 128256 in 38 us, 256 in 62, one greedy row in 11; one CTA per row with scalar loads and float atomics took 2594 for
+// the 121, the cluster without candidate lists 69.
 constexpr int SAMP_CL = 8;              // CTAs per row: a portable cluster
 constexpr int SAMP_SEG = SAMP_BINS / SAMP_CL;
 
@@ -91,17 +95,21 @@ __device__ __forceinline__ uint32_t cl_ld(const void* p, uint32_t rank) {
   return v;
 }
 
+constexpr int SAMP_LIST = 1024;         // candidates the first CTA takes on alone
+
 template <int NW>
 struct SampShared {
   uint32_t slot[2][2][SAMP_CL];         // [parity][value][rank]: block results of a reduction
   uint32_t wred[2][NW];
   uint32_t hist[SAMP_BINS];
-  float seg_total[SAMP_CL], scan[SAMP_SEG / 32];
+  float seg_total[SAMP_CL], scan[NW];
   int hit;
   uint32_t cand_bin[SAMP_CL], cand_before[SAMP_CL];
-  uint32_t kept[SAMP_CL * NW];          // kept mass of every warp of the row
+  uint32_t kept[SAMP_CL * NW];          // kept mass of every warp of the row; before that, its candidates
   int pick;
   float pick_run, pick_u;
+  float own_d[SAMP_LIST], all_d[SAMP_LIST];      // candidates: of this CTA (an equal part per warp), of the row (first CTA)
+  int own_i[SAMP_LIST], all_i[SAMP_LIST];
 };
 
 __device__ __forceinline__ void samp_load8(const __nv_bfloat16* p, float (&v)[8]) {
@@ -114,23 +122,19 @@ __device__ __forceinline__ void samp_load8(const float* p, float (&v)[8]) {
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-// STAGED: the CTA's slice fits shared memory (V up to ~800 K bf16 / 400 K fp32); otherwise every pass reads the row again
-template <typename T, int NT, bool STAGED>
-__global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT) sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
-  constexpr int NW = NT / 32;
-  extern __shared__ __align__(16) uint8_t samp_dyn[];
+template <typename T, int NT>
+__global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT, NT == 256 ? 6 : 1)
+sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
+  constexpr int NW = NT / 32, WCAP = SAMP_LIST / NW;
   __shared__ SampShared<NW> sh;
   const int rank = (int)cl_rank(), row = blockIdx.x / SAMP_CL;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int V = p.V;
   const T* lr = logits + (size_t)row * p.stride;
-  const int slice = rank * NW * per_warp;                              // first logit of this CTA
-  const int w0 = slice + warp * per_warp, w1 = min(w0 + per_warp, V);  // this warp's contiguous range
-  T* stage = reinterpret_cast<T*>(samp_dyn);
+  const int w0 = (rank * NW + warp) * per_warp, w1 = min(w0 + per_warp, V);      // this warp's contiguous range
   const bool vec = (reinterpret_cast<uintptr_t>(lr) & 15) == 0;
 
   auto get8 = [&](int i, float (&v)[8]) {                              // 8 logits from i; those beyond the row are NaN (every comparison fails)
-    if (STAGED) { samp_load8(stage + (i - slice), v); return; }
     if (vec && i + 8 <= V) { samp_load8(lr + i, v); return; }
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = i + j < V ? to_f<T>(lr[i + j]) : __int_as_float(0x7fffffff);
@@ -152,36 +156,33 @@ __global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT) sample_ker
     par ^= 1;                                                          // (the next writers of this half have passed the next barrier)
   };
 
-  // ---- stage the slice, maximum and its lowest index (torch.argmax)
-  float mx = -INFINITY;
+  const float inv_t = 1.f / fmaxf(p.temperature[row], 1e-6f);
+  const int topk = p.top_k[row];
+  const bool greedy = topk == 1;
+  const float top_p = p.top_p[row], min_p = p.min_p[row];
+  const bool need_k = topk > 0 && topk < V, need_p = top_p < 1.f;
+  const bool need_z = p.out_logprobs || (!greedy && need_p && !need_k);
+
+  // ---- first pass: maximum, its lowest index (torch.argmax), and the partition sum over a running maximum
+  float mx = -INFINITY, z = 0.f;
   int am = 0x7fffffff;
-  if (STAGED) {
-    if (vec) {
-#pragma unroll 4
-      for (int i = w0 + lane * 8; i < w1; i += 256) {
-        T* dst = stage + (i - slice);
-        if (i + 8 <= V) {
-#pragma unroll
-          for (int k = 0; k < (int)sizeof(T) / 2; ++k) st128(dst + k * (16 / sizeof(T)), ldg128(lr + i + k * (16 / sizeof(T))));
-        } else {
-          for (int j = 0; j < 8; ++j) dst[j] = i + j < V ? lr[i + j] : T(__int_as_float(0x7fffffff));
-        }
-      }
-    } else {
 #pragma unroll 2
-      for (int i = w0 + lane * 8; i < w1; i += 256) {
-        T* dst = stage + (i - slice);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) dst[j] = i + j < V ? lr[i + j] : T(__int_as_float(0x7fffffff));
-      }
-    }
-  }
   for (int i = w0 + lane * 8; i < w1; i += 256) {
     float v[8];
     get8(i, v);
+    const float before = mx;
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       if (v[j] > mx) { mx = v[j]; am = i + j; }
+    if (need_z && mx > -INFINITY) {
+      if (mx > before) z *= __expf((before - mx) * inv_t);
+      if (i + 8 <= V) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) z += __expf((v[j] - mx) * inv_t);
+      } else {
+        for (int j = 0; i + j < V; ++j) z += __expf((to_f<T>(lr[i + j]) - mx) * inv_t);
+      }
+    }
   }
   const float own_max = mx;
 #pragma unroll
@@ -213,35 +214,11 @@ __global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT) sample_ker
   }
   if (arg == 0x7fffffff) arg = 0;                                      // a row without a finite logit
   par ^= 1;
-
-  const float inv_t = 1.f / fmaxf(p.temperature[row], 1e-6f);
-  const int topk = p.top_k[row];
-  const bool greedy = topk == 1;
-  const float top_p = p.top_p[row];
-  const bool need_k = topk > 0 && topk < V, need_p = top_p < 1.f;
-
-  // f(logit's d, its index offset) over this thread's valid logits
-  auto each = [&](auto&& f) {
-#pragma unroll 2
-    for (int i = w0 + lane * 8; i < w1; i += 256) {
-      float v[8];
-      get8(i, v);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f((gmax - v[j]) * inv_t);
-    }
-  };
   float Z = 0.f;
-  if (p.out_logprobs || (!greedy && need_p && !need_k)) {
-    float z = 0.f, unused = 0.f;
-    for (int i = w0 + lane * 8; i < w1; i += 256) {
-      float v[8];
-      get8(i, v);
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (i + j < V) z += __expf((v[j] - gmax) * inv_t);
-    }
-    reduce2(z, unused);
-    Z = z;
+  if (need_z) {
+    float unused = 0.f;
+    Z = own_max > -INFINITY ? z * __expf((own_max - gmax) * inv_t) : z;
+    reduce2(Z, unused);
   }
   auto finish = [&](int token) {
     p.out_tokens[row] = token;
@@ -252,12 +229,28 @@ __global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT) sample_ker
     if (rank == 0 && tid == 0) finish(arg);
     return;                            // (nobody reads this CTA's shared memory after the barrier above)
   }
+  // a seeded request draws from (its seed, ITS OWN output position): the stream does not depend on which step / row / batch it landed in
+  const bool own_seed = p.seeds && p.seeds[2 * row + 1] >= 0;
+  const long long step = p.step_ptr ? *p.step_ptr : p.step;
+  const float u01 = own_seed ? rng_uniform((unsigned long long)p.seeds[2 * row], 0ull, (unsigned long long)p.seeds[2 * row + 1])
+                             : rng_uniform(p.global_seed, (unsigned long long)row, (unsigned long long)step);
 
-  // ---- threshold in d: keep { d <= d_max }
+  // f(d) over this thread's logits
+  auto each = [&](auto&& f) {
+#pragma unroll 2
+    for (int i = w0 + lane * 8; i < w1; i += 256) {
+      float v[8];
+      get8(i, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f((gmax - v[j]) * inv_t);
+    }
+  };
   constexpr float W1 = 1.f / 64.f;
-  const float scale = fminf(16384.f, 4294967040.f / (float)V);
-  float d_max = INFINITY;
+  const float scale = fminf(16384.f, 4294967040.f / (float)V), inv_scale = 1.f / scale;
   auto bin1 = [](float d) { return min(SAMP_BINS - 1, (int)(d * (1.f / W1))); };
+  auto fixed_mass = [&](float d, int b) { return (uint32_t)(__expf(b * W1 - d) * scale + 0.5f); };
+  const auto count = [](int, uint32_t s) { return (float)s; };
+  const auto mass = [&](int bin, uint32_t s) { return (float)s * inv_scale * __expf(-bin * W1); };
   auto clear = [&]() {
     for (int i = tid; i < SAMP_BINS; i += NT) sh.hist[i] = 0;
     __syncthreads();
@@ -267,18 +260,18 @@ __global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT) sample_ker
     for (int o = 16; o > 0; o >>= 1) last += __shfl_xor_sync(0xffffffffu, last, o);
     if (lane == 0 && last) atomicAdd(&sh.hist[SAMP_BINS - 1], last);
   };
-  // first bin whose inclusive prefix reaches the target (SAMP_BINS: none does) and the exclusive prefix before it.  value(bin, sum) weighs a bin
-  auto find_bin = [&](float target, float& before, auto&& value) -> int {
+  // first bin whose inclusive prefix reaches the target (SAMP_BINS: none does) and the exclusive prefix before it.  value(bin, sum) weighs a bin.
+  // The row's histogram is the sum of the CTAs'; each scans a segment of it
+  auto find_row = [&](float target, float& before, auto&& value) -> int {
     if (tid == 0) sh.hit = SAMP_BINS;
     cl_sync();                                                         // every CTA's histogram is complete
-    float own = 0.f, li = 0.f;
+    float li = 0.f;
     const int bin = rank * SAMP_SEG + tid;
     if (tid < SAMP_SEG) {
       uint32_t s = 0;
 #pragma unroll
       for (int r = 0; r < SAMP_CL; ++r) s += cl_ld(&sh.hist[bin], r);
-      own = value(bin, s);
-      li = own;
+      li = value(bin, s);
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const float t = __shfl_up_sync(0xffffffffu, li, o);
@@ -317,109 +310,272 @@ __global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT) sample_ker
       if (sh.cand_bin[r] < SAMP_BINS) { found = (int)sh.cand_bin[r]; before = __uint_as_float(sh.cand_before[r]); }
     return found;
   };
-  // refine bin b1: the smallest d edge whose kept count / mass reaches ``target``, given what lies before the bin
-  auto refine = [&](int b1, float target, auto&& weigh) -> float {
-    const float lo = b1 * W1, far = b1 == SAMP_BINS - 1 ? d_max : fminf(d_max, lo + W1);
-    clear();
-    uint32_t last = 0;
-    each([&](float d) {
-      if (d >= lo && d <= far && bin1(d) == b1) {
-        const int b = min(SAMP_BINS - 1, (int)((d - lo) * (SAMP_BINS / W1)));
-        if (b == SAMP_BINS - 1) ++last;
-        else atomicAdd(&sh.hist[b], 1u);
+  // the same inside one CTA (BPT consecutive bins a thread)
+  auto find_list = [&](float target, float& before, auto&& value) -> int {
+    constexpr int BPT = SAMP_BINS / NT;
+    if (tid == 0) sh.hit = SAMP_BINS;
+    __syncthreads();                                                   // the histogram is complete
+    float v[BPT], own = 0.f;
+#pragma unroll
+    for (int k = 0; k < BPT; ++k) { v[k] = value(tid * BPT + k, sh.hist[tid * BPT + k]); own += v[k]; }
+    float li = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float t = __shfl_up_sync(0xffffffffu, li, o);
+      if (lane >= o) li += t;
+    }
+    if (lane == 31) sh.scan[warp] = li;
+    __syncthreads();
+    float base = 0.f;
+    for (int w = 0; w < warp; ++w) base += sh.scan[w];
+    const float prev = __shfl_up_sync(0xffffffffu, li, 1);
+    float run = base + (lane ? prev : 0.f);
+    const bool mine = base + li >= target && (run < target || tid == 0);
+    if (mine) atomicMin(&sh.hit, tid);
+    __syncthreads();
+    const int hit = sh.hit;
+    if (hit == SAMP_BINS) return SAMP_BINS;
+    if (tid == hit) {
+      int b = BPT - 1;
+      for (int k = 0; k < BPT; ++k) {
+        if (run + v[k] >= target) { b = k; break; }
+        if (k < BPT - 1) run += v[k];
       }
-    });
-    flush_last(last);
-    float before = 0.f;
-    const int b2 = find_bin(target, before, weigh);
-    if (b1 == SAMP_BINS - 1 && b2 >= SAMP_BINS - 1) return INFINITY;
-    return lo + (float)(min(b2, SAMP_BINS - 1) + 1) * (W1 / SAMP_BINS);
+      sh.cand_bin[0] = tid * BPT + b;
+      sh.cand_before[0] = __float_as_uint(run);
+    }
+    __syncthreads();
+    before = __uint_as_float(sh.cand_before[0]);
+    return (int)sh.cand_bin[0];
   };
-  float base_mass = Z;
-  if (need_k) {
-    // The k-th largest of the threads' own maxima bounds the k-th largest logit from below: 2048 of them (or 8192) are histogrammed first, and only
-    // what lies above that bound then meets the atomics, instead of the whole row
-    float dm = INFINITY;
-    const auto count = [](int, uint32_t s) { return (float)s; };
-    if (topk <= SAMP_CL * NT / 2) {
+  // d_max of the kept set { d <= d_max }, given that it lies within { d <= lim }; every thread gets the same.  Over the row or over the list
+  auto solve = [&](float lim, auto&& over, auto&& find, auto&& sums) -> float {
+    float d_max = INFINITY;
+    // refine bin b1: the smallest d edge whose kept count / mass reaches ``target``, given what lies before the bin
+    auto refine = [&](int b1, float target, auto&& weigh) -> float {
+      const float lo = b1 * W1, far = b1 == SAMP_BINS - 1 ? d_max : fminf(d_max, lo + W1);
       clear();
-      const float d = (gmax - own_max) * inv_t;
-      if (d >= 0.f) atomicAdd(&sh.hist[bin1(d)], 1u);
-      float unused = 0.f;
-      const int b = find_bin((float)topk, unused, count);
-      if (b < SAMP_BINS - 1) dm = (b + 1) * W1;
-    }
-    clear();
-    uint32_t last = 0;
-    each([&](float d) {
-      if (d >= 0.f && d <= dm) {
-        const int b = bin1(d);
-        if (b == SAMP_BINS - 1) ++last;
-        else atomicAdd(&sh.hist[b], 1u);
-      }
-    });
-    flush_last(last);
-    float before = 0.f;
-    const int b1 = find_bin((float)topk, before, count);
-    if (b1 < SAMP_BINS) d_max = refine(b1, (float)topk - before, count);
-    if (need_p) {
-      float m = 0.f, unused = 0.f;
-      const float edge = d_max;
-      each([&](float d) { if (d >= 0.f && d <= edge) m += __expf(-d); });
-      reduce2(m, unused);
-      base_mass = m;
-    }
-  }
-  if (need_p) {
-    const float target = top_p * base_mass;
-    const float dm = d_max;
-    // all logits of r below (1 - p) base / V together cannot reach the mass that is cut off: half of that bound keeps the broad tail out of the atomics
-    const float tail = 0.5f * (1.f - top_p) * base_mass / (float)V;
-    const float d_tail = tail > 0.f ? fminf(dm, -__logf(tail)) : dm;
-    clear();
-    uint32_t last = 0;
-    each([&](float d) {
-      if (d >= 0.f && d <= d_tail) {
-        const int b = bin1(d);
-        const uint32_t q = (uint32_t)(__expf(b * W1 - d) * scale + 0.5f);
-        if (b == SAMP_BINS - 1) last += q;
-        else atomicAdd(&sh.hist[b], q);
-      }
-    });
-    flush_last(last);
-    float before = 0.f;
-    const float inv_scale = 1.f / scale;
-    int b1 = find_bin(target, before, [&](int bin, uint32_t s) { return (float)s * inv_scale * __expf(-bin * W1); });
-    b1 = min(b1, SAMP_BINS - 1);
-    float m_before, m_in;
-    int moved = 0;                                                     // one direction only: rounding at an edge cannot make it swing
-    while (true) {                                                     // (the same numbers in every thread of the cluster)
-      m_before = m_in = 0.f;
-      const int b = b1;
-      const float far = b == SAMP_BINS - 1 ? dm : fminf(dm, (b + 1) * W1);
-      each([&](float d) {
-        if (d >= 0.f && d <= far) {
-          const int k = bin1(d);
-          if (k <= b) {
-            const float r = __expf(-d);
-            if (k < b) m_before += r;
-            else m_in += r;
-          }
+      uint32_t last = 0;
+      over([&](float d) {
+        if (d >= lo && d <= far && bin1(d) == b1) {
+          const int b = min(SAMP_BINS - 1, (int)((d - lo) * (SAMP_BINS / W1)));
+          if (b == SAMP_BINS - 1) ++last;
+          else atomicAdd(&sh.hist[b], 1u);
         }
       });
-      reduce2(m_before, m_in);
-      if (m_before >= target && b1 > 0 && moved <= 0) { moved = -1; --b1; continue; }
-      if (m_before + m_in < target && b1 < SAMP_BINS - 1 && moved >= 0) { moved = 1; ++b1; continue; }
-      break;
+      flush_last(last);
+      float before = 0.f;
+      const int b2 = find(target, before, weigh);
+      if (b1 == SAMP_BINS - 1 && b2 >= SAMP_BINS - 1) return INFINITY;
+      return lo + (float)(min(b2, SAMP_BINS - 1) + 1) * (W1 / SAMP_BINS);
+    };
+    float base_mass = Z;
+    if (need_k) {
+      clear();
+      uint32_t last = 0;
+      over([&](float d) {
+        if (d >= 0.f && d <= lim) {
+          const int b = bin1(d);
+          if (b == SAMP_BINS - 1) ++last;
+          else atomicAdd(&sh.hist[b], 1u);
+        }
+      });
+      flush_last(last);
+      float before = 0.f;
+      const int b1 = find((float)topk, before, count);
+      if (b1 < SAMP_BINS) d_max = refine(b1, (float)topk - before, count);
+      if (need_p) {
+        float m = 0.f, unused = 0.f;
+        const float edge = d_max;
+        over([&](float d) { if (d >= 0.f && d <= edge) m += __expf(-d); });
+        sums(m, unused);
+        base_mass = m;
+      }
     }
-    if (moved < 0 || m_before + m_in >= target)
-      d_max = fminf(d_max, refine(b1, target - m_before, [&](int b, uint32_t s) { return (float)s * __expf(-(b1 * W1 + (b + 0.5f) * (W1 / SAMP_BINS))); }));
-  }
-  // keep { r >= thr }, r = p / p_max
-  const float thr = d_max < INFINITY ? fmaxf(p.min_p[row], __expf(-d_max)) : p.min_p[row];
-  const float d_far = thr > 0.f ? -__logf(thr) + 0.01f : INFINITY;     // beyond it no r can reach thr: saves the exponential
+    if (need_p) {
+      const float target = top_p * base_mass;
+      const float dm = d_max, reach = fminf(dm, lim);
+      clear();
+      uint32_t last = 0;
+      over([&](float d) {
+        if (d >= 0.f && d <= reach) {
+          const int b = bin1(d);
+          const uint32_t q = fixed_mass(d, b);
+          if (b == SAMP_BINS - 1) last += q;
+          else atomicAdd(&sh.hist[b], q);
+        }
+      });
+      flush_last(last);
+      float before = 0.f;
+      int b1 = min(find(target, before, mass), SAMP_BINS - 1);
+      float m_before, m_in;
+      int moved = 0;                                                   // one direction only: rounding at an edge cannot make it swing
+      while (true) {                                                   // (the same numbers in every thread)
+        m_before = m_in = 0.f;
+        const int b = b1;
+        const float far = b == SAMP_BINS - 1 ? dm : fminf(dm, (b + 1) * W1);
+        over([&](float d) {
+          if (d >= 0.f && d <= far) {
+            const int k = bin1(d);
+            if (k <= b) {
+              const float r = __expf(-d);
+              if (k < b) m_before += r;
+              else m_in += r;
+            }
+          }
+        });
+        sums(m_before, m_in);
+        if (m_before >= target && b1 > 0 && moved <= 0) { moved = -1; --b1; continue; }
+        if (m_before + m_in < target && b1 < SAMP_BINS - 1 && moved >= 0) { moved = 1; ++b1; continue; }
+        break;
+      }
+      if (moved < 0 || m_before + m_in >= target)
+        d_max = fminf(d_max, refine(b1, target - m_before, [&](int b, uint32_t s) { return (float)s * __expf(-(b1 * W1 + (b + 0.5f) * (W1 / SAMP_BINS))); }));
+    }
+    return d_max;
+  };
+  // keep { r >= thr }, r = p / p_max; beyond d_far no r can reach thr, which saves the exponential
+  auto threshold = [&](float d_max) { return d_max < INFINITY ? fmaxf(min_p, __expf(-d_max)) : min_p; };
+  auto beyond = [](float thr) { return thr > 0.f ? -__logf(thr) + 0.01f : INFINITY; };
 
-  // ---- kept mass of every warp (index order), the warp that holds the drawn point, then the token inside it
+  float d_max = INFINITY;
+  if (need_k || need_p) {
+    // ---- a bound on the boundary: the k-th largest of the threads' own maxima, or the point where their mass alone reaches the nucleus; else what lies
+    // so low (r below (1 - p) / V of the mass, halved for rounding) that all of it together cannot reach the mass that is cut off
+    float lim = INFINITY;
+    const float od = (gmax - own_max) * inv_t;
+    if (need_k ? topk <= SAMP_CL * NT / 2 : true) {
+      clear();
+      if (od >= 0.f) {
+        const int b = bin1(od);
+        atomicAdd(&sh.hist[b], need_k ? 1u : fixed_mass(od, b));
+      }
+      float unused = 0.f;
+      const int b = need_k ? find_row((float)topk, unused, count) : find_row(top_p * Z * 1.0002f, unused, mass);
+      if (b < SAMP_BINS - 1) lim = (b + 1) * W1;
+    }
+    if (!need_k) {
+      const float tail = 0.5f * (1.f - top_p) * Z / (float)V;
+      if (tail > 0.f) lim = fminf(lim, -__logf(tail));
+    }
+    // ---- second pass: candidates { d <= lim } in index order, an equal part of the list per warp
+    int mine = 0;
+    for (int i0 = w0; i0 < w1; i0 += 256) {
+      const int i = i0 + lane * 8;
+      float d[8];
+      unsigned bits = 0;
+      if (i < w1) {
+        get8(i, d);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          d[j] = (gmax - d[j]) * inv_t;
+          if (d[j] >= 0.f && d[j] <= lim) bits |= 1u << j;
+        }
+      }
+      if (!__any_sync(0xffffffffu, bits)) continue;
+      int at = __popc(bits);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += t;
+      }
+      const int end = mine + __shfl_sync(0xffffffffu, at, 31);
+      at += mine - __popc(bits);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (bits >> j & 1) {
+          if (at < WCAP) { sh.own_d[warp * WCAP + at] = d[j]; sh.own_i[warp * WCAP + at] = i + j; }
+          ++at;
+        }
+      mine = end;
+      if (mine > WCAP) break;
+    }
+    if (lane < SAMP_CL) cl_st(&sh.kept[rank * NW + warp], lane, (uint32_t)(mine > WCAP ? SAMP_LIST + 1 : mine));
+    cl_sync();
+    int first = 0, total = 0;                                          // this warp's place in the row's list
+    for (int k = lane; k < SAMP_CL * NW; k += 32) {
+      const int c = min((int)sh.kept[k], SAMP_LIST + 1);
+      total += c;
+      if (k < rank * NW + warp) first += c;
+    }
+    first = warp_sum(first);
+    total = warp_sum(total);
+    if (total <= SAMP_LIST) {
+      __syncwarp();
+      for (int k = lane; k < mine; k += 32) {
+        cl_st(&sh.all_d[first + k], 0, __float_as_uint(sh.own_d[warp * WCAP + k]));
+        cl_st(&sh.all_i[first + k], 0, (uint32_t)sh.own_i[warp * WCAP + k]);
+      }
+      cl_sync();
+      if (rank != 0) return;
+      auto over = [&](auto&& f) {
+        for (int k = tid; k < total; k += NT) f(sh.all_d[k]);
+      };
+      auto sums = [&](float& a, float& b) {
+        a = warp_sum(a); b = warp_sum(b);
+        __syncthreads();
+        if (lane == 0) { sh.wred[0][warp] = __float_as_uint(a); sh.wred[1][warp] = __float_as_uint(b); }
+        __syncthreads();
+        a = b = 0.f;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) { a += __uint_as_float(sh.wred[0][w]); b += __uint_as_float(sh.wred[1][w]); }
+      };
+      const float thr = threshold(solve(lim, over, find_list, sums));
+      // an equal run of the list per thread, scanned in order
+      constexpr int PER = SAMP_LIST / NT;
+      float r[PER], own = 0.f;
+#pragma unroll
+      for (int k = 0; k < PER; ++k) {
+        const int e = tid * PER + k;
+        const float v = e < total ? __expf(-sh.all_d[e]) : -1.f;
+        r[k] = v >= thr && e < total ? v : 0.f;
+        own += r[k];
+      }
+      float li = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, li, o);
+        if (lane >= o) li += t;
+      }
+      __syncthreads();
+      if (lane == 31) sh.scan[warp] = li;
+      if (tid == 0) sh.hit = NT;
+      __syncthreads();
+      float base = 0.f, sum = 0.f;
+      for (int w = 0; w < NW; ++w) {
+        if (w == warp) base = sum;
+        sum += sh.scan[w];
+      }
+      const float u = u01 * sum;
+      const float prev = __shfl_up_sync(0xffffffffu, li, 1);
+      if (own > 0.f && base + li > u) atomicMin(&sh.hit, tid);
+      __syncthreads();
+      int hit = sh.hit;
+      if (hit == NT) {                                                 // rounding at the very end: the last kept candidate (or none: the maximum)
+        __syncthreads();
+        if (tid == 0) sh.hit = -1;
+        __syncthreads();
+        if (own > 0.f) atomicMax(&sh.hit, tid);
+        __syncthreads();
+        hit = sh.hit;
+      }
+      if (hit < 0) {
+        if (tid == 0) finish(arg);
+      } else if (tid == hit) {
+        float run = base + (lane ? prev : 0.f);
+        int e = -1;
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+          if (r[k] > 0.f && (e < 0 || !(run > u))) { e = tid * PER + k; run += r[k]; }
+        finish(sh.all_i[e]);
+      }
+      return;
+    }
+    d_max = solve(lim, each, find_row, reduce2);
+  }
+  const float thr = threshold(d_max), d_far = beyond(thr);
+
+  // ---- whole row: kept mass of every warp (index order), the warp that holds the drawn point, then the token inside it
   float cm = 0.f;
   each([&](float d) {
     if (d <= d_far) {
@@ -428,6 +584,7 @@ __global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT) sample_ker
     }
   });
   cm = warp_sum(cm);
+  if (need_k || need_p) cl_sync();                                     // (the candidate counts in ``kept`` have been read)
   if (lane < SAMP_CL) cl_st(&sh.kept[rank * NW + warp], lane, __float_as_uint(cm));
   cl_sync();
   if (warp == 0) {
@@ -442,11 +599,7 @@ __global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT) sample_ker
       if (lane >= o) incl += t;
     }
     const float total = __shfl_sync(0xffffffffu, incl, 31);
-    // a seeded request draws from (its seed, ITS OWN output position): the stream does not depend on which step / row / batch it landed in
-    const bool own = p.seeds && p.seeds[2 * row + 1] >= 0;
-    const long long step = p.step_ptr ? *p.step_ptr : p.step;
-    float u = (own ? rng_uniform((unsigned long long)p.seeds[2 * row], 0ull, (unsigned long long)p.seeds[2 * row + 1])
-                   : rng_uniform(p.global_seed, (unsigned long long)row, (unsigned long long)step)) * total;
+    float u = u01 * total;
     const float up = __shfl_up_sync(0xffffffffu, incl, 1);
     unsigned who = __ballot_sync(0xffffffffu, incl > u && s > 0.f);
     if (who == 0) {                                                    // rounding at the very end: the last kept logit
@@ -527,14 +680,7 @@ template <typename T, int NT>
 static void launch_sample(const void* logits, const SampleParams& p, int B, cudaStream_t stream) {
   constexpr int NW = NT / 32;
   const int per_warp = ((p.V + SAMP_CL * NW - 1) / (SAMP_CL * NW) + 255) / 256 * 256;
-  const size_t bytes = (size_t)per_warp * NW * sizeof(T);
-  if (bytes <= 200 * 1024) {
-    auto kern = sample_kernel<T, NT, true>;
-    if (bytes > 32 * 1024) SGLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    kern<<<B * SAMP_CL, NT, bytes, stream>>>((const T*)logits, p, per_warp);
-  } else {
-    sample_kernel<T, NT, false><<<B * SAMP_CL, NT, 0, stream>>>((const T*)logits, p, per_warp);
-  }
+  sample_kernel<T, NT><<<B * SAMP_CL, NT, 0, stream>>>((const T*)logits, p, per_warp);
   SGLB_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -545,8 +691,9 @@ void sample(const void* logits, bool bf16, int B, int V, int stride, const float
   if (B <= 0) return;
   SampleParams p{temperature, top_k, top_p, min_p, seeds, out_slots, next_token_buf, out_tokens, out_logprobs, global_seed,
                  step_ptr, step, V, stride};
-  // few rows: one CTA per SM, so its threads hide the latency alone; many rows: small CTAs, several per SM (the line is where the chip is full)
-  if (B <= 18) {
+  // few rows: one CTA per SM, so its threads hide the latency alone; more rows: small CTAs, several per SM (18 rows: 27 us with 1024 threads, 24 rows:
+  // 23 us with 256)
+  if (B <= 8) {
     if (bf16) launch_sample<__nv_bfloat16, 1024>(logits, p, B, stream);
     else launch_sample<float, 1024>(logits, p, B, stream);
   } else {

@@ -542,10 +542,11 @@ __global__ void __launch_bounds__(128) mamba2_scan_kernel(const Mamba2Params p) 
 //   y_t = (decay 0..t) C_t S  +  sum_{s <= t} (decay s+1..t) (C_t . B_s) dt_s x_s  + D x_t          S <- (decay of all) S + sum_s (decay s+1..7) dt_s B_s x_s^T
 // with the same fp32 sums in another order: two multiply-adds per element and token, packed two to an instruction, eight tokens per barrier pair.  The
 // decays are products of at most eight factors of the tokens' own (never quotients or exponentials of differences), so nothing cancels.
-// A CTA owns 64 columns of a head: lane l holds columns 2l, 2l + 1 of the N / 4 state rows of its warp, so that B and C are read from shared memory
-// as broadcasts (one wavefront per four values for 64 x 4 products) and the warps' partial read-outs meet in shared memory.
-// Bound by shared-memory wavefronts (about 1000 a block of tokens) and, for one long request, by the chain of blocks.
-// 3001 tokens in 5 requests, 64 heads of 64 x 128: 776 -> 649 us.
+// A CTA owns 64 columns of a head: lane l holds columns 2l, 2l + 1 of its warp's 16 state rows, B and C are read from shared memory as broadcasts and
+// the warps' partial read-outs meet there.  One more warp brings the next block and works out its steps and decays.
+// Bound by the chain of blocks of the longest request (about 2 us each: two barriers around dependent multiply-adds) and by what shared memory hands to
+// registers.  3001 tokens in 5 requests, 64 heads of 64 x 128: 776 us token by token, 585 us in blocks (649 with four warps of 32 rows that also did
+// the loading; 724 with 8 x 8 tiles in four warps, whose longer chains cost more than their fewer reads saved).
 typedef unsigned long long f2;
 __device__ __forceinline__ f2 f2_pack(float a, float b) {
   f2 r;
@@ -573,24 +574,72 @@ __device__ __forceinline__ void m2_cp16(float* dst, const float* src, bool valid
 }
 
 template <typename TZ, int N>
-__global__ void __launch_bounds__(128) mamba2_block_kernel(const Mamba2Params p) {
-  constexpr int L = 8, PC = 64, NW = N / 4, NP = NW / 2;      // tokens a block, columns of the CTA, state rows of a warp and their pairs
-  constexpr int RS = N + 4;                                   // padded row of B / C
+__global__ void __launch_bounds__(2 * N + 32, N == 128 ? 2 : 3) mamba2_block_kernel(const Mamba2Params p) {
+  constexpr int L = 8, PC = 64, NW = 16, NP = NW / 2, W = N / NW;      // tokens a block, columns of the CTA, state rows of a warp, their pairs, warps
+  constexpr int RS = N + 4, OT = W / 2;                       // padded row of B / C, output tokens the threads cover at once
+  constexpr int Q = W == 8 ? 4 : 2, TPW = L / W;              // parts a product C_t . B_s is cut into, tokens t of a warp there
   __shared__ __align__(16) float sB[2][L * RS], sC[2][L * RS], sX[2][L * PC];
-  __shared__ __align__(16) float sY[4][L * PC], sM[L * L], sDt[L], sDa[L];
+  __shared__ __align__(16) float sY[W][L * PC], sM[L * L], sDt[2][L], sDa[2][L];
   const int b = blockIdx.y;
   const int q0 = p.cu_q[b], n = p.cu_q[b + 1] - q0;
   if (n <= 0) return;
   const int h = blockIdx.x / p.pchunks, pc = blockIdx.x - h * p.pchunks;
   const int H = p.H, P = p.P, g = h / (H / p.G), inner = H * P;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool fixed = p.decay || p.gates;
-  const float a_exp = fixed ? 0.f : expf(p.A_log[h]);
-  const float dskip = p.D ? p.D[h] : 0.f;
-  const float dtb = fixed ? 0.f : p.dt_bias[h];
   const TZ* zg = reinterpret_cast<const TZ*>(p.z);
-  const TZ* dg = reinterpret_cast<const TZ*>(p.dt_raw);
 
+  if (warp == W) {
+    const bool fixed = p.decay || p.gates;
+    const float a_exp = fixed ? 0.f : expf(p.A_log[h]), dtb = fixed ? 0.f : p.dt_bias[h], fixed_decay = p.decay ? p.decay[h] : 0.f;
+    const TZ* dg = reinterpret_cast<const TZ*>(p.dt_raw);
+    float dt_in = 0.f, da_in = 0.f;
+    auto fetch = [&](int t0) {                                // raw step of token t0 + lane
+      if (lane >= L || t0 + lane >= n) return;
+      if (p.gates) {
+        const float* gt = p.gates + ((size_t)(q0 + t0 + lane) * H + h) * p.gstride;
+        da_in = gt[0];
+        dt_in = gt[1];
+      } else if (dg) dt_in = ld_f<TZ>(dg + (size_t)(q0 + t0 + lane) * p.lddt + h);
+    };
+    auto bring = [&](int t0, int buf) {
+      const float* row0 = p.u + (size_t)(q0 + t0) * p.ldu;
+#pragma unroll
+      for (int t = 0; t < L; ++t) {
+        const bool ok = t0 + t < n;
+        const float* row = row0 + (size_t)(ok ? t : 0) * p.ldu;
+        if (lane < N / 4) {
+          m2_cp16(&sB[buf][t * RS + lane * 4], row + inner + g * N + lane * 4, ok);
+          m2_cp16(&sC[buf][t * RS + lane * 4], row + inner + (p.G + g) * N + lane * 4, ok);
+        }
+        if (lane < PC / 4) m2_cp16(&sX[buf][t * PC + lane * 4], row + h * P + pc * PC + lane * 4, ok);
+      }
+      if (lane < L) {                                         // tokens beyond the end: step 0, decay 1, zero rows
+        float dt = 0.f, da = 1.f;
+        if (t0 + lane < n) {
+          dt = p.gates ? dt_in : p.decay ? 1.f : m2_softplus(dt_in + dtb);
+          da = p.gates ? da_in : p.decay ? fixed_decay : expf(-a_exp * dt);
+        }
+        sDt[buf][lane] = dt;
+        sDa[buf][lane] = da;
+      }
+    };
+    fetch(0);
+    bring(0, 0);
+    fetch(L);
+    int buf = 0;
+    for (int t0 = 0; t0 < n; t0 += L, buf ^= 1) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();                                        // block t0 is there; everyone is done with the block before it
+      if (t0 + L < n) {
+        bring(t0 + L, buf ^ 1);
+        fetch(t0 + 2 * L);
+      }
+      __syncthreads();
+    }
+    return;
+  }
+
+  const float dskip = p.D ? p.D[h] : 0.f;
   float* st = p.state + ((size_t)p.req_slots[b] * H + h) * N * P + (size_t)warp * NW * P + pc * PC + lane * 2;
   f2 S[NP][2];                                                // [row pair][column]
   const bool fresh = p.seq_lens[b] - n == 0;
@@ -604,68 +653,52 @@ __global__ void __launch_bounds__(128) mamba2_block_kernel(const Mamba2Params p)
     S[j][0] = f2_pack(r0.x, r1.x);
     S[j][1] = f2_pack(r0.y, r1.y);
   }
-
-  float dt_in = 0.f, da_in = 0.f;
-  auto issue = [&](int t0, int buf) {
-    const float* row0 = p.u + (size_t)(q0 + t0) * p.ldu;
+  const int op = tid & (PC - 1), ot = tid >> 6;               // this thread's outputs: column op of tokens ot, ot + OT, ...
+  float zz[L / OT];
+  auto gate = [&](int t0) {
 #pragma unroll
-    for (int k = 0; k < L * N / 4 / 128; ++k) {
-      const int i = tid + k * 128, t = i / (N / 4), c = (i % (N / 4)) * 4;
-      const bool ok = t0 + t < n;
-      const float* src = row0 + (size_t)(ok ? t : 0) * p.ldu + inner + g * N + c;
-      m2_cp16(&sB[buf][t * RS + c], src, ok);
-      m2_cp16(&sC[buf][t * RS + c], src + p.G * N, ok);
-    }
-    const int t = tid >> 4, c = (tid & 15) * 4;
-    const bool ok = t0 + t < n;
-    m2_cp16(&sX[buf][t * PC + c], row0 + (size_t)(ok ? t : 0) * p.ldu + h * P + pc * PC + c, ok);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    if (tid < L) {
-      const bool live = t0 + tid < n;
-      if (p.gates) {
-        const float* gt = p.gates + ((size_t)(q0 + t0 + tid) * H + h) * p.gstride;
-        da_in = live ? gt[0] : 1.f;
-        dt_in = live ? gt[1] : 0.f;
-      } else if (dg) dt_in = live ? ld_f<TZ>(dg + (size_t)(q0 + t0 + tid) * p.lddt + h) : 0.f;
-    }
+    for (int k = 0; k < L / OT; ++k)
+      zz[k] = zg && t0 + ot + OT * k < n ? ld_f<TZ>(zg + (size_t)(q0 + t0 + ot + OT * k) * p.ldz + h * P + pc * PC + op) : 0.f;
   };
-
-  issue(0, 0);
   int buf = 0;
   for (int t0 = 0; t0 < n; t0 += L, buf ^= 1) {
-    if (tid < L) {                                            // tokens beyond the end: step 0, decay 1, zero rows
-      const bool live = t0 + tid < n;
-      float dt = 0.f, da = 1.f;
-      if (live) {
-        dt = p.gates ? dt_in : p.decay ? 1.f : m2_softplus(dt_in + dtb);
-        da = p.gates ? da_in : p.decay ? p.decay[h] : expf(-a_exp * dt);
-      }
-      sDt[tid] = dt;
-      sDa[tid] = da;
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (t0 + L < n) issue(t0 + L, buf ^ 1);                   // (its last readers have passed the barrier above)
+    gate(t0);                                                 // (needed at the end of the block)
     const float* B = sB[buf];
     const float* C = sC[buf];
     const float* X = sX[buf];
-    const int op = tid & (PC - 1), ot = tid >> 6;             // this thread's outputs: column op of tokens ot, ot + 2, ...
-    float zz[L / 2];
+    // read-out of the state before the block: this warp's rows, sixteen independent chains
+    f2 y[L][2];
 #pragma unroll
-    for (int k = 0; k < L / 2; ++k)
-      zz[k] = zg && t0 + ot + 2 * k < n ? ld_f<TZ>(zg + (size_t)(q0 + t0 + ot + 2 * k) * p.ldz + h * P + pc * PC + op) : 0.f;
+    for (int t = 0; t < L; ++t) y[t][0] = y[t][1] = 0;
+#pragma unroll
+    for (int j = 0; j < NP; j += 2) {
+#pragma unroll
+      for (int t = 0; t < L; ++t) {
+        const ulonglong2 cv = *reinterpret_cast<const ulonglong2*>(C + t * RS + warp * NW + 2 * j);
+        y[t][0] = f2_fma(cv.x, S[j][0], y[t][0]);
+        y[t][1] = f2_fma(cv.x, S[j][1], y[t][1]);
+        y[t][0] = f2_fma(cv.y, S[j + 1][0], y[t][0]);
+        y[t][1] = f2_fma(cv.y, S[j + 1][1], y[t][1]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < L; ++t) {
+      const float2 a = f2_get(y[t][0]), c = f2_get(y[t][1]);
+      *reinterpret_cast<float2*>(&sY[warp][t * PC + lane * 2]) = make_float2(a.x + a.y, c.x + c.y);
+    }
     float da[L], dt[L];
 #pragma unroll
     for (int i = 0; i < L; i += 4) {
-      *reinterpret_cast<float4*>(da + i) = *reinterpret_cast<const float4*>(sDa + i);
-      *reinterpret_cast<float4*>(dt + i) = *reinterpret_cast<const float4*>(sDt + i);
+      *reinterpret_cast<float4*>(da + i) = *reinterpret_cast<const float4*>(sDa[buf] + i);
+      *reinterpret_cast<float4*>(dt + i) = *reinterpret_cast<const float4*>(sDt[buf] + i);
     }
     {
-      // M[t][s] = (C_t . B_s) (decay s+1..t) dt_s: two tokens t a warp, a lane per (t, s, half of the rows)
-      const int s = lane & 7, t = 2 * warp + ((lane >> 3) & 1), n0 = (lane >> 4) * (N / 2);
+      // M[t][s] = (C_t . B_s) (decay s+1..t) dt_s: a lane per (t, s, part of the rows); the parts take turns at four values, so no bank serves two
+      const int s = lane & 7, t = TPW * warp + (TPW == 2 ? (lane >> 3) & 1 : 0), n0 = (TPW == 2 ? lane >> 4 : lane >> 3) * 4;
       f2 acc0 = 0, acc1 = 0;
 #pragma unroll
-      for (int i = 0; i < N / 2; i += 4) {
+      for (int i = 0; i < N; i += 4 * Q) {
         const ulonglong2 cv = *reinterpret_cast<const ulonglong2*>(C + t * RS + n0 + i), bv = *reinterpret_cast<const ulonglong2*>(B + s * RS + n0 + i);
         acc0 = f2_fma(cv.x, bv.x, acc0);
         acc1 = f2_fma(cv.y, bv.y, acc1);
@@ -673,29 +706,14 @@ __global__ void __launch_bounds__(128) mamba2_block_kernel(const Mamba2Params p)
       const float2 a = f2_get(acc0), c = f2_get(acc1);
       float m = (a.x + a.y) + (c.x + c.y);
       m += __shfl_xor_sync(0xffffffffu, m, 16);
+      if (TPW == 1) m += __shfl_xor_sync(0xffffffffu, m, 8);
       float w = 0.f;
 #pragma unroll
       for (int i = 0; i < L; ++i) {
         if (i == s) w = dt[i];
         if (i > s && i <= t) w *= da[i];
       }
-      if (lane < 16) sM[t * L + s] = s <= t ? m * w : 0.f;
-    }
-    // read-out of the state before the block: this warp's rows
-#pragma unroll
-    for (int t = 0; t < L; ++t) {
-      f2 y0 = 0, y1 = 0;
-      const float* ct = C + t * RS + warp * NW;
-#pragma unroll
-      for (int j = 0; j < NP; j += 2) {
-        const ulonglong2 cv = *reinterpret_cast<const ulonglong2*>(ct + 2 * j);
-        y0 = f2_fma(cv.x, S[j][0], y0);
-        y1 = f2_fma(cv.x, S[j][1], y1);
-        y0 = f2_fma(cv.y, S[j + 1][0], y0);
-        y1 = f2_fma(cv.y, S[j + 1][1], y1);
-      }
-      const float2 a = f2_get(y0), c = f2_get(y1);
-      *reinterpret_cast<float2*>(&sY[warp][t * PC + lane * 2]) = make_float2(a.x + a.y, c.x + c.y);
+      if (lane < 8 * TPW) sM[t * L + s] = s <= t ? m * w : 0.f;
     }
     // state after the block
     float suffix = 1.f;
@@ -710,11 +728,11 @@ __global__ void __launch_bounds__(128) mamba2_block_kernel(const Mamba2Params p)
     }
     const f2 all = f2_pack(suffix, suffix);
 #pragma unroll
-    for (int j = 0; j < NP; j += 2) {
+    for (int j = 0; j < NP; ++j) { S[j][0] = f2_mul(S[j][0], all); S[j][1] = f2_mul(S[j][1], all); }
 #pragma unroll
-      for (int i = 0; i < 2; ++i) { S[j + i][0] = f2_mul(S[j + i][0], all); S[j + i][1] = f2_mul(S[j + i][1], all); }
+    for (int t = 0; t < L; ++t) {
 #pragma unroll
-      for (int t = 0; t < L; ++t) {
+      for (int j = 0; j < NP; j += 2) {
         const ulonglong2 bv = *reinterpret_cast<const ulonglong2*>(B + t * RS + warp * NW + 2 * j);
         S[j][0] = f2_fma(bv.x, wx[t][0], S[j][0]);
         S[j][1] = f2_fma(bv.x, wx[t][1], S[j][1]);
@@ -730,15 +748,19 @@ __global__ void __launch_bounds__(128) mamba2_block_kernel(const Mamba2Params p)
 #pragma unroll
     for (int t = 0; t < L; ++t) {
       cum *= da[t];
-      if ((t & 1) != ot) continue;
-      float y = (sY[0][t * PC + op] + sY[1][t * PC + op]) + (sY[2][t * PC + op] + sY[3][t * PC + op]);
-      y *= cum;
+      if (t % OT != ot) continue;
+      float v[W], o = 0.f;
 #pragma unroll
-      for (int s = 0; s <= t; ++s) y += sM[t * L + s] * x[s];
-      y += dskip * x[t];
+      for (int w = 0; w < W; ++w) v[w] = sY[w][t * PC + op];
+#pragma unroll
+      for (int w = 0; w < W; w += 2) o += v[w] + v[w + 1];
+      o *= cum;
+#pragma unroll
+      for (int s = 0; s <= t; ++s) o += sM[t * L + s] * x[s];
+      o += dskip * x[t];
       if (t0 + t < n) {
-        if (zg) { const float z = zz[t >> 1]; y *= z / (1.f + expf(-z)); }
-        p.out[(size_t)(q0 + t0 + t) * inner + h * P + pc * PC + op] = y;
+        if (zg) { const float z = zz[t / OT]; o *= z / (1.f + expf(-z)); }
+        p.out[(size_t)(q0 + t0 + t) * inner + h * P + pc * PC + op] = o;
       }
     }
   }
@@ -774,14 +796,14 @@ void launch_m2(const Mamba2Params& p, int B, cudaStream_t stream) {
 template <typename TZ>
 void dispatch_m2(const Mamba2Params& p, int B, int T, cudaStream_t stream) {
   const int N = p.N;
-  // Prompts (two tokens a request and more on average) of the widths whose state rows divide among four warps; rows have to be readable 16 bytes at a
+  // Prompts (two tokens a request and more on average) of state sizes 64 and 128; rows have to be readable 16 bytes at a
   // time.  A single decode token is state traffic, where the token-by-token kernel's smaller CTAs do as well.
   if (p.cu_q && T >= 2 * B && (N == 64 || N == 128) && p.P % 64 == 0 && p.ldu % 4 == 0 && reinterpret_cast<uintptr_t>(p.u) % 16 == 0 &&
       reinterpret_cast<uintptr_t>(p.state) % 8 == 0) {
     Mamba2Params q = p;
     q.pchunks = p.P / 64;
-    if (N == 64) mamba2_block_kernel<TZ, 64><<<dim3(p.H * q.pchunks, B), 128, 0, stream>>>(q);
-    else mamba2_block_kernel<TZ, 128><<<dim3(p.H * q.pchunks, B), 128, 0, stream>>>(q);
+    if (N == 64) mamba2_block_kernel<TZ, 64><<<dim3(p.H * q.pchunks, B), 2 * 64 + 32, 0, stream>>>(q);
+    else mamba2_block_kernel<TZ, 128><<<dim3(p.H * q.pchunks, B), 2 * 128 + 32, 0, stream>>>(q);
     SGLB_CUDA_CHECK(cudaGetLastError());
     return;
   }

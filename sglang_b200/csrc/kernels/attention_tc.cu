@@ -96,6 +96,7 @@ struct AttnParams {
   int causal, window;
   // persistent variant: work items = the (x, y, z) cells of the classic grid, handed out by an atomic counter
   int gx, gy, total_items;
+  int pairs;                  // two-tile kernel: items below are pairs of query tiles, two items each beyond are their single tiles
   int* sched;         // [0] next item, [1] CTAs finished (the last one resets both: graph-replay safe)
   const float* slopes;        // optional [Hq]: distance bias, score -= slopes[h] * (query position - key position), applied after the cap
   const float* log_rates;     // optional [Hq], with slopes: the bias is slopes[h] * ln(1 + log_rates[h] * distance) instead of linear (no cap)
@@ -929,23 +930,35 @@ attn_fwd_tc_persist_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
   }
 }
 
-// merge split-KV partials: one warp per (token, head) row
-__global__ void attn_merge_splits_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
-                                         __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out, int rows,
-                                         int num_splits) {
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+// merge split-KV partials: one warp per (token, head) row; the partials of eight splits are in flight together (the launch is latency: 6.0 -> 3.2 us
+// at 192 rows of 7 splits)
+__global__ void __launch_bounds__(128) attn_merge_splits_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
+                                                                __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out, int rows,
+                                                                int num_splits) {
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
+  constexpr int S = 8;
   float m = -INFINITY;
-  for (int s = 0; s < num_splits; ++s) m = fmaxf(m, part_lse[(size_t)s * rows + row]);
+  for (int s = lane; s < num_splits; s += 32) m = fmaxf(m, part_lse[(size_t)s * rows + row]);
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   float wsum = 0.f;
-  for (int s = 0; s < num_splits; ++s) {
-    const float l = part_lse[(size_t)s * rows + row];
-    const float w = (l == -INFINITY) ? 0.f : __expf(l - m);
-    wsum += w;
-    const float4 v = *reinterpret_cast<const float4*>(part_o + ((size_t)s * rows + row) * ATT_D + lane * 4);
-    acc[0] += w * v.x; acc[1] += w * v.y; acc[2] += w * v.z; acc[3] += w * v.w;
+  for (int s0 = 0; s0 < num_splits; s0 += S) {
+    float l[S];
+    float4 v[S];
+#pragma unroll
+    for (int k = 0; k < S; ++k) {
+      const bool ok = s0 + k < num_splits;
+      l[k] = ok ? part_lse[(size_t)(s0 + k) * rows + row] : -INFINITY;
+      v[k] = ok ? *reinterpret_cast<const float4*>(part_o + ((size_t)(s0 + k) * rows + row) * ATT_D + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (s0 == 0) m = warp_max(m);
+#pragma unroll
+    for (int k = 0; k < S; ++k) {
+      const float w = (l[k] == -INFINITY) ? 0.f : __expf(l[k] - m);
+      wsum += w;
+      acc[0] += w * v[k].x; acc[1] += w * v[k].y; acc[2] += w * v[k].z; acc[3] += w * v[k].w;
+    }
   }
   const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
   uint2 o;
@@ -987,12 +1000,371 @@ __global__ void attn_merge_splits_diff_kernel(const float* __restrict__ part_o, 
     if (lane * 4 + i < d.dv) out[(size_t)pair * d.dv + lane * 4 + i] = __float2bfloat16(o[i] * mul);
 }
 
+// ---------------------------------------------------------------- prompts: two query tiles a CTA
+// The persistent kernel above gives a key tile one warpgroup whose soft-max (128 exponentials a thread, 1024 cycles of the special-function unit alone)
+// and whose products (1024 cycles of UMMA) follow one another, with only the next S overlapped: 2100 cycles a tile.  Here a CTA owns two neighbouring
+// 128-row tiles of the same KV head; while one warpgroup works out its probabilities, the tensor core runs the other's P.V and Q.K^T, and both read the
+// same K and V tiles, so the two units are busy at once and every key tile is fetched once for 256 rows.
+//
+//   warp 0 : scheduler + TMA producer      warp 1 : MMA issuer, one thread      warps 4..7 / 8..11 : soft-max + epilogue of tile A / B
+//   TMEM   : S_A | S_B | O_A | O_B (128 columns each); P overwrites its S.  S(j + 1) is issued behind P(j).V(j), which has read P by then (products of
+//            one thread run in the order of issue)
+//   shared : Q 64 KB, two stages of K and V
+// Plain scores only (no cap, bias, window, chunk, tree or splits).  Same arithmetic in the same order per row as the kernel above.
+// Measured: 4096 queries, 32 + 8 heads, at the end of 15011 keys: 1119 -> 956 us; 17 prompts of
+// 68 to 886 tokens (5003): 121 -> 79 us.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+constexpr int ATT2_THREADS = 384;
+constexpr int ATT2_SMEM_BYTES = 2 * ATT_TILE_BYTES + 4 * ATT_TILE_BYTES + 1024 + 256;
+
+__global__ void __launch_bounds__(ATT2_THREADS, 1)
+attn_fwd_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                        const AttnParams p) {
+  constexpr int KT = 128;
+  const int G = p.G, TQ = 128 / G;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sQ = smem;                               // [2 tiles]
+  uint8_t* sK = smem + 2 * ATT_TILE_BYTES;          // [2 stages]
+  uint8_t* sV = smem + 4 * ATT_TILE_BYTES;          // [2 stages]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 6 * ATT_TILE_BYTES);
+  uint64_t* q_full = bars;
+  uint64_t* q_empty = bars + 1;
+  uint64_t* k_full = bars + 2;       // [2 stages]
+  uint64_t* k_empty = bars + 4;
+  uint64_t* v_full = bars + 6;
+  uint64_t* v_empty = bars + 8;
+  uint64_t* s_full = bars + 10;      // [2 tiles]
+  uint64_t* p_full = bars + 12;
+  uint64_t* o_done = bars + 14;      // every P.V (lazy-rescale hand-off)
+  uint64_t* o_final = bars + 16;     // the last P.V of an item
+  uint64_t* o_free = bars + 18;      // the epilogue has read O
+  uint64_t* item_full = bars + 20;   // [2]
+  uint64_t* item_empty = bars + 22;  // [2]
+  volatile int* s_item = reinterpret_cast<volatile int*>(bars + 24);   // [2]
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 25);
+
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
+    mbar_init(q_full, 1); mbar_init(q_empty, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); mbar_init(&o_done[i], 1); mbar_init(&o_final[i], 1); mbar_init(&o_free[i], 4);
+      mbar_init(&item_full[i], 1); mbar_init(&item_empty[i], 9);       // MMA thread + 8 soft-max warps
+    }
+    fence_barrier_init();
+  }
+  if (warp == 1) { tmem_alloc(tmem_ptr, 512); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_ptr;
+
+  struct Item { int b, kvh, t0, q_start, q_len, seq_len, prefix, n_tiles; bool valid, both; };
+  auto decode_item = [&](int idx) {                  // pure function of the item's number: every role works it out for itself
+    Item it;
+    const int pair = idx < p.pairs ? idx : p.pairs + (idx - p.pairs) / 2, single = idx < p.pairs ? -1 : (idx - p.pairs) & 1;
+    const int x = p.gx - 1 - (pair % p.gx);          // longest (latest) query tiles of a request first
+    it.kvh = (pair / p.gx) % p.gy;
+    it.b = pair / (p.gx * p.gy);
+    it.q_start = p.cu_q[it.b];
+    it.q_len = p.cu_q[it.b + 1] - it.q_start;
+    it.seq_len = p.seq_lens[it.b];
+    it.prefix = it.seq_len - it.q_len;
+    it.t0 = x * 2 * TQ + (single > 0 ? TQ : 0);
+    it.valid = it.t0 < it.q_len;
+    it.both = single < 0 && it.t0 + TQ < it.q_len;
+    const int kv_hi = p.causal ? min(it.seq_len, it.prefix + min(it.t0 + (single < 0 ? 2 : 1) * TQ, it.q_len)) : it.seq_len;
+    it.n_tiles = it.valid ? (kv_hi + KT - 1) / KT : 0;
+    return it;
+  };
+
+  if (warp < 4) {
+    if (warp == 0 && lane == 0) {
+      // ------------------------------------------------------------ scheduler + producer
+      uint32_t n_it = 0, n_q = 0, g = 0;
+      for (;;) {
+        const int slot = n_it & 1;
+        mbar_wait(&item_empty[slot], ((n_it >> 1) & 1) ^ 1);
+        const int idx = atomicAdd(p.sched, 1);
+        s_item[slot] = idx;
+        mbar_arrive(&item_full[slot]);
+        ++n_it;
+        if (idx >= p.total_items) break;
+        const Item it = decode_item(idx);
+        if (it.n_tiles == 0) continue;
+        mbar_wait(q_empty, (n_q & 1) ^ 1);
+        mbar_expect_tx(q_full, it.both ? 2 * ATT_TILE_BYTES : ATT_TILE_BYTES);
+        for (int i = 0; i < (it.both ? 2 : 1); ++i) {
+          tma_load_4d(sQ + i * ATT_TILE_BYTES, &tmQ, q_full, 0, 0, it.kvh, it.q_start + it.t0 + i * TQ);
+          tma_load_4d(sQ + i * ATT_TILE_BYTES + ATT_HALF_BYTES, &tmQ, q_full, 64, 0, it.kvh, it.q_start + it.t0 + i * TQ);
+        }
+        ++n_q;
+        const int ps = p.page_size, pages_per_tile = KT / ps;
+        const int* pt = p.page_table + (size_t)p.req_slots[it.b] * p.pt_stride;
+        for (int j = 0; j < it.n_tiles; ++j, ++g) {
+          const int st = g & 1;
+          const uint32_t ph = (g >> 1) & 1;
+          mbar_wait(&k_empty[st], ph ^ 1);
+          mbar_expect_tx(&k_full[st], ATT_TILE_BYTES);
+          for (int i = 0; i < pages_per_tile; ++i) {
+            const int page = pt[min(j * pages_per_tile + i, p.pt_stride - 1)];
+            uint8_t* dst = sK + st * ATT_TILE_BYTES + i * ps * 128;
+            tma_load_3d(dst, &tmK, &k_full[st], 0, it.kvh, page * ps);
+            tma_load_3d(dst + ATT_HALF_BYTES, &tmK, &k_full[st], 64, it.kvh, page * ps);
+          }
+          mbar_wait(&v_empty[st], ph ^ 1);
+          mbar_expect_tx(&v_full[st], ATT_TILE_BYTES);
+          for (int i = 0; i < pages_per_tile; ++i) {
+            const int page = pt[min(j * pages_per_tile + i, p.pt_stride - 1)];
+            uint8_t* dst = sV + st * ATT_TILE_BYTES + i * ps * 128;
+            tma_load_3d(dst, &tmV, &v_full[st], 0, it.kvh, page * ps);
+            tma_load_3d(dst + ATT_HALF_BYTES, &tmV, &v_full[st], 64, it.kvh, page * ps);
+          }
+        }
+      }
+    } else if (warp == 1 && lane == 0) {
+      // ------------------------------------------------------------ MMA issuer
+      constexpr uint32_t idesc_s = make_idesc(UMMA_BF16, UMMA_BF16, 128, KT, 0, 0);
+      constexpr uint32_t idesc_o = make_idesc(UMMA_BF16, UMMA_BF16, 128, ATT_D, 0, 1);
+      auto scores = [&](int tile, int st) {          // S_tile = Q_tile K^T
+        const uint32_t q_addr = smem_u32(sQ + tile * ATT_TILE_BYTES), k_addr = smem_u32(sK + st * ATT_TILE_BYTES);
+#pragma unroll
+        for (int k = 0; k < ATT_D / 16; ++k) {
+          const uint32_t off = (k >> 2) * ATT_HALF_BYTES + (k & 3) * 32;
+          umma_f16_ss(tmem + tile * KT, make_smem_desc_sw128(q_addr + off, 0, 1024), make_smem_desc_sw128(k_addr + off, 0, 1024), idesc_s, k != 0);
+        }
+        umma_commit(&s_full[tile]);
+      };
+      auto values = [&](int tile, int st, bool fresh) {      // O_tile (+)= P_tile V
+        const uint32_t v_addr = smem_u32(sV + st * ATT_TILE_BYTES);
+#pragma unroll
+        for (int k = 0; k < KT / 16; ++k)
+          umma_f16_ts(tmem + 2 * KT + tile * ATT_D, tmem + tile * KT + k * 8, make_smem_desc_sw128(v_addr + k * 2048, ATT_HALF_BYTES, 1024), idesc_o,
+                      !fresh || k != 0);
+        umma_commit(&o_done[tile]);
+      };
+      uint32_t n_it = 0, n_q = 0, n_qb = 0, g = 0, gb = 0;
+      for (;;) {
+        const int slot = n_it & 1;
+        mbar_wait(&item_full[slot], (n_it >> 1) & 1);
+        const int idx = s_item[slot];
+        mbar_arrive(&item_empty[slot]);
+        ++n_it;
+        if (idx >= p.total_items) break;
+        const Item it = decode_item(idx);
+        const int n = it.n_tiles;
+        if (n == 0) continue;
+        mbar_wait(q_full, n_q & 1);
+        mbar_wait(&k_full[g & 1], (g >> 1) & 1);
+        tc_fence_after();
+        scores(0, g & 1);
+        if (it.both) scores(1, g & 1);
+        umma_commit(&k_empty[g & 1]);
+        if (n == 1) umma_commit(q_empty);
+        for (int j = 0; j < n; ++j) {
+          const uint32_t gt = g + j;
+          const int st = gt & 1, nx = st ^ 1;
+          const bool more = j + 1 < n;
+          mbar_wait(&p_full[0], gt & 1);
+          mbar_wait(&v_full[st], (gt >> 1) & 1);
+          if (j == 0) mbar_wait(&o_free[0], (n_q & 1) ^ 1);            // the epilogue of the item before has read O
+          tc_fence_after();
+          values(0, st, j == 0);
+          if (!more) umma_commit(&o_final[0]);
+          if (more) {
+            mbar_wait(&k_full[nx], ((gt + 1) >> 1) & 1);
+            tc_fence_after();
+            scores(0, nx);
+          }
+          if (it.both) {
+            mbar_wait(&p_full[1], (gb + j) & 1);
+            if (j == 0) mbar_wait(&o_free[1], (n_qb & 1) ^ 1);
+            tc_fence_after();
+            values(1, st, j == 0);
+            if (!more) umma_commit(&o_final[1]);
+          }
+          umma_commit(&v_empty[st]);
+          if (more) {
+            if (it.both) scores(1, nx);
+            umma_commit(&k_empty[nx]);
+            if (j + 2 == n) umma_commit(q_empty);
+          }
+        }
+        g += n;
+        ++n_q;
+        if (it.both) { gb += n; ++n_qb; }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ soft-max + epilogue
+    const int tile = (warp - 4) >> 2, q = warp & 3;
+    const int r = (q << 5) + lane;
+    const uint32_t lane_addr = (uint32_t)(q << 5) << 16;
+    const uint32_t s_addr = tmem + lane_addr + tile * KT, o_addr = tmem + lane_addr + 2 * KT + tile * ATT_D;
+    const float scale_log2 = p.scale_log2;
+    uint32_t n_it = 0, n_q = 0, g = 0;
+    for (;;) {
+      const int slot = n_it & 1;
+      mbar_wait(&item_full[slot], (n_it >> 1) & 1);
+      const int idx = s_item[slot];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&item_empty[slot]);
+      ++n_it;
+      if (idx >= p.total_items) break;
+      const Item it = decode_item(idx);
+      if (!it.valid || (tile && !it.both) || it.n_tiles == 0) continue;
+      const int t0 = it.t0 + tile * TQ, tok = t0 + r / G;
+      const bool row_valid = tok < it.q_len, warp_valid = (t0 + (q << 5) / G) < it.q_len;
+      const int q_pos = it.prefix + tok;
+      const int kv_last = p.causal ? min(it.seq_len - 1, q_pos) : it.seq_len - 1;
+      const int clear_to = p.causal ? min(it.prefix + t0 + 1, it.seq_len) : it.seq_len;      // keys below are visible to every row of the tile
+      float m_i = -INFINITY, l_i = 0.f;
+      for (int j = 0; j < it.n_tiles; ++j) {
+        const uint32_t gt = g + j;
+        mbar_wait(&s_full[tile], gt & 1);
+        tc_fence_after();
+        if (warp_valid) {
+          // Columns 64..127 are read twice instead of held: twelve warps share the registers.  P (64 columns) takes the place of S columns that have been
+          // turned into it
+          const int kv0 = j * KT;
+          const bool need_mask = kv0 + KT > clear_to;
+          const int hi = kv_last - kv0;
+          uint32_t x[32], y[32];
+          float mxs[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // (an instruction takes two values into a running maximum)
+          auto mask = [&](uint32_t (&v)[32], int c0) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (c0 + i > hi) v[i] = __float_as_uint(-INFINITY);
+          };
+          auto largest = [&](const uint32_t (&v)[32]) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) mxs[(i >> 1) & 3] = max3(mxs[(i >> 1) & 3], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+          };
+          tmem_ld_32x32b_x32(s_addr + 64, x);
+          tmem_ld_32x32b_x32(s_addr + 96, y);
+          tmem_ld_wait();
+          if (need_mask) { mask(x, 64); mask(y, 96); }
+          largest(x);
+          largest(y);
+          tmem_ld_32x32b_x32(s_addr, x);
+          tmem_ld_32x32b_x32(s_addr + 32, y);
+          tmem_ld_wait();
+          if (need_mask) { mask(x, 0); mask(y, 32); }
+          largest(x);
+          largest(y);
+          const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])) * scale_log2;
+          const float m_new = fmaxf(m_i, mx);
+          const bool need = j > 0 && m_new > m_i + ATT_RESCALE_THRESHOLD;
+          if (j == 0) {
+            m_i = m_new;
+          } else if (__any_sync(0xffffffffu, need)) {
+            const float f = (m_new == -INFINITY) ? 1.f : exp2f(m_i - m_new);
+            mbar_wait(&o_done[tile], (gt - 1) & 1);
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 0; c < 8; ++c) {
+              uint32_t orow[16];
+              tmem_ld_32x32b_x16(o_addr + c * 16, orow);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) orow[i] = __float_as_uint(__uint_as_float(orow[i]) * f);
+              tmem_st_32x32b_x16(o_addr + c * 16, orow);
+            }
+            tmem_st_wait();
+            l_i *= f;
+            m_i = m_new;
+          }
+          const float m_sub = (m_i == -INFINITY) ? 0.f : m_i;
+          uint64_t psum = 0, scale2, sub2;                             // pairs of fp32: one instruction scales, one adds two elements
+          asm("mov.b64 %0, {%1, %1};" : "=l"(scale2) : "f"(scale_log2));
+          asm("mov.b64 %0, {%1, %1};" : "=l"(sub2) : "f"(-m_sub));
+          auto probabilities = [&](const uint32_t (&v)[32], int c) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              uint64_t e, pr;
+              float e0, e1;
+              asm("mov.b64 %0, {%1, %2};" : "=l"(e) : "r"(v[i]), "r"(v[i + 1]));
+              asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(e) : "l"(scale2), "l"(sub2));
+              asm("mov.b64 {%0, %1}, %2;" : "=f"(e0), "=f"(e1) : "l"(e));
+              e0 = ex2_approx(e0);
+              e1 = ex2_approx(e1);
+              asm("mov.b64 %0, {%1, %2};" : "=l"(pr) : "f"(e0), "f"(e1));
+              asm("add.rn.f32x2 %0, %0, %1;" : "+l"(psum) : "l"(pr));
+              pk[i >> 1] = pack_bf16(e0, e1);
+            }
+            tmem_st_32x32b_x16(s_addr + c * 16, pk);
+          };
+          probabilities(x, 0);
+          tmem_ld_32x32b_x32(s_addr + 64, x);
+          probabilities(y, 1);
+          tmem_ld_32x32b_x32(s_addr + 96, y);
+          tmem_ld_wait();
+          if (need_mask) { mask(x, 64); mask(y, 96); }
+          probabilities(x, 2);
+          probabilities(y, 3);
+          float s0, s1;
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(psum));
+          l_i += s0 + s1;
+          tmem_st_wait();
+        }
+        tc_fence_before();
+        mbar_arrive(&p_full[tile]);
+      }
+      g += it.n_tiles;
+      mbar_wait(&o_final[tile], n_q & 1);
+      ++n_q;
+      tc_fence_after();
+      if (warp_valid) {
+        const float inv_l = (l_i > 0.f) ? 1.f / l_i : 0.f;
+        const size_t out_row = ((size_t)(it.q_start + tok)) * p.Hq + it.kvh * G + (r % G);
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t orow[32];
+          tmem_ld_32x32b_x32(o_addr + c * 32, orow);
+          tmem_ld_wait();
+          if (row_valid) {
+            __nv_bfloat16* dst = p.out + out_row * ATT_D + c * 32;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              U4 o;
+              o.x = pack_bf16(__uint_as_float(orow[v * 8 + 0]) * inv_l, __uint_as_float(orow[v * 8 + 1]) * inv_l);
+              o.y = pack_bf16(__uint_as_float(orow[v * 8 + 2]) * inv_l, __uint_as_float(orow[v * 8 + 3]) * inv_l);
+              o.z = pack_bf16(__uint_as_float(orow[v * 8 + 4]) * inv_l, __uint_as_float(orow[v * 8 + 5]) * inv_l);
+              o.w = pack_bf16(__uint_as_float(orow[v * 8 + 6]) * inv_l, __uint_as_float(orow[v * 8 + 7]) * inv_l);
+              st128(dst + v * 8, o);
+            }
+          }
+        }
+        if (row_valid && p.lse) p.lse[out_row] = (l_i > 0.f) ? (m_i + log2f(l_i)) * 0.6931471805599453f : -INFINITY;
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&o_free[tile]);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, 512);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const int done = atomicAdd(p.sched + 1, 1);
+    if (done == (int)gridDim.x - 1) { p.sched[0] = 0; p.sched[1] = 0; __threadfence(); }
+  }
+}
+
 void attn_merge_splits(const float* part_o, const float* part_lse, void* out, float* lse, int rows, int num_splits, const DiffCombine* diff,
                        cudaStream_t stream) {
   if (diff) {
     attn_merge_splits_diff_kernel<<<(rows / 2 + 7) / 8, 256, 0, stream>>>(part_o, part_lse, (__nv_bfloat16*)out, rows / 2, num_splits, *diff);
   } else {
-    attn_merge_splits_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(part_o, part_lse, (__nv_bfloat16*)out, lse, rows, num_splits);
+    attn_merge_splits_kernel<<<(rows + 3) / 4, 128, 0, stream>>>(part_o, part_lse, (__nv_bfloat16*)out, lse, rows, num_splits);
   }
   SGLB_CUDA_CHECK(cudaGetLastError());
 }
@@ -1042,6 +1414,20 @@ void attn_fwd_tc(const void* q, const void* k_cache, const void* v_cache, void* 
   // decode (one query token per request) is latency-bound: small KV tiles, two CTAs per SM
   const bool small = (cu_q == nullptr) && page_size <= 64;
   const bool capped = logit_cap > 0.f || slopes != nullptr;
+  // plain prompts whose pairs of query tiles give every SM one: the two-tile kernel; fewer pairs keep more SMs busy as single tiles
+  if (sched != nullptr && cu_q != nullptr && !capped && !diff && !tree_anc && window <= 0 && p.chunk == 0 && num_splits == 1 && max_q_len > TQ &&
+      (long long)T * Hkv >= 2LL * TQ * num_sms) {
+    p.gx = (max_q_len + 2 * TQ - 1) / (2 * TQ);
+    p.gy = Hkv;
+    const int all = p.gx * p.gy * B, ctas = std::min(all, num_sms), rest = all % ctas;
+    // a last round of pairs for fewer than half of the SMs is dealt out as single tiles, which take little more than half the time of a pair
+    p.pairs = 2 * rest <= ctas ? all - rest : all;
+    p.total_items = p.pairs + 2 * (all - p.pairs);
+    SGLB_CUDA_CHECK(cudaFuncSetAttribute(attn_fwd_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT2_SMEM_BYTES));
+    attn_fwd_tc_pair_kernel<<<ctas, ATT2_THREADS, ATT2_SMEM_BYTES, stream>>>(tmQ, tmK, tmV, p);
+    SGLB_CUDA_CHECK(cudaGetLastError());
+    return;
+  }
 #define SGLB_ATT_LAUNCH(KT_, CAP_)                                                                                         \
   do {                                                                                                                    \
     static bool configured = false;                                                                                       \

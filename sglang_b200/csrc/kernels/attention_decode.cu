@@ -42,7 +42,9 @@ constexpr int DA_TILE_BYTES = DA_KT * DA_D * 2;          // 32 KB  (K or V tile:
 constexpr int DA_HALF_BYTES = DA_TILE_BYTES / 2;
 constexpr int DA_Q_BYTES = 2 * DA_NQ * 128;              // 4 KB   (two d halves of [16 rows x 128 B])
 constexpr int DA_P_BYTES = 2 * DA_NQ * 128;              // 4 KB   (two 64-key chunks of [16 rows x 128 B]), double buffered
-constexpr int DA_SMEM_BYTES = 2 * DA_STAGES * DA_TILE_BYTES + 2 * DA_Q_BYTES + 2 * DA_P_BYTES + 1024 /*align*/ + 1024 /*barriers + scratch*/;
+constexpr int DA_ORDER = 256;             // batches up to this size are taken longest request first
+constexpr int DA_SMEM_BYTES = 2 * DA_STAGES * DA_TILE_BYTES + 2 * DA_Q_BYTES + 2 * DA_P_BYTES + 1024 /*align*/ + 1024 /*barriers + scratch*/ +
+                              2 * DA_ORDER * 4 + 16 /*lengths, order, total*/;
 constexpr float DA_RESCALE_THRESHOLD = 8.0f;
 
 constexpr int DA_PLAIN = 0, DA_CAP = 1, DA_DIFF = 2;      // MODE of a kernel instance
@@ -99,6 +101,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 26);
   volatile uint32_t* dbg = reinterpret_cast<volatile uint32_t*>(bars + 27); // [6] role state for the timeout dump
   float* red = reinterpret_cast<float*>(bars + 32);                         // [2][4 warps][GMAX] row-max exchange, then [4][GMAX] sums
+  int* s_len = reinterpret_cast<int*>(sP + 2 * DA_P_BYTES + 1024);          // [DA_ORDER] key tiles of every request, then the order they are taken in
+  int* s_order = s_len + DA_ORDER;
+  int* s_total = s_order + DA_ORDER;
 #define DA_WAIT(bar_, par_) mbar_wait((bar_), (par_), dbg, 6)
 
   // PROF builds: the elected thread of each role charges the cycles of a statement to a slot of its local table
@@ -129,6 +134,32 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   for (int i = threadIdx.x; i < DA_STAGES * DA_TILE_BYTES / 16; i += DA_THREADS) reinterpret_cast<U4*>(sV)[i] = U4{0, 0, 0, 0};
   fence_proxy_async_smem();
   if (warp == 1) { tmem_alloc(tmem_ptr, 64); tmem_relinquish(); }
+  // Longest request first, and no split shorter than a sixth of an SM's share of all key tiles: the queue then ends on small items.  In the batch's own
+  // order a long request at its end kept 56 CTAs busy alone for half of the launch.
+  const bool ordered = p.B > 1 && p.B <= DA_ORDER;
+  auto key_tiles = [&](int b) {
+    const int len = p.seq_lens[b];
+    int lo = 0;
+    if (p.window > 0) lo = max(0, len - p.window);
+    if (p.chunk > 0) lo = (len - 1) / p.chunk * p.chunk;
+    lo /= DA_KT;
+    return (len + DA_KT - 1) / DA_KT - (lo - min((p.keep_first + DA_KT - 1) / DA_KT, lo));
+  };
+  if (ordered) {
+    if (threadIdx.x == 0) *s_total = 0;
+    __syncthreads();
+    int sum = 0;
+    for (int b = threadIdx.x; b < p.B; b += DA_THREADS) { const int t = key_tiles(b); s_len[b] = t; sum += t; }
+    sum = warp_sum(sum);
+    if (lane == 0) atomicAdd(s_total, sum);
+    __syncthreads();
+    for (int b = threadIdx.x; b < p.B; b += DA_THREADS) {
+      const int t = s_len[b];
+      int rank = 0;
+      for (int o = 0; o < p.B; ++o) rank += s_len[o] > t || (s_len[o] == t && o < b);
+      s_order[rank] = b;
+    }
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -142,11 +173,12 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     int b, kvh, split, seq_len, kv_hi, tile_begin, n_tiles, keep_tiles, tile_skip;
     __device__ __forceinline__ int tile(int j) const { const int L = tile_begin + j; return L < keep_tiles ? L : L + tile_skip; }
   };
+  const int min_split = ordered ? (int)(((long long)*s_total * p.Hkv + 6 * gridDim.x - 1) / (6 * gridDim.x)) : 1;
   auto decode_item = [&](int idx) {
     Item it;
     const int per_b = p.Hkv * p.num_splits;
-    it.b = idx / per_b;
-    const int y = idx - it.b * per_b;
+    const int nth = idx / per_b, y = idx - nth * per_b;
+    it.b = ordered ? s_order[nth] : nth;
     it.kvh = y / p.num_splits; it.split = y - it.kvh * p.num_splits;
     it.seq_len = p.seq_lens[it.b];
     it.kv_hi = it.seq_len;
@@ -157,27 +189,33 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     it.keep_tiles = min((p.keep_first + DA_KT - 1) / DA_KT, tile_lo);
     it.tile_skip = tile_lo - it.keep_tiles;
     const int tile_hi = (it.kv_hi + DA_KT - 1) / DA_KT - it.tile_skip;
-    const int per_split = (tile_hi + p.num_splits - 1) / p.num_splits;
+    const int per_split = max((tile_hi + p.num_splits - 1) / p.num_splits, min_split);
     it.tile_begin = it.split * per_split;
     it.n_tiles = max(0, min(tile_hi, it.tile_begin + per_split) - it.tile_begin);
     return it;
   };
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
     // ------------------------------------------------------------ scheduler + TMA producer
+    // A lane per (page, d half) of a tile: addresses are worked out side by side and a tile's copies leave in one instruction for K and one for V; the
+    // page ids of the next tile are fetched while this one is issued.  One thread that walked the pages spent 3900 cycles on a tile of 16 copies, more
+    // than the 2700 its 64 KB take at an SM's share of the memory rate.
     uint32_t n_it = 0, n_q = 0, g = 0;
-    const int ps = p.page_size, pages_per_tile = DA_KT / ps;
-    int next_idx = atomicAdd(p.sched, 1);
+    const int ps = p.page_size, pages_per_tile = DA_KT / ps, my_page = lane >> 1;
+    const int my_off = my_page * ps * 128 + (lane & 1) * DA_HALF_BYTES, my_d = (lane & 1) * 64;
+    int next_idx = lane == 0 ? atomicAdd(p.sched, 1) : 0;
     for (;;) {
       const int slot = n_it & 1;
       DA_T(0, DA_WAIT(&item_empty[slot], ((n_it >> 1) & 1) ^ 1));
       // the queue atomic is a ~1 us L2 round trip: fetch the NEXT item's index now and consume it one iteration later, so the round trip
-      // overlaps this item's TMA issue instead of stalling the only thread that feeds the ring
-      const int idx = next_idx;
-      if (idx < p.total_items) next_idx = atomicAdd(p.sched, 1);
-      DA_DBG(1, n_it, g);
-      s_item[slot] = idx;
-      mbar_arrive(&item_full[slot]);
+      // overlaps this item's TMA issue instead of stalling the only warp that feeds the ring
+      const int idx = __shfl_sync(0xffffffffu, next_idx, 0);
+      if (lane == 0) {
+        if (idx < p.total_items) next_idx = atomicAdd(p.sched, 1);
+        DA_DBG(1, n_it, g);
+        s_item[slot] = idx;
+        mbar_arrive(&item_full[slot]);
+      }
       ++n_it;
       if (idx >= p.total_items) break;
       const Item it = decode_item(idx);
@@ -186,38 +224,36 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const int qs = n_q & 1;
         uint8_t* qdst = sQ + qs * DA_Q_BYTES;
         DA_T(1, DA_WAIT(&q_empty[qs], ((n_q >> 1) & 1) ^ 1));
-        mbar_expect_tx(&q_full[qs], 2 * G * 128);
-        tma_load_4d(qdst, &tmQ, &q_full[qs], 0, 0, it.kvh, it.b);
-        tma_load_4d(qdst + DA_NQ * 128, &tmQ, &q_full[qs], 64, 0, it.kvh, it.b);
+        if (lane == 0) {
+          mbar_expect_tx(&q_full[qs], 2 * G * 128);
+          tma_load_4d(qdst, &tmQ, &q_full[qs], 0, 0, it.kvh, it.b);
+          tma_load_4d(qdst + DA_NQ * 128, &tmQ, &q_full[qs], 64, 0, it.kvh, it.b);
+        }
+        __syncwarp();
         ++n_q;
       }
       const int* pt = p.page_table + (size_t)p.req_slots[it.b] * p.pt_stride;
+      auto live_pages = [&](int j) { return min(pages_per_tile, (it.kv_hi - it.tile(j) * DA_KT + ps - 1) / ps); };      // only pages that hold live keys
+      auto page_id = [&](int j) { return my_page < live_pages(j) ? pt[it.tile(j) * DA_KT / ps + my_page] : 0; };
+      int next_page = page_id(0);
       for (int j = 0; j < it.n_tiles; ++j, ++g) {
         const int st = g % DA_STAGES;
         const uint32_t ph = (g / DA_STAGES) & 1;
-        const int key0 = it.tile(j) * DA_KT;
-        const int n_pages = min(pages_per_tile, (it.kv_hi - key0 + ps - 1) / ps);     // only pages that hold live keys
-        const int pg0 = key0 / ps;
+        const int n_pages = live_pages(j), slot0 = next_page * ps;
         const uint32_t bytes = (uint32_t)n_pages * ps * 256;
+        if (j + 1 < it.n_tiles) next_page = page_id(j + 1);
         DA_T(2, DA_WAIT(&k_empty[st], ph ^ 1));
         if constexpr (PROF) pacc[4] += 1;
-        mbar_expect_tx(&k_full[st], bytes);
-        for (int i = 0; i < n_pages; ++i) {
-          const int page = pt[pg0 + i];
-          uint8_t* dst = sK + st * DA_TILE_BYTES + i * ps * 128;
-          tma_load_3d(dst, &tmK, &k_full[st], 0, it.kvh, page * ps);
-          tma_load_3d(dst + DA_HALF_BYTES, &tmK, &k_full[st], 64, it.kvh, page * ps);
-        }
+        if (lane == 0) mbar_expect_tx(&k_full[st], bytes);
+        __syncwarp();
+        if (my_page < n_pages) tma_load_3d(sK + st * DA_TILE_BYTES + my_off, &tmK, &k_full[st], my_d, it.kvh, slot0);
         DA_T(3, DA_WAIT(&v_empty[st], ph ^ 1));
-        mbar_expect_tx(&v_full[st], bytes);
-        for (int i = 0; i < n_pages; ++i) {
-          const int page = pt[pg0 + i];
-          uint8_t* dst = sV + st * DA_TILE_BYTES + i * ps * 128;
-          tma_load_3d(dst, &tmV, &v_full[st], 0, it.kvh, page * ps);
-          tma_load_3d(dst + DA_HALF_BYTES, &tmV, &v_full[st], 64, it.kvh, page * ps);
-        }
+        if (lane == 0) mbar_expect_tx(&v_full[st], bytes);
+        __syncwarp();
+        if (my_page < n_pages) tma_load_3d(sV + st * DA_TILE_BYTES + my_off, &tmV, &v_full[st], my_d, it.kvh, slot0);
       }
     }
+    __syncwarp();
   } else if (warp == 1 && lane == 0) {
     // ------------------------------------------------------------ MMA issuer
     constexpr uint32_t idesc_s = make_idesc(UMMA_BF16, UMMA_BF16, DA_KT, DA_NQ, 0, 0);      // A = K (K-major), B = Q (K-major)

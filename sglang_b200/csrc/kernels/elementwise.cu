@@ -19,6 +19,9 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(__nv_bfloat16* __restrict_
   const int nvec = H >> 3;
   float v[MAXV][8];
   float ss = 0.f;
+  U4 ww[MAXV];                     // weights: on their way while the row is summed (a decode batch's norm is one chain of latencies)
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) ww[i] = threadIdx.x + i * 256 < nvec ? ldg128(w + (threadIdx.x + i * 256) * 8) : U4{0, 0, 0, 0};
 #pragma unroll
   for (int i = 0; i < MAXV; ++i) {
     const int vi = threadIdx.x + i * 256;
@@ -52,8 +55,8 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(__nv_bfloat16* __restrict_
   for (int i = 0; i < MAXV; ++i) {
     const int vi = threadIdx.x + i * 256;
     if (vi < nvec) {
-      U4 ww = ldg128(w + vi * 8);
-      float g[8] = {bf16_lo(ww.x), bf16_hi(ww.x), bf16_lo(ww.y), bf16_hi(ww.y), bf16_lo(ww.z), bf16_hi(ww.z), bf16_lo(ww.w), bf16_hi(ww.w)};
+      const U4 q = ww[i];
+      float g[8] = {bf16_lo(q.x), bf16_hi(q.x), bf16_lo(q.y), bf16_hi(q.y), bf16_lo(q.z), bf16_hi(q.z), bf16_lo(q.w), bf16_hi(q.w)};
       float o[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) o[k] = v[i][k] * rs * (GEMMA ? (1.f + g[k]) : g[k]);

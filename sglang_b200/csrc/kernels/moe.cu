@@ -195,12 +195,12 @@ void moe_align(const int* topk_ids, const float* topk_w, int n_pairs, int E, int
 }
 
 // ---------------------------------------------------------------- gather into expert-sorted order
-// A warp per row, so that no row waits for another's index; padding rows cost one load.
+// 64 threads a row, so that no row waits for another's index and few rows still spread over the chip; padding rows cost one load.
 template <bool SCALE>
 __global__ void __launch_bounds__(256) moe_gather_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ sorted_row,
                                                          const int* __restrict__ num_tiles, __nv_bfloat16* __restrict__ xs, int H,
                                                          int x_stride, int K, int cap_rows, int tile, const float* __restrict__ row_w) {
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 6), lane = threadIdx.x & 63;
   if (row >= min(cap_rows, __ldg(num_tiles) * tile)) return;
   const int pair = __ldg(sorted_row + row), nvec = H >> 3;
   if (pair < 0) return;
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const __nv_bfloat16* __
   const __nv_bfloat16* src = x + (size_t)(pair / K) * x_stride;
   [[maybe_unused]] const float w = SCALE ? __ldg(row_w + row) : 1.f;
 #pragma unroll 8
-  for (int v = lane; v < nvec; v += 32) {
+  for (int v = lane; v < nvec; v += 64) {
     U4 a = ldg128(src + v * 8);
     if (SCALE)
       a = U4{pack_bf16(bf16_lo(a.x) * w, bf16_hi(a.x) * w), pack_bf16(bf16_lo(a.y) * w, bf16_hi(a.y) * w),
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const __nv_bfloat16* __
 void moe_gather(const void* x, const int* sorted_row, const int* num_tiles, void* xs, int H, int x_stride, int K, int cap_rows,
                 int tile, cudaStream_t stream, const float* row_w) {
   if (H % 8) throw std::runtime_error("sglb moe_gather: hidden size must be a multiple of 8");
-  const int grid = (cap_rows + 7) / 8;
+  const int grid = (cap_rows + 3) / 4;
   if (row_w)
     moe_gather_kernel<true><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, sorted_row, num_tiles, (__nv_bfloat16*)xs, H, x_stride, K, cap_rows, tile, row_w);
   else

@@ -1203,7 +1203,8 @@ void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::
   auto stream = cur_stream();
   const int pairs = T * K;
   // Up to 64 rows an expert on average the block is bound by the weights: rows become the narrow operand (gemm_grouped_decode.cu) in tiles that hold
-  // twice the average, so that few experts need a second one; beyond, 128-row tiles (gemm_tc.cu), whose two token tiles an expert read its weights once.
+  // twice the average, so that few experts need a second one (both products at 5 rows an expert 617 -> 454 us, at 21 rows 292 -> 227 us); beyond, at
+  // least half of a 128-row tile (gemm_tc.cu) is live on average and its wider tiles take less from L2 per product.
   const bool decode = pairs <= 64ll * E;
   int tile = 128;
   if (decode)

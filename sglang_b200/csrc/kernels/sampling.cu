@@ -78,6 +78,9 @@ constexpr int SAMP_CL = 8;              // CTAs per row: a portable cluster
 constexpr int SAMP_SEG = SAMP_BINS / SAMP_CL;
 
 __device__ __forceinline__ uint32_t cl_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+// the two halves of a first barrier: a CTA's shared memory may be written by its peers only once it has started, and this is what tells them so
+__device__ __forceinline__ void cl_started() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cl_all_started() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cl_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -127,6 +130,7 @@ __global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT, NT == 256 
 sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
   constexpr int NW = NT / 32, WCAP = SAMP_LIST / NW;
   __shared__ SampShared<NW> sh;
+  cl_started();
   const int rank = (int)cl_rank(), row = blockIdx.x / SAMP_CL;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int V = p.V;
@@ -193,6 +197,7 @@ sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
   }
   if (lane == 0) { sh.wred[0][warp] = __float_as_uint(mx); sh.wred[1][warp] = (uint32_t)am; }
   __syncthreads();
+  cl_all_started();                                                    // (long past by now: the pass over the row lies between)
   if (warp == 0) {
     mx = lane < NW ? __uint_as_float(sh.wred[0][lane]) : -INFINITY;
     am = lane < NW ? (int)sh.wred[1][lane] : 0x7fffffff;

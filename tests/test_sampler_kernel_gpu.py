@@ -93,3 +93,14 @@ def test_flat_and_masked_rows():
     tok = ops.sample(logits, ones, k, ones * 0.9, ones * 0, global_seed=5, step=1)
     assert int(tok[1]) == 4321 and 0 <= int(tok[2]) < V
     assert abs(int(tok[0]) - _uniform(5, 0, 1) * V) <= 2 + 1e-5 * V and abs(int(tok[3]) - _uniform(5, 3, 1) * V) <= 2 + 1e-5 * V
+
+
+@pytest.mark.parametrize("B", [3, 300])
+@pytest.mark.parametrize("V", [1, 7, 256, 2047])
+def test_short_rows(B, V):
+    """most CTAs of a row's cluster have nothing to read and reach the exchange of maxima at once: none may write to a peer that has not started"""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    one, k = torch.ones(B, device="cuda"), torch.ones(B, device="cuda", dtype=torch.int32)
+    for _ in range(20):
+        logits = torch.randn(B, V, generator=g, device="cuda")
+        assert torch.equal(ops.sample(logits, one, k, one, one * 0, global_seed=3, step=1).long(), logits.argmax(-1))

@@ -79,3 +79,15 @@ def test_group_quant(M, K, pad, ue8m0):
     back = got.view(M, kg, 128) * s.double()[..., None]
     # half an ulp of e4m3 (2^-4 of a value, 2^-10 of the scale below the smallest normal), a whole one where the product with 1 / scale lands on a tie
     assert bool(((back - xg).abs() <= xg.abs() * 2 ** -4 * 1.001 + s.double()[..., None] * 2 ** -10).all())
+
+
+def test_silu_and_mul_rounds_as_the_fused_epilogue():
+    """the same bits as the product whose epilogue applies it (csrc/kernels/gemm_tc.cu), which an identity matrix hands exactly the same numbers: every
+    gate bf16 has between 2^-20 and 80, times every mantissa"""
+    assert ops.load_native()
+    gates = torch.arange(-(1 << 15), 1 << 15, device="cuda").to(torch.int16).view(torch.bfloat16)
+    gates = gates[(gates.float().abs() < 80) & (gates.float().abs() > 2 ** -20)]
+    up = 1 + torch.arange(128, device="cuda").to(torch.bfloat16) / 128
+    x = torch.cat([gates[:, None].expand(-1, 128), up[None].expand(gates.numel(), -1)], dim=1).contiguous()
+    fused = ops.gemm_tc(x, torch.eye(256, device="cuda", dtype=torch.bfloat16), epilogue=ops.EPI_SILU_SPLIT)
+    assert int((ops.silu_and_mul(x) != fused).sum()) == 0

@@ -1281,23 +1281,33 @@ attn_fwd_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             m_i = m_new;
           }
           const float m_sub = (m_i == -INFINITY) ? 0.f : m_i;
-          uint64_t psum = 0, scale2, sub2;                             // pairs of fp32: one instruction scales, one adds two elements
+          float psum = 0.f;
+          uint64_t scale2, sub2;                                       // pairs of fp32: one instruction scales two elements
           asm("mov.b64 %0, {%1, %1};" : "=l"(scale2) : "f"(scale_log2));
           asm("mov.b64 %0, {%1, %1};" : "=l"(sub2) : "f"(-m_sub));
           auto probabilities = [&](const uint32_t (&v)[32], int c) {
             uint32_t pk[16];
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-              uint64_t e, pr;
-              float e0, e1;
-              asm("mov.b64 %0, {%1, %2};" : "=l"(e) : "r"(v[i]), "r"(v[i + 1]));
-              asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(e) : "l"(scale2), "l"(sub2));
-              asm("mov.b64 {%0, %1}, %2;" : "=f"(e0), "=f"(e1) : "l"(e));
-              e0 = ex2_approx(e0);
-              e1 = ex2_approx(e1);
-              asm("mov.b64 %0, {%1, %2};" : "=l"(pr) : "f"(e0), "f"(e1));
-              asm("add.rn.f32x2 %0, %0, %1;" : "+l"(psum) : "l"(pr));
-              pk[i >> 1] = pack_bf16(e0, e1);
+            for (int i = 0; i < 32; i += 4) {
+              float e[4];
+#pragma unroll
+              for (int k = 0; k < 4; k += 2) {
+                uint64_t t;
+                asm("mov.b64 %0, {%1, %2};" : "=l"(t) : "r"(v[i + k]), "r"(v[i + k + 1]));
+                asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(t) : "l"(scale2), "l"(sub2));
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(e[k]), "=f"(e[k + 1]) : "l"(t));
+                e[k] = ex2_approx(e[k]);
+                e[k + 1] = ex2_approx(e[k + 1]);
+                pk[(i + k) >> 1] = pack_bf16(e[k], e[k + 1]);
+              }
+              uint64_t even, odd;                                      // neighbours are added two pairs at once, then one after the other into the sum
+              float a, b;
+              asm("mov.b64 %0, {%1, %2};" : "=l"(even) : "f"(e[0]), "f"(e[2]));
+              asm("mov.b64 %0, {%1, %2};" : "=l"(odd) : "f"(e[1]), "f"(e[3]));
+              asm("add.rn.f32x2 %0, %0, %1;" : "+l"(even) : "l"(odd));
+              asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(even));
+              psum += a;
+              psum += b;
             }
             tmem_st_32x32b_x16(s_addr + c * 16, pk);
           };
@@ -1309,9 +1319,7 @@ attn_fwd_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           if (need_mask) { mask(x, 64); mask(y, 96); }
           probabilities(x, 2);
           probabilities(y, 3);
-          float s0, s1;
-          asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(psum));
-          l_i += s0 + s1;
+          l_i += psum;
           tmem_st_wait();
         }
         tc_fence_before();

@@ -12,7 +12,7 @@
 //
 //   prompt shapes (gemm_fp8_block_kernel): rows of A are the UMMA M dimension, 256 / 128 / 64 weight rows the N dimension, persistent CTAs.
 //     warp 0 : TMA producer      warp 1 : MMA issuer      warp 2 : TMEM alloc      warps 4.. : promotion + epilogue, 64 columns each at most
-//   decode shapes (gemm_fp8_swap_kernel, up to 128 tokens): 128 weight rows are the M dimension, the tokens the N dimension, so no tensor or TMA
+//   decode shapes (gemm_fp8_swap_kernel, up to 64 tokens): 128 weight rows are the M dimension, the tokens the N dimension, so no tensor or TMA
 //     work goes into padding rows; a cluster shares a tile's K blocks and adds its partial sums through distributed shared memory.
 //
 // Reference counterparts: python/sglang/srt/layers/quantization/fp8_kernel.py (per_token_group_quant_fp8,
@@ -195,7 +195,8 @@ static void launch_fp8(const void* A, const float* xs, const void* W, const floa
 // ---------------------------------------------------------------- decode shapes: weights as the UMMA M dimension
 // Bound by streaming the weights.  Every CTA owns (128 weight rows) x (a share of the K blocks); the CTAs of a cluster share one tile, park their
 // fp32 partial sums in their own shared memory and each adds up (in rank order) and writes an equal part of the tokens.  Small CTAs (three 16 KB
-// weight stages) so that three or four of them per SM keep ~200 KB in flight and hide one another's start and end.
+// weight stages): an SM holds four, three or two of them at 16, 32 and 64 tokens, which keep 192, 144 or 96 KB of weights in flight and hide one
+// another's start and end.
 // Measured, 9 tokens, [7168 x 8192] and [8192 x 3584]: 43.6 -> 15.1 us a product on average (the version before ran 32-wide tiles of 128 padded rows).
 constexpr int F8S_THREADS = 192;
 template <int NT>
@@ -396,11 +397,12 @@ void gemm_fp8_block(const void* A, const float* xs, const void* W, const float* 
   if (M <= 0 || N <= 0) return;
   if (K % 16 || N % 8 || lda % 16 || ldw % 16) throw std::runtime_error("sglb fp8 gemm: K, lda, ldw must be multiples of 16 and N of 8");
 #define SGLB_F8(F) F(A, xs, W, ws, C, M, N, K, lda, ldw, ldc, xs_stride, ws_stride, num_sms, stream)
-  // up to 128 tokens fit one UMMA N dimension beside 128 weight rows; from there on a weight tile would be read once per 128 tokens either way
+  // Up to 64 tokens: a promotion thread holds its weight row's 64 sums and an SM two CTAs.  128 sums leave one CTA an SM behind one serial chain, so
+  // from 65 tokens on the rows of A are the M dimension.  us at [7168 x 8192] / [8192 x 3584] / [28672 x 4096] / [4096 x 14336], weights from memory:
+  // 64 tokens 21 / 13 / 30 / 18 here, 27 / 14 / 26 / 44 there; 65 tokens 44 / 30 / 60 / 54 here (128 tokens wide), 27 / 15 / 26 / 44 there
   if (M <= 16) { SGLB_F8(launch_fp8_swap<16>); return; }
   if (M <= 32) { SGLB_F8(launch_fp8_swap<32>); return; }
   if (M <= 64) { SGLB_F8(launch_fp8_swap<64>); return; }
-  if (M <= 128) { SGLB_F8(launch_fp8_swap<128>); return; }
   // the width whose waves take the least time: a tile costs its columns plus a start and an end worth about 32 of them
   const int m_tiles = (M + F8_BM - 1) / F8_BM;
   int bn = 0;

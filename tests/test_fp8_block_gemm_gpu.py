@@ -27,3 +27,19 @@ def test_edges(M, N, K):
     bound = ref.abs() * 2 ** -8 + (x.square() @ w.square().T).sqrt() * 2 ** -16
     assert bool(((out[:, :N].double() - ref).abs() <= bound).all()), float(((out[:, :N].double() - ref).abs() / bound).max())
     assert bool((out[:, N:] == 7).all())
+
+
+@pytest.mark.parametrize("N,K", [(1024, 4096), (7168, 1024)])
+def test_rows_of_one_kernel_are_alike(N, K):
+    """from 65 rows on one kernel sums K in sequence: a row's bits do not follow how many others there are"""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    xq = (torch.randn(200, K, generator=g, device="cuda") * 40).to(torch.float8_e4m3fn)
+    wq = (torch.randn(N, K, generator=g, device="cuda") * 40).to(torch.float8_e4m3fn)
+    xs = torch.rand(200, K // 128, generator=g, device="cuda") * 0.02 + 0.001
+    ws = torch.rand(N // 128, K // 128, generator=g, device="cuda") * 0.02 + 0.001
+    whole = torch.empty(200, N, device="cuda", dtype=torch.bfloat16)
+    torch.ops.sglb.gemm_fp8_block(xq, xs, wq, ws, whole)
+    for M in (65, 96, 128, 129):
+        out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+        torch.ops.sglb.gemm_fp8_block(xq[:M], xs[:M], wq, ws, out)
+        assert torch.equal(out, whole[:M])

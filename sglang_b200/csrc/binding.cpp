@@ -1202,10 +1202,12 @@ void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::
   c10::cuda::CUDAGuard g(x.device());
   auto stream = cur_stream();
   const int pairs = T * K;
-  // Up to 64 rows an expert on average the block is bound by the weights: rows become the narrow operand (gemm_grouped_decode.cu) in tiles that hold
-  // twice the average, so that few experts need a second one (both products at 5 rows an expert 617 -> 454 us, at 21 rows 292 -> 227 us); beyond, at
-  // least half of a 128-row tile (gemm_tc.cu) is live on average and its wider tiles take less from L2 per product.
-  const bool decode = pairs <= 64ll * E;
+  // Up to 48 rows an expert on average the block is bound by the weights: rows become the narrow operand (gemm_grouped_decode.cu) in tiles that hold
+  // twice the average, so that few experts need a second one; beyond, 128-row tiles (gemm_tc.cu) take less from L2 per product.  us a block here / there,
+  // 8 experts of 4096 x 14336, 2 chosen: 492 / 624 at 24 rows, 492 / 542 at 32, 538 / 542 at 40, 552 / 549 at 48, 560 / 550 at 56, 606 / 536 at 64;
+  // 128 experts of 2048 x 768, 8 chosen: 291 / 320 at 32, 340 / 358 at 44, 352 / 360 at 48, 371 / 370 at 56, 396 / 386 at 64.  Under expert parallelism
+  // the pairs are those of all ranks, so the line is met sooner by their number.
+  const bool decode = pairs <= 48ll * E;
   int tile = 128;
   if (decode)
     for (int t : {16, 32, 64, 128}) {

@@ -647,7 +647,7 @@ sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float e = i < w1 ? __expf((v[j] - gmax) * inv_t) : 0.f;
-      const bool keep = i < w1 && e >= thr;
+      const bool keep = i < w1 && e >= thr && e > 0.f;                 // (a masked logit has no mass, and what rounding leaves over is not its own)
       r[j] = keep ? e : 0.f;
       s += r[j];
       if (keep) mine = i + j;

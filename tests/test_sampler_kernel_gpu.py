@@ -104,3 +104,18 @@ def test_short_rows(B, V):
     for _ in range(20):
         logits = torch.randn(B, V, generator=g, device="cuda")
         assert torch.equal(ops.sample(logits, one, k, one, one * 0, global_seed=3, step=1).long(), logits.argmax(-1))
+
+
+def test_masked_logits_are_never_drawn():
+    """the drawn point at the very end of the kept mass, where rounding decides whether any running sum passes it: the last logit that has mass, not a
+    masked one behind it"""
+    B, V, live = 512, 3000, 1000
+    assert _uniform(11, 0, 24699704) == 1 - 2.0 ** -24
+    g = torch.Generator(device="cuda").manual_seed(8)
+    logits = torch.randn(B, V, generator=g, device="cuda")
+    logits[:, live:] = float("-inf")
+    one = torch.ones(B, device="cuda")
+    seeds = torch.tensor([[11, 24699704]] * B, device="cuda")
+    for p in (1.0, 0.9999999):
+        tok = ops.sample(logits, one, one.int() * 0, one * p, one * 0, seeds=seeds, global_seed=1, step=1)
+        assert int(tok.max()) < live and int(tok.min()) > live - 50

@@ -251,7 +251,7 @@ sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
     }
   };
   constexpr float W1 = 1.f / 64.f;
-  const float scale = fminf(16384.f, 4294967040.f / (float)V), inv_scale = 1.f / scale;
+  const float scale = fminf(16384.f, floorf(4294967040.f / (float)V)), inv_scale = 1.f / scale;      // whole: V logits of a bin's largest r fit 32 bits
   auto bin1 = [](float d) { return min(SAMP_BINS - 1, (int)(d * (1.f / W1))); };
   auto fixed_mass = [&](float d, int b) { return (uint32_t)(__expf(b * W1 - d) * scale + 0.5f); };
   const auto count = [](int, uint32_t s) { return (float)s; };

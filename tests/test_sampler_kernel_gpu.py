@@ -119,3 +119,22 @@ def test_masked_logits_are_never_drawn():
     for p in (1.0, 0.9999999):
         tok = ops.sample(logits, one, one.int() * 0, one * p, one * 0, seeds=seeds, global_seed=1, step=1)
         assert int(tok.max()) < live and int(tok.min()) > live - 50
+
+
+@pytest.mark.parametrize("V,top_p", [(262144, 0.9), (524288, 0.5)])
+def test_plateaus(V, top_p, tail=0.0):
+    """rows whose logits all meet in one bin: their fixed-point mass does not overflow, which would send the search through every bin (a pass over a row
+    takes some microseconds, so all passes of a bounded search end within two milliseconds)"""
+    logits = torch.full((2, V), tail, device="cuda")
+    logits[:, 5] = 0.0
+    one, lp = torch.ones(2, device="cuda"), torch.empty(2, device="cuda")
+    draw = lambda: ops.sample(logits, one, one.int() * 0, one * top_p, one * 0, out_logprobs=lp, global_seed=9, step=2)  # noqa: E731
+    draw()
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    a.record()
+    tok = draw()
+    b.record()
+    b.synchronize()
+    assert a.elapsed_time(b) < 2.0, a.elapsed_time(b)
+    for i in range(2):
+        _check_row(logits[i], 1.0, 0, top_p, 0.0, _uniform(9, i, 2), int(tok[i]), float(lp[i]))

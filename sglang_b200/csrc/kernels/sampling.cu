@@ -64,8 +64,8 @@ struct SampleParams {
 // top-k / top-p: two-level histogram over d = (max - logit) / T (r = p / p_max = e^-d): 2048 bins of width 1/64 cover r down to e^-32, a second
 // 2048 bins refine the one that holds the boundary (7.6e-6 in d).  Shared-memory atomics are native for integers only (a float add is a
 // compare-and-swap loop that collapses on the popular bins of a broad tail), so both levels count integers: elements, or r over the bin's largest r
-// in fixed point.  The fixed-point mass only nominates a bin; the masses before and inside it are then summed in fp32 and the nomination is moved
-// until they enclose the target.  Elements beyond d = 32 (masked ones, cold temperatures) meet in the last bin and are added up in registers.
+// in fixed point.  The fixed-point mass only nominates a bin; the masses before and inside it are then summed in fp32 and the nomination is moved,
+// to its neighbour and then by halves, until they enclose the target.  Elements beyond d = 32 (masked ones, cold temperatures) meet in the last bin and are added up in registers.
 //
 // What can be kept is usually a handful of candidates: the threads' own maxima (2048 or 8192 of them) bound the boundary from below, one pass collects
 // what lies above that bound, and the first CTA alone finishes the row on that list without further cluster barriers.  A row whose list would not fit
@@ -414,7 +414,8 @@ sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
       float before = 0.f;
       int b1 = min(find(target, before, mass), SAMP_BINS - 1);
       float m_before, m_in;
-      int moved = 0;                                                   // one direction only: rounding at an edge cannot make it swing
+      int first = 0, last_bin = SAMP_BINS - 1;                         // where the bin can be: the nominated one, its neighbour, then by halves
+      bool nominated = true;
       while (true) {                                                   // (the same numbers in every thread)
         m_before = m_in = 0.f;
         const int b = b1;
@@ -430,11 +431,18 @@ sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
           }
         });
         sums(m_before, m_in);
-        if (m_before >= target && b1 > 0 && moved <= 0) { moved = -1; --b1; continue; }
-        if (m_before + m_in < target && b1 < SAMP_BINS - 1 && moved >= 0) { moved = 1; ++b1; continue; }
-        break;
+        if (m_before >= target && b1 > first) {
+          last_bin = b1 - 1;
+          b1 = nominated ? last_bin : (first + last_bin) >> 1;
+        } else if (m_before + m_in < target && b1 < last_bin) {
+          first = b1 + 1;
+          b1 = nominated ? first : (first + last_bin) >> 1;
+        } else {
+          break;
+        }
+        nominated = false;
       }
-      if (moved < 0 || m_before + m_in >= target)
+      if (last_bin < SAMP_BINS - 1 || m_before + m_in >= target)       // (else rounding holds the whole row below the target)
         d_max = fminf(d_max, refine(b1, target - m_before, [&](int b, uint32_t s) { return (float)s * __expf(-(b1 * W1 + (b + 0.5f) * (W1 / SAMP_BINS))); }));
     }
     return d_max;

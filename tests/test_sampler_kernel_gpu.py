@@ -121,10 +121,11 @@ def test_masked_logits_are_never_drawn():
         assert int(tok.max()) < live and int(tok.min()) > live - 50
 
 
-@pytest.mark.parametrize("V,top_p", [(262144, 0.9), (524288, 0.5)])
-def test_plateaus(V, top_p, tail=0.0):
-    """rows whose logits all meet in one bin: their fixed-point mass does not overflow, which would send the search through every bin (a pass over a row
-    takes some microseconds, so all passes of a bounded search end within two milliseconds)"""
+@pytest.mark.parametrize("V,top_p", [(262144, 0.9), (524288, 0.5), (200000, 0.99999)])
+@pytest.mark.parametrize("tail", [0.0, -1.011266])
+def test_plateaus(V, top_p, tail):
+    """rows whose logits nearly all meet in one bin: their fixed-point mass neither overflows nor, where each rounds down (16200.45 / 16384 of the bin's
+    largest), sends the search through every bin: a pass over a row takes some microseconds, so all passes of a bounded search end within two milliseconds"""
     logits = torch.full((2, V), tail, device="cuda")
     logits[:, 5] = 0.0
     one, lp = torch.ones(2, device="cuda"), torch.empty(2, device="cuda")

@@ -67,7 +67,7 @@ struct SampleParams {
 // in fixed point.  The fixed-point mass only nominates a bin; the masses before and inside it are then summed in fp32 and the nomination is moved,
 // to its neighbour and then by halves, until they enclose the target.  Elements beyond d = 32 (masked ones, cold temperatures) meet in the last bin and are added up in registers.
 //
-// What can be kept is usually a handful of candidates: the threads' own maxima (2048 or 8192 of them) bound the boundary from below, one pass collects
+// What can be kept is usually a handful of candidates: the threads' own maxima (2048 of them) bound the boundary from below, one pass collects
 // what lies above that bound, and the first CTA alone finishes the row on that list without further cluster barriers.  A row whose list would not fit
 // (a broad nucleus, a large k) goes through the same steps on the whole row with all eight.
 //
@@ -76,6 +76,9 @@ struct SampleParams {
 // the 121, the cluster without candidate lists 69.
 constexpr int SAMP_CL = 8;              // CTAs per row: a portable cluster
 constexpr int SAMP_SEG = SAMP_BINS / SAMP_CL;
+// One width for every batch, so that a row's sums, and with them a seeded request's token, do not follow how many rows there are.  256 threads, several
+// CTAs an SM, against 1024, one: 16 and 21 us against 21 and 23 for 8 rows of 32000 and 128256, 23 against 33 for 32 of 128256, 11 either way for one
+constexpr int SAMP_NT = 256;
 
 __device__ __forceinline__ uint32_t cl_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 // the two halves of a first barrier: a CTA's shared memory may be written by its peers only once it has started, and this is what tells them so
@@ -125,10 +128,10 @@ __device__ __forceinline__ void samp_load8(const float* p, float (&v)[8]) {
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-template <typename T, int NT>
-__global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(NT, NT == 256 ? 6 : 1)
+template <typename T>
+__global__ void __cluster_dims__(SAMP_CL, 1, 1) __launch_bounds__(SAMP_NT, 6)
 sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
-  constexpr int NW = NT / 32, WCAP = SAMP_LIST / NW;
+  constexpr int NT = SAMP_NT, NW = NT / 32, WCAP = SAMP_LIST / NW;
   __shared__ SampShared<NW> sh;
   cl_started();
   const int rank = (int)cl_rank(), row = blockIdx.x / SAMP_CL;
@@ -689,11 +692,11 @@ sample_kernel(const T* __restrict__ logits, SampleParams p, int per_warp) {
   if (lane == 0) finish(token);
 }
 
-template <typename T, int NT>
+template <typename T>
 static void launch_sample(const void* logits, const SampleParams& p, int B, cudaStream_t stream) {
-  constexpr int NW = NT / 32;
+  constexpr int NW = SAMP_NT / 32;
   const int per_warp = ((p.V + SAMP_CL * NW - 1) / (SAMP_CL * NW) + 255) / 256 * 256;
-  sample_kernel<T, NT><<<B * SAMP_CL, NT, 0, stream>>>((const T*)logits, p, per_warp);
+  sample_kernel<T><<<B * SAMP_CL, SAMP_NT, 0, stream>>>((const T*)logits, p, per_warp);
   SGLB_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -704,15 +707,8 @@ void sample(const void* logits, bool bf16, int B, int V, int stride, const float
   if (B <= 0) return;
   SampleParams p{temperature, top_k, top_p, min_p, seeds, out_slots, next_token_buf, out_tokens, out_logprobs, global_seed,
                  step_ptr, step, V, stride};
-  // few rows: one CTA per SM, so its threads hide the latency alone; more rows: small CTAs, several per SM (18 rows: 27 us with 1024 threads, 24 rows:
-  // 23 us with 256)
-  if (B <= 8) {
-    if (bf16) launch_sample<__nv_bfloat16, 1024>(logits, p, B, stream);
-    else launch_sample<float, 1024>(logits, p, B, stream);
-  } else {
-    if (bf16) launch_sample<__nv_bfloat16, 256>(logits, p, B, stream);
-    else launch_sample<float, 256>(logits, p, B, stream);
-  }
+  if (bf16) launch_sample<__nv_bfloat16>(logits, p, B, stream);
+  else launch_sample<float>(logits, p, B, stream);
 }
 
 // ---------------------------------------------------------------- grammar bitmask: logits[b, v] = -inf where bit == 0

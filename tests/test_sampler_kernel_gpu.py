@@ -1,5 +1,5 @@
 """The cluster sampler (csrc/kernels/sampling.cu) against a float64 oracle that draws with the same counter generator: every row's token and
-log-probability, at vocabularies around the slice, warp and vector edges, at batch sizes on both sides of the launch rule, for rows that ask for
+log-probability, at vocabularies around the slice, warp and vector edges, at several batch sizes, for rows that ask for
 different settings."""
 import pytest
 import torch
@@ -139,3 +139,21 @@ def test_plateaus(V, top_p, tail):
     assert a.elapsed_time(b) < 2.0, a.elapsed_time(b)
     for i in range(2):
         _check_row(logits[i], 1.0, 0, top_p, 0.0, _uniform(9, i, 2), int(tok[i]), float(lp[i]))
+
+
+def test_a_row_does_not_follow_its_batch():
+    """a seeded row's token and log-probability, bit for bit, alone and among others"""
+    B, V = 40, 128256
+    g = torch.Generator(device="cuda").manual_seed(21)
+    logits = (torch.randn(B, V, generator=g, device="cuda") * 2).to(torch.bfloat16)
+    kinds = [(1.0, 1, 1.0, 0.0), (0.7, 0, 0.9, 0.0), (0.8, 50, 0.95, 0.0), (1.0, 0, 1.0, 0.05), (1.3, 0, 1.0, 0.0)]
+    t, k, p, m = (torch.tensor([kinds[i % 5][j] for i in range(B)], device="cuda") for j in range(4))
+    seeds = torch.tensor([[77 + i, i] for i in range(B)], device="cuda")
+    def draw(n):
+        lp = torch.empty(n, device="cuda")
+        tok = ops.sample(logits[:n], t[:n].float(), k[:n].int(), p[:n].float(), m[:n].float(), seeds=seeds[:n], out_logprobs=lp, global_seed=4, step=n)
+        return tok, lp
+    tok, lp = draw(B)
+    for n in (1, 5, 8, 9, 17):
+        a, b = draw(n)
+        assert torch.equal(a, tok[:n]) and torch.equal(b, lp[:n])

@@ -1145,8 +1145,8 @@ void per_token_group_quant_fp8(const at::Tensor& x, at::Tensor q, at::Tensor sca
   count();
 }
 
-// out[M,N] bf16 = block-scaled (xq[M,K] e4m3, xs[M,K/128]) @ (wq[N,K] e4m3, ws[N/128,K/128])^T
-void gemm_fp8_block(const at::Tensor& xq, const at::Tensor& xs, const at::Tensor& wq, const at::Tensor& ws, at::Tensor out) {
+// out[M,N] bf16 = block-scaled (xq[M,K] e4m3, xs[M,K/128]) @ (wq[N,K] e4m3, ws[N/128,K/128])^T.  ``fixed_order``: a row's sums in one order whatever M is
+void gemm_fp8_block(const at::Tensor& xq, const at::Tensor& xs, const at::Tensor& wq, const at::Tensor& ws, at::Tensor out, bool fixed_order) {
   CHECK_CUDA(xq); CHECK_BF16(out); CHECK_LAST_CONTIG(xq); CHECK_LAST_CONTIG(wq); CHECK_LAST_CONTIG(out);
   TORCH_CHECK(xq.element_size() == 1 && wq.element_size() == 1 && xq.dim() == 2 && wq.dim() == 2 && xq.size(1) == wq.size(1));
   TORCH_CHECK(xs.scalar_type() == at::kFloat && ws.scalar_type() == at::kFloat && xs.stride(-1) == 1 && ws.stride(-1) == 1);
@@ -1156,13 +1156,13 @@ void gemm_fp8_block(const at::Tensor& xq, const at::Tensor& xs, const at::Tensor
   c10::cuda::CUDAGuard g(xq.device());
   sglb::gemm_fp8_block(xq.data_ptr(), xs.data_ptr<float>(), wq.data_ptr(), ws.data_ptr<float>(), out.data_ptr(), (int)xq.size(0),
                        (int)wq.size(0), (int)xq.size(1), (int)xq.stride(0), (int)wq.stride(0), (int)out.stride(0), (int)xs.stride(0),
-                       (int)ws.stride(0), num_sms(), cur_stream());
+                       (int)ws.stride(0), fixed_order, num_sms(), cur_stream());
   count();
 }
 
 // x[M,K] bf16 through the group quantiser and the block-scaled product in one call: a decode batch's two launches take less time than a second trip
 // through the dispatcher and three allocations from Python
-at::Tensor fp8_block_linear(const at::Tensor& x, const at::Tensor& wq, const at::Tensor& ws, bool ue8m0) {
+at::Tensor fp8_block_linear(const at::Tensor& x, const at::Tensor& wq, const at::Tensor& ws, bool ue8m0, bool fixed_order) {
   CHECK_CUDA(x);
   TORCH_CHECK(x.dim() == 2 && wq.dim() == 2);
   TORCH_CHECK(x.size(1) % 128 == 0, "fp8 block gemm: scale shapes must be [M, K/128] and [N/128, K/128]");
@@ -1171,7 +1171,7 @@ at::Tensor fp8_block_linear(const at::Tensor& x, const at::Tensor& wq, const at:
   auto s = at::empty({x.size(0), x.size(1) / 128}, x.options().dtype(at::kFloat));
   auto out = at::empty({x.size(0), wq.size(0)}, x.options());
   per_token_group_quant_fp8(x, q, s, 128, ue8m0);
-  gemm_fp8_block(q, s, wq, ws, out);
+  gemm_fp8_block(q, s, wq, ws, out, fixed_order);
   return out;
 }
 
@@ -1304,8 +1304,8 @@ TORCH_LIBRARY(sglb, m) {
   m.def("slab_reduce_add_rmsnorm(Tensor slabs, Tensor(a!)? residual, Tensor w, Tensor(b!) out, float eps, bool gemma) -> ()",
         &slab_reduce_add_rmsnorm);
   m.def("per_token_group_quant_fp8(Tensor x, Tensor(a!) q, Tensor(b!) scales, int group, bool ue8m0) -> ()", &per_token_group_quant_fp8);
-  m.def("fp8_block_linear(Tensor x, Tensor wq, Tensor ws, bool ue8m0) -> Tensor", &fp8_block_linear);
-  m.def("gemm_fp8_block(Tensor xq, Tensor xs, Tensor wq, Tensor ws, Tensor(a!) out) -> ()", &gemm_fp8_block);
+  m.def("fp8_block_linear(Tensor x, Tensor wq, Tensor ws, bool ue8m0, bool fixed_order=False) -> Tensor", &fp8_block_linear);
+  m.def("gemm_fp8_block(Tensor xq, Tensor xs, Tensor wq, Tensor ws, Tensor(a!) out, bool fixed_order=False) -> ()", &gemm_fp8_block);
   m.def("moe_topk_softmax(Tensor logits, Tensor(a!) out_w, Tensor(b!) out_ids, bool renorm) -> ()", &moe_topk_softmax);
   m.def("moe_grouped_mlp(Tensor x, Tensor w13, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset) -> ()",
         &moe_grouped_mlp);

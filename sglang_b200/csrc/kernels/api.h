@@ -81,7 +81,7 @@ void gemm_bf16_skinny_push(const void* A, const void* W, int M, int N, int K, in
 
 // gemm_fp8.cu
 void gemm_fp8_block(const void* A, const float* xs, const void* W, const float* ws, void* C, int M, int N, int K, int lda, int ldw,
-                    int ldc, int xs_stride, int ws_stride, int num_sms, cudaStream_t stream);
+                    int ldc, int xs_stride, int ws_stride, bool fixed_order, int num_sms, cudaStream_t stream);
 void per_token_group_quant_fp8(const void* x, void* q, float* scales, int M, int K, int x_stride, bool ue8m0, cudaStream_t stream);
 
 // moe.cu

@@ -393,16 +393,19 @@ static void launch_fp8_swap(const void* A, const float* xs, const void* W, const
 }
 
 void gemm_fp8_block(const void* A, const float* xs, const void* W, const float* ws, void* C, int M, int N, int K, int lda, int ldw,
-                    int ldc, int xs_stride, int ws_stride, int num_sms, cudaStream_t stream) {
+                    int ldc, int xs_stride, int ws_stride, bool fixed_order, int num_sms, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return;
   if (K % 16 || N % 8 || lda % 16 || ldw % 16) throw std::runtime_error("sglb fp8 gemm: K, lda, ldw must be multiples of 16 and N of 8");
 #define SGLB_F8(F) F(A, xs, W, ws, C, M, N, K, lda, ldw, ldc, xs_stride, ws_stride, num_sms, stream)
   // Up to 64 tokens: a promotion thread holds its weight row's 64 sums and an SM two CTAs.  128 sums leave one CTA an SM behind one serial chain, so
   // from 65 tokens on the rows of A are the M dimension.  us at [7168 x 8192] / [8192 x 3584] / [28672 x 4096] / [4096 x 14336], weights from memory:
   // 64 tokens 21 / 13 / 30 / 18 here, 27 / 14 / 26 / 44 there; 65 tokens 44 / 30 / 60 / 54 here (128 tokens wide), 27 / 15 / 26 / 44 there
-  if (M <= 16) { SGLB_F8(launch_fp8_swap<16>); return; }
-  if (M <= 32) { SGLB_F8(launch_fp8_swap<32>); return; }
-  if (M <= 64) { SGLB_F8(launch_fp8_swap<64>); return; }
+  // fixed_order: the swapped kernel's shares of K follow the token bucket, the other kernel adds K block by block at any M and width
+  if (!fixed_order) {
+    if (M <= 16) { SGLB_F8(launch_fp8_swap<16>); return; }
+    if (M <= 32) { SGLB_F8(launch_fp8_swap<32>); return; }
+    if (M <= 64) { SGLB_F8(launch_fp8_swap<64>); return; }
+  }
   // the width whose waves take the least time: a tile costs its columns plus a start and an end worth about 32 of them
   const int m_tiles = (M + F8_BM - 1) / F8_BM;
   int bn = 0;

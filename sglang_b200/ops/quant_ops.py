@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import torch
 
+from ..environ import envs
 from . import torch_ref
 
 
@@ -27,10 +28,10 @@ def per_token_group_quant_fp8(x: torch.Tensor, group: int = 128, ue8m0: bool = F
 def fp8_block_linear(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, block: int = 128, ue8m0: bool = False,
                      out_dtype=torch.bfloat16) -> torch.Tensor:
     if x.is_cuda and x.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and block == 128 and x.dim() == 2 and x.stride(1) == 1 and _has("fp8_block_linear"):
-        return torch.ops.sglb.fp8_block_linear(x, wq, ws, ue8m0)
+        return torch.ops.sglb.fp8_block_linear(x, wq, ws, ue8m0, envs.SGLB_FIXED_ORDER.get())
     xq, xs = per_token_group_quant_fp8(x, block, ue8m0)
     if x.is_cuda and _has("gemm_fp8_block"):
         out = torch.empty(x.shape[0], wq.shape[0], dtype=out_dtype, device=x.device)
-        torch.ops.sglb.gemm_fp8_block(xq, xs, wq, ws, out)
+        torch.ops.sglb.gemm_fp8_block(xq, xs, wq, ws, out, envs.SGLB_FIXED_ORDER.get())
         return out
     return torch_ref.fp8_block_gemm(xq, xs, wq, ws, block, out_dtype)

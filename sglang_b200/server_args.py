@@ -190,13 +190,15 @@ class ServerArgs:
         if self.enable_deterministic_inference:
             # reduction orders must not depend on what else is in the batch: no split-K / stream-K GEMM variants (their split count follows
             # the token count), one attention split per request (model_runner._pick_splits), the library all-reduce for every size (the
-            # size-based switch between the one-shot kernel and NCCL changes the summation order with the batch)
+            # size-based switch between the one-shot kernel and NCCL changes the summation order with the batch), and the one form of the own
+            # kernels that have several (SGLB_FIXED_ORDER)
             import os as _os
 
             _os.environ["SGLB_SKINNY"] = "off"
             _os.environ["SGLB_STREAMK_MAX_M"] = "0"
             _os.environ["SGLB_TP_LIBRARY_AR_MIN_BYTES"] = "0"
             _os.environ["SGLB_RS_AG_MIN_BYTES"] = "0"
+            _os.environ["SGLB_FIXED_ORDER"] = "1"
         if self.model_impl not in ("auto", "sglang", "transformers"):
             raise ValueError("--model-impl must be auto, sglang or transformers")
         if self.model_impl != "auto":          # travels with the other config overrides to every process that reads the model config

@@ -178,3 +178,16 @@ def test_deterministic_inference_flag_pins_reduction_orders(monkeypatch):
     finally:
         eng.runner.is_cuda = False
         eng.shutdown()
+
+
+def test_deterministic_inference_flag_asks_for_one_kernel_form(monkeypatch):
+    from sglang_b200.environ import envs
+    from sglang_b200.server_args import ServerArgs
+
+    for k in ("SGLB_SKINNY", "SGLB_STREAMK_MAX_M", "SGLB_TP_LIBRARY_AR_MIN_BYTES", "SGLB_RS_AG_MIN_BYTES", "SGLB_FIXED_ORDER"):
+        monkeypatch.setenv(k, "1")                    # (whatever the flag sets is undone)
+        monkeypatch.delenv(k)
+    ServerArgs(model_path="dummy:tiny-llama")
+    assert not envs.SGLB_FIXED_ORDER.get()
+    ServerArgs(model_path="dummy:tiny-llama", enable_deterministic_inference=True)
+    assert envs.SGLB_FIXED_ORDER.get()

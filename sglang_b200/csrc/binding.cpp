@@ -1192,7 +1192,7 @@ void moe_topk_softmax(const at::Tensor& logits, at::Tensor out_w, at::Tensor out
 void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, const at::Tensor& topk_w,
                           const at::Tensor& topk_ids, c10::optional<at::Tensor> out, int64_t expert_offset,
                           const int64_t* peer_slots, const int64_t* peer_flags, int rank, int world, const uint32_t* epoch,
-                          uint32_t* done, int act = 0, float act_limit = 0.f, float act_alpha = 0.f, bool weight_input = false) {
+                          uint32_t* done, bool fixed_order, int act = 0, float act_limit = 0.f, float act_alpha = 0.f, bool weight_input = false) {
   CHECK_CUDA(x); CHECK_BF16(x); CHECK_BF16(w13); CHECK_BF16(w2); CHECK_I32(topk_ids); CHECK_LAST_CONTIG(x);
   TORCH_CHECK(x.dim() == 2 && w13.dim() == 3 && w2.dim() == 3 && w13.is_contiguous() && w2.is_contiguous());
   TORCH_CHECK(topk_w.scalar_type() == at::kFloat && topk_w.is_contiguous() && topk_ids.is_contiguous());
@@ -1207,7 +1207,8 @@ void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::
   // 8 experts of 4096 x 14336, 2 chosen: 492 / 624 at 24 rows, 492 / 542 at 32, 538 / 542 at 40, 552 / 549 at 48, 560 / 550 at 56, 606 / 536 at 64;
   // 128 experts of 2048 x 768, 8 chosen: 291 / 320 at 32, 340 / 358 at 44, 352 / 360 at 48, 371 / 370 at 56, 396 / 386 at 64.  Under expert parallelism
   // the pairs are those of all ranks, so the line is met sooner by their number.
-  const bool decode = pairs <= 48ll * E;
+  // fixed_order: the first kernel's tiles and shares of K follow the number of pairs, the 128-row kernel adds a row's K in one order whatever they are.
+  const bool decode = !fixed_order && pairs <= 48ll * E;
   int tile = 128;
   if (decode)
     for (int t : {16, 32, 64, 128}) {
@@ -1262,30 +1263,32 @@ void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::
 }
 
 void moe_grouped_mlp(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, const at::Tensor& topk_w,
-                     const at::Tensor& topk_ids, at::Tensor out, int64_t expert_offset) {
+                     const at::Tensor& topk_ids, at::Tensor out, int64_t expert_offset, bool fixed_order) {
   CHECK_BF16(out);
-  moe_grouped_mlp_impl(x, w13, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr);
+  moe_grouped_mlp_impl(x, w13, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, fixed_order);
 }
 
 void moe_grouped_mlp_glu(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, const at::Tensor& topk_w,
-                         const at::Tensor& topk_ids, at::Tensor out, int64_t expert_offset, double limit, double alpha) {
+                         const at::Tensor& topk_ids, at::Tensor out, int64_t expert_offset, double limit, double alpha,
+                         bool fixed_order) {
   CHECK_BF16(out);
-  moe_grouped_mlp_impl(x, w13, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, 1, (float)limit, (float)alpha);
+  moe_grouped_mlp_impl(x, w13, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, fixed_order, 1, (float)limit,
+                       (float)alpha);
 }
 
 void moe_grouped_mlp_relu2(const at::Tensor& x, const at::Tensor& w1, const at::Tensor& w2, const at::Tensor& topk_w, const at::Tensor& topk_ids,
-                           at::Tensor out, int64_t expert_offset, bool weight_input) {
+                           at::Tensor out, int64_t expert_offset, bool weight_input, bool fixed_order) {
   CHECK_BF16(out);
-  moe_grouped_mlp_impl(x, w1, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, 2, 0.f, 0.f, weight_input);
+  moe_grouped_mlp_impl(x, w1, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, fixed_order, 2, 0.f, 0.f, weight_input);
 }
 
 void moe_grouped_mlp_push(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, const at::Tensor& topk_w,
                           const at::Tensor& topk_ids, int64_t expert_offset, const at::Tensor& peer_slot_ptrs,
-                          const at::Tensor& peer_flag_ptrs, int64_t rank, int64_t world, at::Tensor epoch, at::Tensor done) {
+                          const at::Tensor& peer_flag_ptrs, int64_t rank, int64_t world, at::Tensor epoch, at::Tensor done, bool fixed_order) {
   TORCH_CHECK(!peer_slot_ptrs.is_cuda() && !peer_flag_ptrs.is_cuda());
   moe_grouped_mlp_impl(x, w13, w2, topk_w, topk_ids, c10::nullopt, expert_offset, peer_slot_ptrs.data_ptr<int64_t>(),
                        peer_flag_ptrs.data_ptr<int64_t>(), (int)rank, (int)world, reinterpret_cast<const uint32_t*>(epoch.data_ptr<int>()),
-                       reinterpret_cast<uint32_t*>(done.data_ptr<int>()));
+                       reinterpret_cast<uint32_t*>(done.data_ptr<int>()), fixed_order);
 }
 
 }  // namespace
@@ -1307,12 +1310,12 @@ TORCH_LIBRARY(sglb, m) {
   m.def("fp8_block_linear(Tensor x, Tensor wq, Tensor ws, bool ue8m0, bool fixed_order=False) -> Tensor", &fp8_block_linear);
   m.def("gemm_fp8_block(Tensor xq, Tensor xs, Tensor wq, Tensor ws, Tensor(a!) out, bool fixed_order=False) -> ()", &gemm_fp8_block);
   m.def("moe_topk_softmax(Tensor logits, Tensor(a!) out_w, Tensor(b!) out_ids, bool renorm) -> ()", &moe_topk_softmax);
-  m.def("moe_grouped_mlp(Tensor x, Tensor w13, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset) -> ()",
+  m.def("moe_grouped_mlp(Tensor x, Tensor w13, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset, bool fixed_order=False) -> ()",
         &moe_grouped_mlp);
   m.def("moe_grouped_mlp_glu(Tensor x, Tensor w13, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset, float limit, "
-        "float alpha) -> ()", &moe_grouped_mlp_glu);
+        "float alpha, bool fixed_order=False) -> ()", &moe_grouped_mlp_glu);
   m.def("moe_grouped_mlp_push(Tensor x, Tensor w13, Tensor w2, Tensor topk_w, Tensor topk_ids, int expert_offset, Tensor peer_slot_ptrs, "
-        "Tensor peer_flag_ptrs, int rank, int world, Tensor(a!) epoch, Tensor(b!) done) -> ()", &moe_grouped_mlp_push);
+        "Tensor peer_flag_ptrs, int rank, int world, Tensor(a!) epoch, Tensor(b!) done, bool fixed_order=False) -> ()", &moe_grouped_mlp_push);
   m.def("gemm_push(Tensor a, Tensor w, Tensor peer_slot_ptrs, Tensor peer_flag_ptrs, int rank, int world, Tensor(a!) epoch, "
         "Tensor(b!) done, int bn) -> ()", &gemm_push);
   m.def("nvl_local_reduce_add_rmsnorm(Tensor slot, int flags_ptr, Tensor(a!)? residual, Tensor w, Tensor(b!) out, int world, int nslabs, float eps, "
@@ -1380,7 +1383,7 @@ TORCH_LIBRARY(sglb, m) {
         "Tensor(c!) v_cache, Tensor loc, Tensor(d!) q_out, int pad=0) -> ()", &conv_attention_prepare);
   m.def("norm_add_f32(Tensor(a!) x, Tensor src, Tensor? ids, Tensor w, Tensor(b!)? out, float eps, bool zero_centred=True) -> ()", &norm_add_f32);
   m.def("moe_sigmoid_route(Tensor logits, bool renorm, float scale, Tensor(a!) w, Tensor(b!) ids) -> ()", &moe_sigmoid_route);
-  m.def("moe_grouped_mlp_relu2(Tensor x, Tensor w1, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset, bool weight_input) -> ()",
+  m.def("moe_grouped_mlp_relu2(Tensor x, Tensor w1, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset, bool weight_input, bool fixed_order=False) -> ()",
         &moe_grouped_mlp_relu2);
   m.def("attention_sink_gate(Tensor o, Tensor lse, Tensor sinks, int Dv, Tensor(a!) out) -> ()", &attention_sink_gate);
   m.def("moe_softmax_bias_route(Tensor logits, Tensor? corr, int n_real, Tensor(a!) w, Tensor(b!) ids, Tensor(c!) ident) -> ()", &moe_softmax_bias_route);

@@ -11,6 +11,7 @@ from typing import Tuple
 
 import torch
 
+from ..environ import envs
 from . import silu_and_mul, linear, torch_ref
 
 
@@ -41,7 +42,7 @@ def fused_moe(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_w: torc
         if (x.is_cuda and x.dtype == torch.bfloat16 and _has("moe_grouped_mlp_relu2") and H % 32 == 0 and I % 32 == 0 and w13.shape[0] <= 512
                 and x.stride(1) == 1 and x.stride(0) % 8 == 0):
             out = torch.empty_like(x)
-            torch.ops.sglb.moe_grouped_mlp_relu2(x, w13, w2, topk_w, topk_ids, out, expert_offset, weight_input)
+            torch.ops.sglb.moe_grouped_mlp_relu2(x, w13, w2, topk_w, topk_ids, out, expert_offset, weight_input, envs.SGLB_FIXED_ORDER.get())
             return out
         if not x.is_cuda:
             return torch_ref.fused_moe(x, w13, w2, topk_w, topk_ids, expert_offset, fn, weight_input)
@@ -59,11 +60,11 @@ def fused_moe(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_w: torc
             and x.stride(0) % 8 == 0):
         # expert-sorted rows through the tcgen05 grouped GEMMs, no host sync: align -> gather -> gate|up GEMM -> clamped GLU -> down GEMM -> combine
         out = torch.empty_like(x)
-        torch.ops.sglb.moe_grouped_mlp_glu(x, w13, w2, topk_w, topk_ids, out, expert_offset, float(limit), float(alpha))
+        torch.ops.sglb.moe_grouped_mlp_glu(x, w13, w2, topk_w, topk_ids, out, expert_offset, float(limit), float(alpha), envs.SGLB_FIXED_ORDER.get())
         return out
     if act is None and x.dtype == torch.bfloat16 and _has("moe_grouped_mlp") and H % 32 == 0 and I % 32 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0:
         out = torch.empty_like(x)
-        torch.ops.sglb.moe_grouped_mlp(x, w13, w2, topk_w, topk_ids, out, expert_offset)
+        torch.ops.sglb.moe_grouped_mlp(x, w13, w2, topk_w, topk_ids, out, expert_offset, envs.SGLB_FIXED_ORDER.get())
         return out
     return _fused_moe_sorted(x, w13, w2, topk_w, topk_ids, expert_offset, fn)
 

@@ -200,7 +200,7 @@ class NvlComm:
         off = self._slot(ch)
         torch.ops.sglb.moe_grouped_mlp_push(x, w13, w2, topk_w, topk_ids, expert_offset, self.buf_ptrs + off,
                                             self.flag_ptrs + ch * MAX_RANKS * 4, self.rank, self.world, self.epochs[ch:ch + 1],
-                                            self.done[ch, 1:])
+                                            self.done[ch, 1:], envs.SGLB_FIXED_ORDER.get())
         self.calls += 1
         return off
 

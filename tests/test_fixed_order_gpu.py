@@ -5,7 +5,7 @@ import torch
 
 from sglang_b200 import ops
 from sglang_b200.environ import envs
-from sglang_b200.ops import quant_ops, torch_ref
+from sglang_b200.ops import moe_ops, quant_ops, torch_ref
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +30,18 @@ def test_fp8_products(N, K):
         out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
         torch.ops.sglb.gemm_fp8_block(xq, xs, wq, ws, out, True)
         assert torch.equal(out, whole[:M]), M
+
+
+@pytest.mark.parametrize("E,top,H,I", [(8, 2, 1024, 2048), (64, 4, 256, 96)])
+@pytest.mark.parametrize("act", [None, ("relu2",), ("clamped_glu", 4.0, 1.702)])
+def test_expert_blocks(E, top, H, I, act):
+    """row tiles of 16 to 128, shared K, the line between the two kernels"""
+    g = torch.Generator(device="cuda").manual_seed(E)
+    T = 60 * E // top                                              # beyond the line
+    x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+    w13 = (torch.randn(E, I if act == ("relu2",) else 2 * I, H, generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    w2 = (torch.randn(E, H, I, generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    w, ids = moe_ops.topk_softmax(torch.randn(T, E, generator=g, device="cuda"), top, True)
+    whole = moe_ops.fused_moe(x, w13, w2, w, ids, act=act)
+    for M in (1, 5, 2 * E // top, 10 * E // top, 30 * E // top, 47 * E // top, 49 * E // top):
+        assert torch.equal(moe_ops.fused_moe(x[:M], w13, w2, w[:M].contiguous(), ids[:M].contiguous(), act=act), whole[:M]), M

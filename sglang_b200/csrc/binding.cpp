@@ -442,7 +442,7 @@ void rglru_scan(const at::Tensor& gates, c10::optional<at::Tensor> bias, const a
 void mamba2_scan(const at::Tensor& u, c10::optional<at::Tensor> z, c10::optional<at::Tensor> dt_raw, c10::optional<at::Tensor> dt_bias,
                  c10::optional<at::Tensor> A_log, c10::optional<at::Tensor> D, at::Tensor state, const at::Tensor& req_slots, const at::Tensor& seq_lens,
                  c10::optional<at::Tensor> cu_q, int64_t H, int64_t P, int64_t N, int64_t G, at::Tensor out, c10::optional<at::Tensor> decay,
-                 c10::optional<at::Tensor> gates) {
+                 c10::optional<at::Tensor> gates, bool fixed_order) {
   CHECK_CUDA(u); CHECK_I32(req_slots); CHECK_I32(seq_lens);
   auto f32c = [](const at::Tensor& t) { return t.scalar_type() == at::kFloat && t.is_contiguous(); };
   TORCH_CHECK(f32c(u) && f32c(state) && f32c(out) && u.dim() == 2 && u.size(1) >= H * P + 2 * G * N);
@@ -468,10 +468,12 @@ void mamba2_scan(const at::Tensor& u, c10::optional<at::Tensor> z, c10::optional
   if (cu_q.has_value()) { CHECK_I32(*cu_q); TORCH_CHECK(cu_q->numel() == B + 1); } else TORCH_CHECK(u.size(0) == B);
   if (u.size(0) == 0) return;
   c10::cuda::CUDAGuard g(u.device());
+  // fixed_order: sums over eight tokens follow where a prompt is cut and whom it shares the batch with, so every request goes token by token, as batches of
+  // one token a request do
   sglb::mamba2_scan(u.data_ptr<float>(), (int)u.stride(0), z.has_value() ? z->data_ptr() : nullptr, z.has_value() ? (int)z->stride(0) : 0,
                     fixed ? nullptr : dt_raw->data_ptr(), fixed ? 0 : (int)dt_raw->stride(0), in_bf16,
                     fixed ? nullptr : dt_bias->data_ptr<float>(), fixed ? nullptr : A_log->data_ptr<float>(), opt_ptr<float>(D),
-                    state.data_ptr<float>(), req_slots.data_ptr<int>(), seq_lens.data_ptr<int>(), opt_ptr<int>(cu_q), B, (int)u.size(0), (int)H, (int)P, (int)N,
+                    state.data_ptr<float>(), req_slots.data_ptr<int>(), seq_lens.data_ptr<int>(), opt_ptr<int>(cu_q), B, fixed_order ? B : (int)u.size(0), (int)H, (int)P, (int)N,
                     (int)G, out.data_ptr<float>(), opt_ptr<float>(decay), opt_ptr<float>(gates), gates.has_value() ? (int)gates->size(2) : 0, cur_stream());
   count();
 }
@@ -1364,7 +1366,7 @@ TORCH_LIBRARY(sglb, m) {
   m.def("rglru_scan(Tensor gates, Tensor? bias, Tensor u, Tensor lam, Tensor y, Tensor(a!) state, Tensor req_slots, Tensor seq_lens, Tensor? cu_q, int blocks, "
         "float power, Tensor(b!) out) -> ()", &rglru_scan);
   m.def("mamba2_scan(Tensor u, Tensor? z, Tensor? dt_raw, Tensor? dt_bias, Tensor? A_log, Tensor? D, Tensor(a!) state, Tensor req_slots, Tensor seq_lens, "
-        "Tensor? cu_q, int H, int P, int N, int G, Tensor(b!) out, Tensor? decay=None, Tensor? gates=None) -> ()", &mamba2_scan);
+        "Tensor? cu_q, int H, int P, int N, int G, Tensor(b!) out, Tensor? decay=None, Tensor? gates=None, bool fixed_order=False) -> ()", &mamba2_scan);
   m.def("mamba1_scan(Tensor u, Tensor dt_raw, Tensor? dt_bias, Tensor A_log, Tensor Bm, Tensor Cm, Tensor? D, Tensor? z, Tensor(a!) state, Tensor req_slots, "
         "Tensor seq_lens, Tensor? cu_q, Tensor(b!) out) -> ()", &mamba1_scan);
   m.def("attention_prepare(Tensor qkv, int H, int G, int D, int Dv, Tensor positions, Tensor(a!) k_cache, Tensor(b!) v_cache, Tensor loc, Tensor? q_norm_w, "

@@ -593,12 +593,16 @@ def mamba2_scan(u: torch.Tensor, z: Optional[torch.Tensor], dt_raw: Optional[tor
             and (z is None or (z.stride(1) == 1 and z.dtype in (torch.bfloat16, torch.float32) and (fixed or z.dtype == dt_raw.dtype)))):
         out = torch.empty(u.shape[0], H * P, dtype=torch.float32, device=u.device)
         f = lambda t: None if t is None else t.float().contiguous()
+        fixed_order = envs.SGLB_FIXED_ORDER.get()
         if gates is not None:
-            torch.ops.sglb.mamba2_scan(u, z, None, None, None, f(D), state, req_slots, seq_lens, cu_q, int(H), int(P), int(N), int(G), out, None, gates)
+            torch.ops.sglb.mamba2_scan(u, z, None, None, None, f(D), state, req_slots, seq_lens, cu_q, int(H), int(P), int(N), int(G), out, None, gates,
+                                       fixed_order)
         elif decay is not None:
-            torch.ops.sglb.mamba2_scan(u, z, None, None, None, f(D), state, req_slots, seq_lens, cu_q, int(H), int(P), int(N), int(G), out, f(decay), None)
+            torch.ops.sglb.mamba2_scan(u, z, None, None, None, f(D), state, req_slots, seq_lens, cu_q, int(H), int(P), int(N), int(G), out, f(decay), None,
+                                       fixed_order)
         else:
-            torch.ops.sglb.mamba2_scan(u, z, dt_raw, f(dt_bias), f(A_log), f(D), state, req_slots, seq_lens, cu_q, int(H), int(P), int(N), int(G), out, None, None)
+            torch.ops.sglb.mamba2_scan(u, z, dt_raw, f(dt_bias), f(A_log), f(D), state, req_slots, seq_lens, cu_q, int(H), int(P), int(N), int(G), out, None, None,
+                                       fixed_order)
         return out
     return torch_ref.mamba2_scan(u, z, dt_raw, dt_bias, A_log, D, state, req_slots, seq_lens, q_lens, H, P, N, G, decay, gates)
 

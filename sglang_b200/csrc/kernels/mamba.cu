@@ -544,8 +544,8 @@ __global__ void __launch_bounds__(128) mamba2_scan_kernel(const Mamba2Params p) 
 // decays are products of at most eight factors of the tokens' own (never quotients or exponentials of differences), so nothing cancels.
 // A CTA owns 64 columns of a head: lane l holds columns 2l, 2l + 1 of its warp's 16 state rows, B and C are read from shared memory as broadcasts and
 // the warps' partial read-outs meet there.  One more warp brings the next block and works out its steps and decays.
-// Bound by the chain of blocks of the longest request (about 2 us each: two barriers around dependent multiply-adds) and by what shared memory hands to
-// registers.  3001 tokens in 5 requests, 64 heads of 64 x 128: 776 us token by token, 585 us in blocks (649 with four warps of 32 rows that also did
+// Bound by the chain of blocks of the longest request (two barriers around dependent multiply-adds; its 153 blocks are the tail of the launch below, at
+// less than 3.8 us each) and by what shared memory hands to registers.  3001 tokens in 5 requests, 64 heads of 64 x 128: 776 us token by token, 585 us in blocks (649 with four warps of 32 rows that also did
 // the loading; 724 with 8 x 8 tiles in four warps, whose longer chains cost more than their fewer reads saved).
 typedef unsigned long long f2;
 __device__ __forceinline__ f2 f2_pack(float a, float b) {

@@ -470,11 +470,16 @@ void mamba2_scan(const at::Tensor& u, c10::optional<at::Tensor> z, c10::optional
   c10::cuda::CUDAGuard g(u.device());
   // fixed_order: sums over eight tokens follow where a prompt is cut and whom it shares the batch with, so every request goes token by token, as batches of
   // one token a request do
+  const int tokens = fixed_order ? B : (int)u.size(0);
+  at::Tensor ws;
+  if (const size_t bytes = sglb::mamba2_scan_workspace(u.data_ptr<float>(), (int)u.stride(0), cu_q.has_value(), B, tokens, (int)H, (int)P, (int)N, (int)G))
+    ws = at::empty({(int64_t)bytes}, u.options().dtype(at::kByte));
   sglb::mamba2_scan(u.data_ptr<float>(), (int)u.stride(0), z.has_value() ? z->data_ptr() : nullptr, z.has_value() ? (int)z->stride(0) : 0,
                     fixed ? nullptr : dt_raw->data_ptr(), fixed ? 0 : (int)dt_raw->stride(0), in_bf16,
                     fixed ? nullptr : dt_bias->data_ptr<float>(), fixed ? nullptr : A_log->data_ptr<float>(), opt_ptr<float>(D),
-                    state.data_ptr<float>(), req_slots.data_ptr<int>(), seq_lens.data_ptr<int>(), opt_ptr<int>(cu_q), B, fixed_order ? B : (int)u.size(0), (int)H, (int)P, (int)N,
-                    (int)G, out.data_ptr<float>(), opt_ptr<float>(decay), opt_ptr<float>(gates), gates.has_value() ? (int)gates->size(2) : 0, cur_stream());
+                    state.data_ptr<float>(), req_slots.data_ptr<int>(), seq_lens.data_ptr<int>(), opt_ptr<int>(cu_q), B, tokens, (int)H, (int)P, (int)N, (int)G,
+                    out.data_ptr<float>(), opt_ptr<float>(decay), opt_ptr<float>(gates), gates.has_value() ? (int)gates->size(2) : 0,
+                    ws.defined() ? ws.data_ptr() : nullptr, cur_stream());
   count();
 }
 

@@ -138,7 +138,8 @@ void attention_sink_gate(const void* o, int ldo, const float* lse, const float* 
 // mamba.cu (ragged Mamba-2 recurrence), residual_f32.cu (sandwich norms), elementwise.cu (bigram embedding), moe.cu (identity / shared experts)
 void mamba2_scan(const float* u, int ldu, const void* z, int ldz, const void* dt_raw, int lddt, bool bf16, const float* dt_bias, const float* A_log,
                  const float* D, float* state, const int* req_slots, const int* seq_lens, const int* cu_q, int B, int T, int H, int P, int N, int G, float* out,
-                 const float* decay, const float* gates, int gstride, cudaStream_t stream);
+                 const float* decay, const float* gates, int gstride, void* ws, cudaStream_t stream);
+size_t mamba2_scan_workspace(const float* u, int ldu, bool ragged, int B, int T, int H, int P, int N, int G);      // 0: none needed
 void mlstm_prepare(const void* proj, int ld, bool bf16, const float* raw, int T, int B, int H, int D, int Dv, float cap, float* mstate, const int* req_slots,
                    const int* seq_lens, const int* cu_q, float* u, float* gates, cudaStream_t stream);
 void mlstm_readout(const float* y, const float* gates, int T, int H, int Dv, const void* w, float eps, const void* gate, int ldg, void* out, bool out_bf16,

@@ -14,6 +14,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "mamba2.h"
 #include "tma_host.h"
 
 namespace sglb {
@@ -352,20 +353,6 @@ bool gated_delta_update(float* state, const int* req_slots, const float* u, int 
 // Reference counterpart: layers/attention/mamba/ops (chunked SSD scan for prompts, selective_state_update for decode).
 namespace {
 
-struct Mamba2Params {
-  const float* u; int ldu;                       // conv outputs [T, ldu] = [x (H*P) | B (G*N) | C (G*N)]
-  const void* z; int ldz;                        // gate rows (model dtype) or null
-  const void* dt_raw; int lddt;                  // [T, >= H] (model dtype)
-  const float* dt_bias; const float* A_log; const float* D;
-  const float* decay;                            // non-null: step size 1 and the head's constant decay (dt_raw, dt_bias, A_log unused)
-  const float* gates; int gstride;               // non-null: [T, H, gstride] with every token's decay at [0] and step at [1] (likewise)
-  float* state;                                  // [slots, H, N, P]
-  const int* req_slots; const int* seq_lens; const int* cu_q;
-  float* out;                                    // [T, H*P]
-  int H, P, N, G, pchunks;
-};
-
-__device__ __forceinline__ float m2_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ void m2_cp4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
@@ -537,15 +524,15 @@ __global__ void __launch_bounds__(128) mamba2_scan_kernel(const Mamba2Params p) 
   }
 }
 
-// ---------------------------------------------------------------- prompts: eight tokens a step
+// ---------------------------------------------------------------- short prompts: eight tokens a step
 // The recurrence token by token costs three multiply-adds per state element and token and a serial step per token.  Over a block of eight tokens it is
 //   y_t = (decay 0..t) C_t S  +  sum_{s <= t} (decay s+1..t) (C_t . B_s) dt_s x_s  + D x_t          S <- (decay of all) S + sum_s (decay s+1..7) dt_s B_s x_s^T
 // with the same fp32 sums in another order: two multiply-adds per element and token, packed two to an instruction, eight tokens per barrier pair.  The
 // decays are products of at most eight factors of the tokens' own (never quotients or exponentials of differences), so nothing cancels.
 // A CTA owns 64 columns of a head: lane l holds columns 2l, 2l + 1 of its warp's 16 state rows, B and C are read from shared memory as broadcasts and
 // the warps' partial read-outs meet there.  One more warp brings the next block and works out its steps and decays.
-// Bound by the chain of blocks of the longest request (two barriers around dependent multiply-adds; its 153 blocks are the tail of the launch below, at
-// less than 3.8 us each) and by what shared memory hands to registers.  3001 tokens in 5 requests, 64 heads of 64 x 128: 776 us token by token, 585 us in blocks (649 with four warps of 32 rows that also did
+// Bound by the chain of blocks of the longest request (two barriers around dependent multiply-adds) and by what shared memory hands to registers; longer
+// prompts take the kernel in mamba_chunk.cu.  3001 tokens in 5 requests, 64 heads of 64 x 128: 776 us token by token, 585 us in blocks (649 with four warps of 32 rows that also did
 // the loading; 724 with 8 x 8 tiles in four warps, whose longer chains cost more than their fewer reads saved).
 typedef unsigned long long f2;
 __device__ __forceinline__ f2 f2_pack(float a, float b) {
@@ -818,9 +805,16 @@ void dispatch_m2(const Mamba2Params& p, int B, int T, cudaStream_t stream) {
 
 }  // namespace
 
+// Prompts go 64 tokens a step from 24 tokens a request and 24 more on.  us there / eight tokens a step, 64 heads of 64 x 128: one request of 24 tokens
+// 21.5 / 17.4, 40: 22.6 / 21.6, 64: 24.6 / 29.7; four requests of 64 tokens in all 25.6 / 23.6, 128: 29.7 / 37.2; twelve of 192: 48 / 42, 288: 50 / 50,
+// 480: 53 / 73 (16 heads of 128 x 128 cross at the same lengths)
+size_t mamba2_scan_workspace(const float* u, int ldu, bool ragged, int B, int T, int H, int P, int N, int G) {
+  return ragged && T >= 24ll * (B + 1) ? mamba2_chunk_workspace(u, ldu, B, T, H, P, N, G) : 0;
+}
+
 void mamba2_scan(const float* u, int ldu, const void* z, int ldz, const void* dt_raw, int lddt, bool bf16, const float* dt_bias, const float* A_log,
                  const float* D, float* state, const int* req_slots, const int* seq_lens, const int* cu_q, int B, int T, int H, int P, int N, int G, float* out,
-                 const float* decay, const float* gates, int gstride, cudaStream_t stream) {
+                 const float* decay, const float* gates, int gstride, void* ws, cudaStream_t stream) {
   if (B <= 0) return;
   if (N > 1024 || B > 65535 || H % G) throw std::runtime_error("sglb mamba2_scan: state size up to 1024, heads a multiple of groups");
   if (!decay && !gates && (!dt_raw || !dt_bias || !A_log)) throw std::runtime_error("sglb mamba2_scan: step-size inputs, a constant decay or per-token gates");
@@ -828,7 +822,8 @@ void mamba2_scan(const float* u, int ldu, const void* z, int ldz, const void* dt
   p.decay = decay; p.gates = gates; p.gstride = gstride;
   p.u = u; p.ldu = ldu; p.z = z; p.ldz = ldz; p.dt_raw = dt_raw; p.lddt = lddt; p.dt_bias = dt_bias; p.A_log = A_log; p.D = D; p.state = state;
   p.req_slots = req_slots; p.seq_lens = seq_lens; p.cu_q = cu_q; p.out = out; p.H = H; p.P = P; p.N = N; p.G = G; p.pchunks = 1;
-  if (bf16) dispatch_m2<__nv_bfloat16>(p, B, T, stream);
+  if (ws) mamba2_chunk_scan(p, bf16, B, T, ws, stream);
+  else if (bf16) dispatch_m2<__nv_bfloat16>(p, B, T, stream);
   else dispatch_m2<float>(p, B, T, stream);
 }
 

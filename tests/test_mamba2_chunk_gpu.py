@@ -1,0 +1,117 @@
+"""The 64-token form of the Mamba-2 recurrence (csrc/kernels/mamba_chunk.cu) against float64: lengths around the chunk, one and two heads a CTA, both state
+sizes, every source of step and decay; its error must be that of fp32 sums.  Values that are not finite stay with their column and the tokens behind them."""
+import pytest
+import torch
+
+from sglang_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _i32(v):
+    return torch.tensor(v, dtype=torch.int32, device="cuda")
+
+
+def _inputs(H, P, N, G, lens, mode, dt_t, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    T, B = sum(lens), len(lens)
+    u = torch.nn.functional.silu(rnd(T, H * P + 2 * G * N))
+    z = rnd(T, H * P + 8).to(dt_t)[:, : H * P] if mode != "decay" else None
+    D = 1 + 0.1 * rnd(H) if mode != "gates" else None
+    state = rnd(B + 2, H, N, P)
+    kw, args = {}, (None, None, None)
+    if mode == "step":
+        raw, bias, A_log = rnd(T, H).to(dt_t), rnd(H) - 3, rnd(H).abs()
+        args = (raw, bias, A_log)
+        dt = torch.log1p(torch.exp(raw.double() + bias.double()))
+        da = torch.exp(-A_log.double().exp() * dt)
+    elif mode == "decay":
+        kw["decay"] = torch.rand(H, generator=g, device="cuda") * 0.2 + 0.8
+        dt, da = torch.ones(T, H, device="cuda", dtype=torch.float64), kw["decay"].double().expand(T, H)
+    else:                                                        # (a decay of zero forgets everything: no logarithm of it may be taken)
+        kw["gates"] = torch.rand(T, H, 3, generator=g, device="cuda").masked_fill_(torch.rand(T, H, 1, generator=g, device="cuda") < 0.02, 0.0).contiguous()
+        da, dt = kw["gates"][..., 0].double(), kw["gates"][..., 1].double()
+    old = [50 if i % 2 else 0 for i in range(B)]
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    rows = [B - i for i in range(B)]
+    call = lambda st, **more: ops.mamba2_scan(u, z, *args, D, st, _i32(rows), _i32([a + b for a, b in zip(lens, old)]), _i32(cu), _i32(lens),  # noqa: E731
+                                              H, P, N, G, **kw, **more)
+    return u, z, D, dt, da, state, old, cu, rows, call
+
+
+def _oracle(H, P, N, G, lens, u, z, D, dt, da, state, old, cu, rows):
+    x, b, c = u.double().split([H * P, G * N, G * N], dim=-1)
+    x, b, c = x.view(-1, H, P), b.view(-1, G, N).repeat_interleave(H // G, 1), c.view(-1, G, N).repeat_interleave(H // G, 1)
+    ref, s0 = torch.empty_like(x), state.double().clone()
+    for r, n in enumerate(lens):
+        S = s0[rows[r]] if old[r] else torch.zeros_like(s0[0])
+        for t in range(cu[r], cu[r + 1]):
+            S = S * da[t][:, None, None] + (dt[t][:, None] * b[t])[:, :, None] * x[t][:, None, :]
+            ref[t] = torch.einsum("hnp,hn->hp", S, c[t])
+        s0[rows[r]] = S
+    if D is not None:
+        ref = ref + D.double()[None, :, None] * x
+    ref = ref.view(-1, H * P)
+    return (ref if z is None else ref * torch.nn.functional.silu(z.double())), s0
+
+
+@pytest.mark.parametrize("H,P,N,G", [(8, 64, 128, 2), (2, 64, 64, 1), (2, 128, 128, 2), (3, 256, 64, 1)])
+@pytest.mark.parametrize("lens", [[48], [64], [65, 0, 63], [1, 128, 130, 7], [31, 33, 1, 200]])
+@pytest.mark.parametrize("mode", ["step", "decay", "gates"])
+@pytest.mark.parametrize("bf16", [True, False])
+def test_against_float64(H, P, N, G, lens, mode, bf16):
+    u, z, D, dt, da, state, old, cu, rows, call = _inputs(H, P, N, G, lens, mode, torch.bfloat16 if bf16 else torch.float32, sum(lens) * 13 + H)
+    ref, s0 = _oracle(H, P, N, G, lens, u, z, D, dt, da, state, old, cu, rows)
+    y = call(state)
+    # fp32 sums of N products and of up to 64 tokens: a few 2^-24 of the whole in the 2-norm
+    for got, want in ((y, ref), (state, s0)):
+        assert float((got.double() - want).norm() / want.norm()) < 6e-7, float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan"), 3.4e38])
+def test_values_that_are_not_finite_stay_behind(bad):
+    H, P, N, G, lens = 4, 64, 128, 1, [100, 90]
+    u, z, D, dt, da, state, old, cu, rows, call = _inputs(H, P, N, G, lens, "step", torch.float32, 7)
+    want, _ = _oracle(H, P, N, G, lens, u, z, D, dt, da, state, old, cu, rows)
+    u[30, 5] = bad                                               # request 0, token 30, column 5
+    y = call(state)
+    hit = torch.zeros_like(y, dtype=torch.bool)
+    hit[30:100, 5] = True
+    if bad != 3.4e38:                                            # (finite, but its bf16 rounding is not: what follows may come back to numbers)
+        assert not torch.isfinite(y[hit]).any()
+    assert float((y[~hit].double() - want[~hit]).norm() / want[~hit].norm()) < 6e-7
+
+
+def test_groups_in_slices_and_under_capture(monkeypatch):
+    """more chunks of B, C and their products than the workspace holds at once; replayed from a graph, against the token-by-token order"""
+    H, P, N, G, lens = 16, 128, 128, 16, [9700, 300]
+    u, z, D, dt, da, state, old, cu, rows, call = _inputs(H, P, N, G, lens, "step", torch.bfloat16, 3)
+    s1, s2, keep = state.clone(), state.clone(), state.clone()
+    monkeypatch.setenv("SGLB_FIXED_ORDER", "1")
+    want = call(s1)
+    monkeypatch.delenv("SGLB_FIXED_ORDER")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call(s2)
+    torch.cuda.current_stream().wait_stream(side)
+    # (index tensors have to exist before the capture)
+    rows_t, seq_t, cu_t, q_t = _i32(rows), _i32([a + b for a, b in zip(lens, old)]), _i32(cu), _i32(lens)
+    raw, bias, A_log = (torch.randn(sum(lens), H, device="cuda").to(torch.bfloat16), torch.randn(H, device="cuda") - 3, torch.randn(H, device="cuda").abs())
+    s3, s4 = keep.clone(), keep.clone()
+    eager = ops.mamba2_scan(u, z, raw, bias, A_log, D, s3, rows_t, seq_t, cu_t, q_t, H, P, N, G)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = ops.mamba2_scan(u, z, raw, bias, A_log, D, s4, rows_t, seq_t, cu_t, q_t, H, P, N, G)
+    s4.copy_(keep)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, eager) and torch.equal(s3, s4)
+    # both orders are fp32 sums: each within a few 2^-24 of the exact one (the token order's chain is 9700 long)
+    got = call(keep)
+    assert float((got.double() - want.double()).norm() / want.double().norm()) < 3e-6
+    assert float((keep.double() - s1.double()).norm() / s1.double().norm()) < 3e-6
+    assert torch.equal(s2, keep)

@@ -1209,39 +1209,37 @@ void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::
   c10::cuda::CUDAGuard g(x.device());
   auto stream = cur_stream();
   const int pairs = T * K;
-  // Up to 48 rows an expert on average the block is bound by the weights: rows become the narrow operand (gemm_grouped_decode.cu) in tiles that hold
-  // twice the average, so that few experts need a second one; beyond, 128-row tiles (gemm_tc.cu) take less from L2 per product.  us a block here / there,
-  // 8 experts of 4096 x 14336, 2 chosen: 492 / 624 at 24 rows, 492 / 542 at 32, 538 / 542 at 40, 552 / 549 at 48, 560 / 550 at 56, 606 / 536 at 64;
-  // 128 experts of 2048 x 768, 8 chosen: 291 / 320 at 32, 340 / 358 at 44, 352 / 360 at 48, 371 / 370 at 56, 396 / 386 at 64.  Under expert parallelism
-  // the pairs are those of all ranks, so the line is met sooner by their number.
-  // fixed_order: the first kernel's tiles and shares of K follow the number of pairs, the 128-row kernel adds a row's K in one order whatever they are.
-  const bool decode = !fixed_order && pairs <= 48ll * E;
-  int tile = 128;
-  if (decode)
-    for (int t : {16, 32, 64, 128}) {
-      tile = t;
-      if (2ll * pairs <= (long long)t * E) break;
-    }
+  // Few rows an expert: small CTAs that share a tile's K stream the weights best (gemm_grouped_decode.cu).  From 6 rows on, pairs of SMs with the rows as the
+  // narrow operand (gemm_grouped_pair.cu), and from 3 where experts are many and their tiles fill the pairs evenly.  us a block here / there, 8 experts of
+  // 4096 x 14336, 2 chosen: 460 / 472 at 5 rows, 475 / 475 at 8, 483 / 473 at 12, 533 / 485 at 38; 128 experts of 2048 x 768, 8 chosen: 162 / 161 at 2.6,
+  // 187 / 178 at 5, 251 / 218 at 21, 342 / 268 at 48.  Under expert parallelism the pairs are those of all ranks, so the line is met sooner by their number.
+  // fixed_order: the first kernel's shares of K follow the number of pairs; 128-row tiles (gemm_tc.cu) add a row's K in one order whatever they are.
+  const bool decode = !fixed_order && pairs <= (E >= 64 ? 3ll : 6ll) * E;
+  const bool two_sm = !decode && !fixed_order && num_sms() >= 2 && sglb::gemm_grouped_pair_fits(pairs + 16 * std::min(E, pairs), E);
+  const int tile = decode || two_sm ? 16 : 128;
   const int max_tiles = pairs / tile + std::min(E, pairs);
   const int live_tiles = std::max(1, std::min(max_tiles, std::min(E, pairs)));
   const int cap = max_tiles * tile;
   auto i32 = x.options().dtype(at::kInt);
-  auto meta = at::empty({cap + pairs + max_tiles + 1}, i32);
+  auto meta = at::empty({cap + pairs + max_tiles + 1 + (two_sm ? E + 1 : 0)}, i32);
   int* sorted_row = meta.data_ptr<int>();
   int* inv_pos = sorted_row + cap;
   int* tile_expert = inv_pos + pairs;
   int* num_tiles = tile_expert + max_tiles;
+  int* expert_start = two_sm ? num_tiles + 1 : nullptr;
   auto row_w = at::empty({cap}, x.options().dtype(at::kFloat));
   sglb::moe_align(topk_ids.data_ptr<int>(), topk_w.data_ptr<float>(), pairs, E, (int)expert_offset, tile, sorted_row, inv_pos,
-                  row_w.data_ptr<float>(), tile_expert, num_tiles, max_tiles, stream);
+                  row_w.data_ptr<float>(), tile_expert, num_tiles, max_tiles, stream, expert_start);
   auto xs = at::empty({cap, H}, x.options());
   sglb::moe_gather(x.data_ptr(), sorted_row, num_tiles, xs.data_ptr(), H, (int)x.stride(0), K, cap, tile, stream,
                    weight_input ? row_w.data_ptr<float>() : nullptr);
   enum { NONE = 0, SILU = 1, ROWSCALE = 2, RELU2 = 3 };
   auto product = [&](const at::Tensor& a, const at::Tensor& w, at::Tensor& c, int n_out, int k, int epi) {
     if (decode)
-      sglb::gemm_grouped_decode(a.data_ptr(), w.data_ptr(), c.data_ptr(), row_w.data_ptr<float>(), sorted_row, tile, n_out, k, k, n_out, E, tile_expert,
+      sglb::gemm_grouped_decode(a.data_ptr(), w.data_ptr(), c.data_ptr(), row_w.data_ptr<float>(), sorted_row, n_out, k, k, n_out, E, tile_expert,
                                 num_tiles, max_tiles, live_tiles, epi, num_sms(), stream);
+    else if (two_sm)
+      sglb::gemm_grouped_pair(a.data_ptr(), w.data_ptr(), c.data_ptr(), row_w.data_ptr<float>(), cap, n_out, k, k, n_out, E, expert_start, epi, num_sms(), stream);
     else
       sglb::gemm_bf16_tc_grouped(a.data_ptr(), w.data_ptr(), c.data_ptr(), epi == ROWSCALE ? row_w.data_ptr<float>() : nullptr, cap, n_out, k, k, n_out, E,
                                  tile_expert, num_tiles, epi == SILU, num_sms(), stream, epi == RELU2);

@@ -53,8 +53,11 @@ void gemm_bf16_tc_grouped(const void* A, const void* W, void* C, const float* ro
                           int ldc, int num_experts, const int* tile_expert, const int* num_m_tiles, bool split_silu, int num_sms,
                           cudaStream_t stream, bool relu2 = false);
 
-// gemm_grouped_decode.cu
-void gemm_grouped_decode(const void* X, const void* W, void* C, const float* row_scale, const int* sorted_row, int tile, int n_out, int K, int lda, int ldc,
+// gemm_grouped_pair.cu, gemm_grouped_decode.cu
+bool gemm_grouped_pair_fits(int cap_rows, int E);
+void gemm_grouped_pair(const void* X, const void* W, void* C, const float* row_scale, int cap_rows, int n_out, int K, int lda, int ldc, int E,
+                       const int* expert_start, int epi, int num_sms, cudaStream_t stream);
+void gemm_grouped_decode(const void* X, const void* W, void* C, const float* row_scale, const int* sorted_row, int n_out, int K, int lda, int ldc,
                          int E, const int* tile_expert, const int* num_tiles, int max_tiles, int live_tiles, int epi, int num_sms, cudaStream_t stream);
 
 // kvio.cu: device pool <-> pinned host pool page movers (HiCache L1 <-> L2), zero-copy over UVA, layer_first / page_first host layouts
@@ -88,7 +91,7 @@ void per_token_group_quant_fp8(const void* x, void* q, float* scales, int M, int
 void moe_topk_softmax(const void* logits, bool bf16, float* out_w, int* out_ids, int T, int E, int K, int stride, bool renorm,
                       cudaStream_t stream);
 void moe_align(const int* topk_ids, const float* topk_w, int n_pairs, int E, int expert_offset, int tile, int* sorted_row, int* inv_pos,
-               float* row_w, int* tile_expert, int* num_tiles, int max_tiles, cudaStream_t stream);
+               float* row_w, int* tile_expert, int* num_tiles, int max_tiles, cudaStream_t stream, int* expert_start = nullptr);
 void moe_gather(const void* x, const int* sorted_row, const int* num_tiles, void* xs, int H, int x_stride, int K, int cap_rows,
                 int tile, cudaStream_t stream, const float* row_w = nullptr);
 void moe_combine(const void* ys, const int* inv_pos, const float* pair_w, void* out, int T, int H, int K, cudaStream_t stream);

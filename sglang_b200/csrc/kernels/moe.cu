@@ -104,7 +104,8 @@ template <int PER>
 __global__ void __launch_bounds__(ALIGN_THREADS) moe_align_kernel(const int* __restrict__ topk_ids, const float* __restrict__ topk_w,
                                                                   int n_pairs, int E, int expert_offset, int tile, int* __restrict__ sorted_row,
                                                                   int* __restrict__ inv_pos, float* __restrict__ row_w,
-                                                                  int* __restrict__ tile_expert, int* __restrict__ num_tiles, int max_tiles) {
+                                                                  int* __restrict__ tile_expert, int* __restrict__ num_tiles, int max_tiles,
+                                                                  int* __restrict__ expert_start) {
   __shared__ int cnt[MOE_MAX_E], cursor[MOE_MAX_E], start[MOE_MAX_E + 1];
   __shared__ int warp_tiles[MOE_MAX_E / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -154,8 +155,9 @@ __global__ void __launch_bounds__(ALIGN_THREADS) moe_align_kernel(const int* __r
     for (int w = 0; w < warp; ++w) before += warp_tiles[w];
     const int t0 = before + incl - nt;
     start[tid] = cursor[tid] = t0 * tile;
+    if (expert_start && tid <= E) expert_start[tid] = t0;
     for (int j = 0; j < nt && t0 + j < max_tiles; ++j) tile_expert[t0 + j] = tid;
-    if (tid == MOE_MAX_E - 1) { start[MOE_MAX_E] = (before + incl) * tile; *num_tiles = min(before + incl, max_tiles); }
+    if (tid == MOE_MAX_E - 1) { start[MOE_MAX_E] = (before + incl) * tile; *num_tiles = min(before + incl, max_tiles); if (expert_start && E == MOE_MAX_E) expert_start[E] = before + incl; }
   }
   __syncthreads();
   auto place = [&](int i, int e, float w) {
@@ -182,11 +184,11 @@ __global__ void __launch_bounds__(ALIGN_THREADS) moe_align_kernel(const int* __r
 }
 
 void moe_align(const int* topk_ids, const float* topk_w, int n_pairs, int E, int expert_offset, int tile, int* sorted_row, int* inv_pos,
-               float* row_w, int* tile_expert, int* num_tiles, int max_tiles, cudaStream_t stream) {
+               float* row_w, int* tile_expert, int* num_tiles, int max_tiles, cudaStream_t stream, int* expert_start) {
   if (E > MOE_MAX_E) throw std::runtime_error("sglb moe_align: more than 512 local experts");
 #define ALIGN(PER) \
   moe_align_kernel<PER><<<1, ALIGN_THREADS, 0, stream>>>(topk_ids, topk_w, n_pairs, E, expert_offset, tile, sorted_row, inv_pos, row_w, tile_expert, \
-                                                         num_tiles, max_tiles)
+                                                         num_tiles, max_tiles, expert_start)
   if (n_pairs <= 4 * ALIGN_THREADS) ALIGN(4);
   else if (n_pairs <= 16 * ALIGN_THREADS) ALIGN(16);
   else ALIGN(0);

@@ -1,0 +1,49 @@
+"""Expert blocks on pairs of SMs (csrc/kernels/gemm_grouped_pair.cu) against float64: rows that fill a tile, miss it by one step of 16 and spill over, every
+tile size the round count can choose, widths that end inside a tile, K remainders, experts without rows and of another rank, both lines of its rule."""
+import pytest
+import torch
+
+from sglang_b200 import ops
+from sglang_b200.ops import moe_ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("E,K,H,I,rows", [
+    (4, 1, 256, 128, [256, 257, 0, 1]), (4, 1, 128, 64, [512, 240, 16, 15]), (2, 1, 4096, 96, [700, 100]), (3, 1, 160, 416, [0, 0, 90]),
+    (8, 1, 2048, 256, [1000] * 8), (8, 1, 512, 1024, [300, 200, 128, 129, 127, 64, 33, 7]), (300, 1, 128, 64, [4] * 300), (8, 1, 256, 2080, [7] * 8), (70, 1, 128, 96, [3] * 69 + [40])])
+@pytest.mark.parametrize("act", [None, ("relu2",), ("clamped_glu", 4.0, 1.702)])
+@pytest.mark.parametrize("off", [0, 3])
+def test_block(E, K, H, I, rows, act, off):
+    assert ops.load_native()
+    g = torch.Generator(device="cuda").manual_seed(sum(rows) + E + H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    ids = torch.cat([torch.full((n,), e + off, dtype=torch.int32) for e, n in enumerate(rows)] + [torch.zeros(5 if off else 0, dtype=torch.int32)]).cuda()
+    ids = ids[torch.randperm(ids.numel(), generator=g, device="cuda")][:, None].contiguous()        # (off: five rows of an expert that is not here)
+    T = ids.shape[0]
+    x, w = rnd(T, H).to(torch.bfloat16), torch.rand(T, 1, generator=g, device="cuda") + 0.1
+    w13 = (rnd(E, (1 if act and act[0] == "relu2" else 2) * I, H) * H ** -0.5).to(torch.bfloat16)
+    w2 = (rnd(E, H, I) * I ** -0.5).to(torch.bfloat16)
+    for weight_input in ((False, True) if act and act[0] == "relu2" else (False,)):
+        y = moe_ops.fused_moe(x, w13, w2, w, ids, off, act, weight_input)
+        ref = torch.zeros(T, H, dtype=torch.float64, device="cuda")
+        for e in range(E):
+            t = (ids[:, 0] == e + off).nonzero()[:, 0]
+            wt = w[t].double()
+            u = (x[t].double() * (wt if weight_input else 1.0)) @ w13[e].double().T
+            if act is None:
+                a, u = u.chunk(2, -1)
+                h = torch.nn.functional.silu(a) * u
+            elif act[0] == "relu2":
+                h = u.clamp(min=0).square()
+            else:
+                a, u = u.chunk(2, -1)
+                a, u = a.clamp(max=act[1]), u.clamp(-act[1], act[1])
+                h = a * torch.sigmoid(act[2] * a) * (u + 1)
+            o = h @ w2[e].double().T
+            ref[t] = o if weight_input else o * wt
+        # three roundings to bf16 on the way (inner activations, an expert's output, the sum): 2^-9 each in the root mean square, relu2 doubles the first
+        err = float((y.double() - ref).norm() / ref.norm())
+        assert err < 4 * 2 ** -9, err
+        far = (y.double() - ref).norm(dim=1) / ref.norm(dim=1).clamp(min=float(ref.norm() / T ** 0.5) * 0.05)
+        assert float(far.max()) < 16 * 2 ** -9, float(far.max())

@@ -35,20 +35,25 @@ __device__ __forceinline__ void fma_pair(float2& sum, float s, uint32_t a, uint3
   sum = *reinterpret_cast<float2*>(&acc);
 }
 
-// Bound by the tensor core once the promotion keeps up: per K block a 128 x 256 tile is 512 cycles of UMMA against, per SM sub-partition, 4 warps x
-// 32 packed multiply-adds and their TMEM loads.  The version before promoted 128 x 128 with one warpgroup (128 scalar multiply-adds behind four
-// exposed TMEM loads per block) and was bound by that chain.  Measured, 3001 tokens, [28672 x 4096] and [4096 x 14336]: 445 -> 318 us a product (together 1.66 PFLOP/s).
+// Bound by the hand-off of an accumulator to the promotion (TMEM loads, 32 packed multiply-adds a warp, and the waits on both sides take about three times
+// the 256 cycles that 128 columns cost the tensor core), so a 256-wide tile has two halves with two accumulators each: one half is drained while the other is
+// formed.  The promotion warps take the registers of the other warpgroup, so that sixteen columns are on their way while sixteen are multiplied.
+// Measured, us a block (quantiser, [2I x H], SiLU, quantiser, [H x I]), before (whole 256-wide accumulators, one thread each for copies and products) and
+// now: 3001 tokens of 4096 / 14336: 715 / 691, 188: 111 / 98; 624 tokens of 8192 / 3584: 105 / 95, 147: 60 / 51, 65: 56 / 46.
 template <int BN>
 struct F8Cfg {
   static constexpr int A_BYTES = F8_BM * F8_BK;
   static constexpr int B_BYTES = BN * F8_BK;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = BN == 256 ? 4 : BN == 128 ? 6 : 8;
-  static constexpr int NACC = BN == 256 ? 2 : 4;                // TMEM accumulator stages
+  static constexpr int HALVES = BN == 256 ? 2 : 1;              // a wide tile's halves have accumulators of their own: one is drained while the other is formed
+  static constexpr int BH = BN / HALVES;
+  static constexpr int NACC = BN == 256 ? 2 : 4;                // TMEM accumulator stages of a half
   static constexpr int TMEM_COLS = NACC * BN;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
   static constexpr int COLS = BN == 64 ? 32 : 64;               // columns of one epilogue warp
   static constexpr int EPI_WARPS = 4 * (BN / COLS);
+  static constexpr int HALF_WARPS = EPI_WARPS / HALVES;
   static constexpr int THREADS = 128 + 32 * EPI_WARPS;
 };
 
@@ -67,8 +72,8 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   uint64_t* full = bars;
   uint64_t* empty = bars + STAGES;
   uint64_t* tfull = bars + 2 * STAGES;
-  uint64_t* tempty = bars + 2 * STAGES + NACC;
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * NACC);
+  uint64_t* tempty = tfull + NACC * Cfg::HALVES;                // (both [half][stage])
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tempty + NACC * Cfg::HALVES);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = (M + F8_BM - 1) / F8_BM, n_tiles = (N + BN - 1) / BN;
@@ -78,7 +83,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   if (warp == 0 && lane == 0) { tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); }
   if (warp == 1 && lane == 0) {
     for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-    for (int i = 0; i < NACC; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], Cfg::EPI_WARPS); }
+    for (int i = 0; i < NACC * Cfg::HALVES; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], Cfg::HALF_WARPS); }
     fence_barrier_init();
   }
   if (warp == 2) { tmem_alloc(tmem_ptr, Cfg::TMEM_COLS); tmem_relinquish(); }
@@ -87,80 +92,113 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
 
-  if (warp == 0 && lane == 0) {
-    int stage = 0; uint32_t phase = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      const int m_blk = tile % m_tiles, n_blk = tile / m_tiles;
-      for (int kb = 0; kb < num_kb; ++kb) {
-        mbar_wait(&empty[stage], phase ^ 1);
-        mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-        tma_load_2d(sA + stage * Cfg::A_BYTES, &tmA, &full[stage], kb * F8_BK, m_blk * F8_BM);
-        tma_load_2d(sB + stage * Cfg::B_BYTES, &tmB, &full[stage], kb * F8_BK, n_blk * BN);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+  // (producer and issuer keep their warp together and elect a lane: addresses and descriptors stay in uniform registers)
+  if (warp < 4) {
+    if constexpr (BN == 256) regs_down<32>();
+    if (warp == 0) {
+      const bool one = elect_one();
+      int stage = 0; uint32_t phase = 0;
+      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+        const int m_blk = tile % m_tiles, n_blk = tile / m_tiles;
+        for (int kb = 0; kb < num_kb; ++kb) {
+          mbar_wait_brief(&empty[stage], phase ^ 1);
+          if (one) {
+            mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
+            tma_load_2d(sA + stage * Cfg::A_BYTES, &tmA, &full[stage], kb * F8_BK, m_blk * F8_BM);
+            tma_load_2d(sB + stage * Cfg::B_BYTES, &tmB, &full[stage], kb * F8_BK, n_blk * BN);
+          }
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
       }
-    }
-  } else if (warp == 1 && lane == 0) {
-    constexpr uint32_t idesc = make_idesc(UMMA_E4M3, UMMA_E4M3, F8_BM, BN, 0, 0);
-    int stage = 0; uint32_t phase = 0;
-    int acc = 0; uint32_t acc_phase = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      for (int kb = 0; kb < num_kb; ++kb) {
-        mbar_wait(&tempty[acc], acc_phase ^ 1);
-        mbar_wait(&full[stage], phase);
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        const uint64_t adesc = make_smem_desc_sw128(smem_u32(sA + stage * Cfg::A_BYTES), 0, 1024);
-        const uint64_t bdesc = make_smem_desc_sw128(smem_u32(sB + stage * Cfg::B_BYTES), 0, 1024);
+    } else if (warp == 1) {
+      constexpr uint32_t idesc = make_idesc(UMMA_E4M3, UMMA_E4M3, F8_BM, Cfg::BH, 0, 0);
+      const uint64_t da = make_smem_desc_sw128(smem_u32(sA), 0, 1024), db = make_smem_desc_sw128(smem_u32(sB), 0, 1024);
+      const bool one = elect_one();
+      int stage = 0; uint32_t phase = 0;
+      int acc = 0; uint32_t acc_phase = 0;
+      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+        for (int kb = 0; kb < num_kb; ++kb) {
+          mbar_wait_brief(&full[stage], phase);
 #pragma unroll
-        for (int k = 0; k < F8_BK / 32; ++k) umma_f8_ss(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, k != 0);
-        umma_commit(&empty[stage]);
-        umma_commit(&tfull[acc]);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
-        if (++acc == NACC) { acc = 0; acc_phase ^= 1; }
+          for (int h = 0; h < Cfg::HALVES; ++h) {
+            mbar_wait_brief(&tempty[h * NACC + acc], acc_phase ^ 1);
+            tc_fence_after();
+            const uint64_t adesc = da + stage * (Cfg::A_BYTES / 16), bdesc = db + stage * (Cfg::B_BYTES / 16) + h * (Cfg::BH * F8_BK / 16);
+            if (one) {
+#pragma unroll
+              for (int k = 0; k < F8_BK / 32; ++k) umma_f8_ss(tmem_base + (h * NACC + acc) * Cfg::BH, adesc + 2 * k, bdesc + 2 * k, idesc, k != 0);
+              umma_commit(&tfull[h * NACC + acc]);
+            }
+          }
+          if (one) umma_commit(&empty[stage]);
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (++acc == NACC) { acc = 0; acc_phase ^= 1; }
+        }
       }
     }
-  } else if (warp >= 4) {
+    __syncwarp();
+  } else {
+    if constexpr (BN == 256) regs_up<112>();
     const int q = warp & 3, c0 = ((warp - 4) >> 2) * COLS;          // a warp reads the TMEM lanes of its index modulo 4
+    const int half = c0 / Cfg::BH;
+    uint64_t *my_full = tfull + half * NACC, *my_empty = tempty + half * NACC;
+    const uint32_t t_half = tmem_base + ((uint32_t)(q * 32) << 16) + half * NACC * Cfg::BH + c0 % Cfg::BH;
+    const bool wide = (ldc & 15) == 0 && (reinterpret_cast<uintptr_t>(C) & 31) == 0;      // 32-byte stores: whole sectors of a row by one lane
+    const float *xs_row, *ws_row;
+    auto scales_of = [&](int tile) {                          // the warp's columns (64 from a multiple of 64) lie in one 128-wide weight block
+      xs_row = xs + (size_t)min((tile % m_tiles) * F8_BM + q * 32 + lane, M - 1) * xs_stride;
+      ws_row = ws + (size_t)(min(tile / m_tiles * BN + c0, N - 1) >> 7) * ws_stride;
+    };
     int acc = 0; uint32_t acc_phase = 0;
+    scales_of(min((int)blockIdx.x, num_tiles - 1));
+    float a_scale = __ldg(xs_row), w_scale = __ldg(ws_row);
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      const int m_blk = tile % m_tiles, n_blk = tile / m_tiles;
-      const int row = m_blk * F8_BM + q * 32 + lane;
-      const int row_c = min(row, M - 1);
-      const int col0 = n_blk * BN + c0;
-      // the warp's columns (64 from a multiple of 64) lie in one 128-wide weight block
-      const float* ws_row = ws + (size_t)(min(col0, N - 1) >> 7) * ws_stride;
+      const int row = (tile % m_tiles) * F8_BM + q * 32 + lane, col0 = tile / m_tiles * BN + c0;
       float2 sum[COLS / 2];
 #pragma unroll
       for (int i = 0; i < COLS / 2; ++i) sum[i] = make_float2(0.f, 0.f);
-      const float* xs_row = xs + (size_t)row_c * xs_stride;
-      float a_scale = __ldg(xs_row), w_scale = __ldg(ws_row);
       for (int kb = 0; kb < num_kb; ++kb) {
         const float s = a_scale * w_scale;
-        if (kb + 1 < num_kb) { a_scale = __ldg(xs_row + kb + 1); w_scale = __ldg(ws_row + kb + 1); }
-        mbar_wait(&tfull[acc], acc_phase);
+        // the next block's scales; those of the next tile's first block while this tile ends
+        if (kb + 1 == num_kb) scales_of(min(tile + (int)gridDim.x, num_tiles - 1));
+        const int next = kb + 1 == num_kb ? 0 : kb + 1;
+        a_scale = __ldg(xs_row + next);
+        w_scale = __ldg(ws_row + next);
+        mbar_wait_brief(&my_full[acc], acc_phase);
         tc_fence_after();
-        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + c0;
+        const uint32_t t_row = t_half + acc * Cfg::BH;
+        // sixteen columns are multiplied while the next are on their way; the accumulator is free once all of them are in registers
+        uint32_t r[2][16];
+        tmem_ld_32x32b_x16(t_row, r[0]);
 #pragma unroll
         for (int c = 0; c < COLS; c += 16) {
-          uint32_t r[16];
-          tmem_ld_32x32b_x16(t_row + c, r);
+          uint32_t (&v)[16] = r[(c >> 4) & 1];
           tmem_ld_wait();
+          if (c + 16 < COLS) {
+            tmem_ld_32x32b_x16(t_row + c + 16, r[((c >> 4) & 1) ^ 1]);
+          } else {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&my_empty[acc]);
+          }
 #pragma unroll
-          for (int i = 0; i < 8; ++i) fma_pair(sum[c / 2 + i], s, r[2 * i], r[2 * i + 1]);
+          for (int i = 0; i < 8; ++i) fma_pair(sum[c / 2 + i], s, v[2 * i], v[2 * i + 1]);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty[acc]);
         if (++acc == NACC) { acc = 0; acc_phase ^= 1; }
       }
       if (row < M) {
+        __nv_bfloat16* dst = C + (size_t)row * ldc + col0;
 #pragma unroll
-        for (int v = 0; v < COLS / 8; ++v) {
-          const int col = col0 + v * 8;
-          if (col < N) {
-            const U4 o = U4{pack_bf16(sum[v * 4].x, sum[v * 4].y), pack_bf16(sum[v * 4 + 1].x, sum[v * 4 + 1].y),
-                            pack_bf16(sum[v * 4 + 2].x, sum[v * 4 + 2].y), pack_bf16(sum[v * 4 + 3].x, sum[v * 4 + 3].y)};
-            st128(C + (size_t)row * ldc + col, o);
+        for (int v = 0; v < COLS / 16; ++v) {
+          uint32_t o[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = pack_bf16(sum[v * 8 + i].x, sum[v * 8 + i].y);
+          if (wide && col0 + v * 16 + 8 < N) {
+            asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + v * 16), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]),
+                         "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
+          } else {
+            if (col0 + v * 16 < N) st128(dst + v * 16, U4{o[0], o[1], o[2], o[3]});
+            if (col0 + v * 16 + 8 < N) st128(dst + v * 16 + 8, U4{o[4], o[5], o[6], o[7]});
           }
         }
       }

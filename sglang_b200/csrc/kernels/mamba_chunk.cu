@@ -85,12 +85,6 @@ __device__ __forceinline__ void mc_arrive(uint64_t* bar, int lane) {      // thi
   __syncwarp();
   if (lane == 0) mbar_arrive(bar);
 }
-__device__ __forceinline__ void mc_wait(uint64_t* bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return;
-  const uint64_t t0 = globaltimer_ns();
-  while (!mbar_try_wait(bar, parity))
-    if (globaltimer_ns() - t0 > SGLB_MBAR_TIMEOUT_NS) __trap();
-}
 // a stride whose multiples the compiler works out where they are used, instead of keeping all of them in registers over the whole loop
 __device__ __forceinline__ size_t mc_stride(size_t v) {
   asm volatile("" : "+l"(v));
@@ -102,9 +96,6 @@ __device__ __forceinline__ float mc_silu(float z) {
   const float d = fminf(1.f + expf(-z), 3e38f), r = rcp_approx(d), q = z * r;
   return fmaf(fmaf(-d, q, z), r, q);
 }
-template <int R> __device__ __forceinline__ void mc_regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
-template <int R> __device__ __forceinline__ void mc_regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
-
 // Chunk c of request b has slot cu_q[b] / 64 + b + c: no two share one, and none lies beyond T / 64 + B.
 __device__ __forceinline__ int mc_slot(int q0, int b) { return q0 / MC_L + b; }
 
@@ -235,7 +226,7 @@ __global__ void __launch_bounds__(MC_SPLIT_THREADS) mamba2_split_kernel(const Ma
     }
     if (lane == 0) *reinterpret_cast<float4*>(s + MC_ALL) = make_float4((float)(blk[0] * blk[1] * blk[2] * blk[3]), (float)blk[1], (float)(blk[1] * blk[2]), (float)blk[2]);
   }
-  mc_wait(&done, 0);
+  mbar_wait_brief(&done, 0);
   tc_fence_after();
   if ((warp & 3) < 2) {
     const int t = (warp & 3) * 32 + lane, s0 = (warp >> 2) * 32;
@@ -315,7 +306,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
 
   if (warp >= 28) {
     // ------------------------------------------------------------ issuer, loader
-    mc_regs_down<32>();
+    regs_down<32>();
     if (warp == 28) {
       // (all lanes stay together and one is elected: descriptors stay in uniform registers, 34 cycles a 64-wide product instead of 60 by a lane alone)
       constexpr uint32_t id_s = make_idesc(UMMA_BF16, UMMA_BF16, 128, N, 0, 1), id_y1 = make_idesc(UMMA_BF16, UMMA_BF16, 128, 64, 0, 0);
@@ -326,9 +317,9 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
       const bool one = elect_one();
       for (int c = 0; c < chunks; ++c) {
         const uint32_t par = c & 1;
-        mc_wait(b_full, par);
-        mc_wait(wx_ready, par);
-        mc_wait(y_read, par ^ 1);
+        mbar_wait_brief(b_full, par);
+        mbar_wait_brief(wx_ready, par);
+        mbar_wait_brief(y_read, par ^ 1);
         tc_fence_after();
 #pragma unroll 1
         for (int i = 0; i < 6; ++i) {
@@ -339,8 +330,8 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
             if (one) umma_f16_ts(tmem + MC_TACC, a + k * 8, w + k * (2048 / 16), id_s, (i | k) != 0);
         }
         if (one) umma_commit(s_full);
-        mc_wait(xm_ready, par);
-        mc_wait(s_read, par);
+        mbar_wait_brief(xm_ready, par);
+        mbar_wait_brief(s_read, par);
         tc_fence_after();
         // two heads: each with the M of both (columns), of which it needs its own
 #pragma unroll 1
@@ -351,7 +342,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
             if (one) umma_f16_ss(tmem + MC_TY2, a + k * (2048 / 16), w + k * 2, id_y2, (i | k) != 0);
         }
         if (one) umma_commit(y2_full);
-        mc_wait(c_full, par);
+        mbar_wait_brief(c_full, par);
 #pragma unroll 1
         for (int i = 0; i < 6; ++i) {
           const uint32_t a = tmem + MC_TS + mc_part_a(i) * (N / 2);
@@ -382,21 +373,21 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
       for (int c = 0; c < chunks; ++c) {
         const uint8_t* src = slot0 + c * chunk_bytes;
         const int ring = c & 1;
-        mc_wait(st_empty + ring, ((c >> 1) & 1) ^ 1);
+        mbar_wait_brief(st_empty + ring, ((c >> 1) & 1) ^ 1);
         if (lane == 0) {
           mbar_expect_tx(st_full + ring, HEADS * MC_STEPS);
           asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                        ::"r"(smem_u32(steps + ring * HEADS * MC_STEPS)), "l"(src + Cfg::SLOT + (head0 - g * (H / p.G)) * MC_STEPS), "n"(HEADS * MC_STEPS),
                        "r"(smem_u32(st_full + ring)) : "memory");
         }
-        if (c > 0) mc_wait(s_full, (c - 1) & 1);
+        if (c > 0) mbar_wait_brief(s_full, (c - 1) & 1);
         if (lane == 0) {
           mbar_expect_tx(b_full, Cfg::IMG);
           asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                        ::"r"(smem_u32(smem + Cfg::B)), "l"(src + Cfg::IMG), "n"(Cfg::IMG), "r"(smem_u32(b_full)) : "memory");
         }
         prefetch(c + 2);
-        if (c > 0) mc_wait(y1_full, (c - 1) & 1);
+        if (c > 0) mbar_wait_brief(y1_full, (c - 1) & 1);
         if (lane == 0) {
           mbar_expect_tx(c_full, Cfg::IMG);
           asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -407,7 +398,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
     __syncwarp();
   } else if (warp >= 24) {
     // ------------------------------------------------------------ M: row mt, blocks of 16 tokens s
-    mc_regs_up<80>();
+    regs_up<80>();
     const int w4 = warp - 24, mt = (w4 & 1) * 32 + lane, mh = PAIR ? w4 >> 1 : 0, mb = mt >> 4;
     const float dskip = p.D ? p.D[head0 + mh] : 0.f;
     const int first = PAIR ? 0 : (w4 >> 1) * 2, last = PAIR ? 3 : first + 1, top = (w4 & 1) * 2 + 1;      // blocks of this thread; the last below the diagonal of its warp
@@ -423,7 +414,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
           *reinterpret_cast<float4*>(next + i) = k <= last && k <= top ? __ldg(gp + (4 * k + i / 4) * MC_L) : make_float4(0.f, 0.f, 0.f, 0.f);
       };
       fetch(first);
-      mc_wait(st_full + ring, (c >> 1) & 1);
+      mbar_wait_brief(st_full + ring, (c >> 1) & 1);
       const float* sp = reinterpret_cast<const float*>(steps + (ring * HEADS + mh) * MC_STEPS);
       const float pin = sp[MC_PIN + mt];
 #pragma unroll 1
@@ -457,7 +448,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
 #pragma unroll
           for (int i = 0; i < 16; ++i) r[i] = 0.f;
         }
-        if (c > 0 && k == first) mc_wait(y2_full, (c - 1) & 1);      // the last chunk's M has been read
+        if (c > 0 && k == first) mbar_wait_brief(y2_full, (c - 1) & 1);      // the last chunk's M has been read
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           uint4 a, m, l;
@@ -473,7 +464,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
     }
   } else if (warp >= 16) {
     // ------------------------------------------------------------ outputs
-    mc_regs_up<72>();
+    regs_up<72>();
     const int q = warp & 3, hf = (warp - 16) >> 2, pl = q * 32 + lane, hs = PAIR ? q >> 1 : 0, col = col0 + pl;
     const uint32_t t_lane = tmem + ((uint32_t)(q * 32) << 16) + hf * 32;
     const TZ* zp = reinterpret_cast<const TZ*>(p.z);
@@ -494,10 +485,10 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
 #pragma unroll
         for (int i = 0; i < 32; ++i) gate[i] = 1.f;
       }
-      mc_wait(st_full + ring, (c >> 1) & 1);
+      mbar_wait_brief(st_full + ring, (c >> 1) & 1);
       const float* sp = reinterpret_cast<const float*>(steps + (ring * HEADS + hs) * MC_STEPS) + MC_P + hf * 32;
-      mc_wait(y2_full, par);
-      mc_wait(y1_full, par);
+      mbar_wait_brief(y2_full, par);
+      mbar_wait_brief(y1_full, par);
       tc_fence_after();
       int* bad = s_bad + (ring * 2 + hf) * MC_COLS + pl;
       if (*bad < MC_L) {
@@ -534,7 +525,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
     }
   } else if (warp >= 8) {
     // ------------------------------------------------------------ inputs
-    mc_regs_down<40>();
+    regs_down<40>();
     const int w8 = warp - 8, q = w8 & 3, hf = w8 >> 2, pl = q * 32 + lane, hs = PAIR ? q >> 1 : 0;
     const float* xp = p.u + (size_t)(q0 + hf * 32) * p.ldu + col0 + pl;
     const uint32_t t_x = tmem + ((uint32_t)(q * 32) << 16) + MC_TX + hf * 16;
@@ -544,8 +535,8 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
     for (int c = 0; c < chunks; ++c) {
       const int left = n - c * MC_L, ring = c & 1;
       const uint32_t prev = (c - 1) & 1;
-      mc_wait(st_full + ring, (c >> 1) & 1);
-      if (c > 0) mc_wait(s_full, prev);                       // the last chunk's w X has been read
+      mbar_wait_brief(st_full + ring, (c >> 1) & 1);
+      if (c > 0) mbar_wait_brief(s_full, prev);                       // the last chunk's w X has been read
       tc_fence_after();
       const float* w = reinterpret_cast<const float*>(steps + (ring * HEADS + hs) * MC_STEPS) + MC_W + hf * 32;
 #pragma unroll 1
@@ -567,7 +558,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
       xp += (size_t)(MC_L - 32) * p.ldu;
       tmem_st_wait();
       mc_arrive(wx_ready, lane);
-      if (c > 0) mc_wait(y2_full, prev);                      // the last chunk's X has been read
+      if (c > 0) mbar_wait_brief(y2_full, prev);                      // the last chunk's X has been read
 #pragma unroll 2
       for (int s = xt; s < MC_L; s += 16) {
         float v[8];
@@ -600,7 +591,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
     }
   } else {
     // ------------------------------------------------------------ state
-    mc_regs_up<88>();
+    regs_up<88>();
     const int q = warp & 3, hf = warp >> 2, pl = q * 32 + lane, hs = PAIR ? q >> 1 : 0, head = head0 + hs;
     const uint32_t t_lane = tmem + ((uint32_t)(q * 32) << 16);
     float* st = p.state + (((size_t)p.req_slots[b] * H + head) * N + hf * NT) * P + (col0 + pl - head * P);
@@ -617,7 +608,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
       const uint32_t par = c & 1;
       // S^T of before the chunk, split
       if (c > 0) {
-        mc_wait(y1_full, par ^ 1);                            // the last chunk's products have read theirs
+        mbar_wait_brief(y1_full, par ^ 1);                            // the last chunk's products have read theirs
         tc_fence_after();
       }
 #pragma unroll
@@ -631,9 +622,9 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mamba2_chunk_kernel(const Mamba
         tmem_st_32x32b_x4(t + N, l);
       }
       tmem_st_wait();
-      mc_wait(st_full + ring, (c >> 1) & 1);
+      mbar_wait_brief(st_full + ring, (c >> 1) & 1);
       const float all = reinterpret_cast<const float*>(steps + (ring * HEADS + hs) * MC_STEPS)[MC_ALL];
-      mc_wait(s_full, par);
+      mbar_wait_brief(s_full, par);
       tc_fence_after();
 #pragma unroll
       for (int j0 = 0; j0 < NT; j0 += 16) {

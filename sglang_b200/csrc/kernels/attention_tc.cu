@@ -1006,13 +1006,14 @@ __global__ void attn_merge_splits_diff_kernel(const float* __restrict__ part_o, 
 // 128-row tiles of the same KV head; while one warpgroup works out its probabilities, the tensor core runs the other's P.V and Q.K^T, and both read the
 // same K and V tiles, so the two units are busy at once and every key tile is fetched once for 256 rows.
 //
-//   warp 0 : scheduler + TMA producer      warp 1 : MMA issuer, one thread      warps 4..7 / 8..11 : soft-max + epilogue of tile A / B
+//   warp 0 : scheduler + TMA producer      warp 1 : MMA issuer      warps 4..7 / 8..11 : soft-max + epilogue of tile A / B
 //   TMEM   : S_A | S_B | O_A | O_B (128 columns each); P overwrites its S.  S(j + 1) is issued behind P(j).V(j), which has read P by then (products of
 //            one thread run in the order of issue)
 //   shared : Q 64 KB, two stages of K and V
 // Plain scores only (no cap, bias, window, chunk, tree or splits).  Same arithmetic in the same order per row as the kernel above.
-// Measured: 4096 queries, 32 + 8 heads, at the end of 15011 keys: 1119 -> 956 us; 17 prompts of
-// 68 to 886 tokens (5003): 121 -> 79 us.
+// A soft-max thread holds its row's 128 scores: the first warpgroup gives it the registers (with an equal share it spilled, and read half of S twice).
+// Measured: 4096 queries, 32 + 8 heads, at the end of 15011 keys: 1119 us in the kernel above, 942 here with one thread each for copies and products and
+// equal registers, 787 now; 2000 at the end of 9000: 321 -> 266; 17 prompts of 68 to 886 tokens (5003): 121 -> 79 us.
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -1085,124 +1086,137 @@ attn_fwd_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   };
 
   if (warp < 4) {
-    if (warp == 0 && lane == 0) {
-      // ------------------------------------------------------------ scheduler + producer
+    regs_down<56>();
+    if (warp == 0) {
+      // ------------------------------------------------------------ scheduler + producer: a lane per copy (one thread takes longer over a tile's 16 copies than
+      // the tensor core over the tile), page ids of a tile fetched while the one before is waited for
       uint32_t n_it = 0, n_q = 0, g = 0;
       for (;;) {
         const int slot = n_it & 1;
-        mbar_wait(&item_empty[slot], ((n_it >> 1) & 1) ^ 1);
-        const int idx = atomicAdd(p.sched, 1);
-        s_item[slot] = idx;
-        mbar_arrive(&item_full[slot]);
+        mbar_wait_brief(&item_empty[slot], ((n_it >> 1) & 1) ^ 1);
+        int idx = lane == 0 ? atomicAdd(p.sched, 1) : 0;
+        idx = __shfl_sync(0xffffffffu, idx, 0);
+        if (lane == 0) {
+          s_item[slot] = idx;
+          mbar_arrive(&item_full[slot]);
+        }
         ++n_it;
         if (idx >= p.total_items) break;
         const Item it = decode_item(idx);
         if (it.n_tiles == 0) continue;
-        mbar_wait(q_empty, (n_q & 1) ^ 1);
-        mbar_expect_tx(q_full, it.both ? 2 * ATT_TILE_BYTES : ATT_TILE_BYTES);
-        for (int i = 0; i < (it.both ? 2 : 1); ++i) {
-          tma_load_4d(sQ + i * ATT_TILE_BYTES, &tmQ, q_full, 0, 0, it.kvh, it.q_start + it.t0 + i * TQ);
-          tma_load_4d(sQ + i * ATT_TILE_BYTES + ATT_HALF_BYTES, &tmQ, q_full, 64, 0, it.kvh, it.q_start + it.t0 + i * TQ);
-        }
+        mbar_wait_brief(q_empty, (n_q & 1) ^ 1);
+        const int q_copies = it.both ? 4 : 2;
+        if (lane == 0) mbar_expect_tx(q_full, it.both ? 2 * ATT_TILE_BYTES : ATT_TILE_BYTES);
+        __syncwarp();
+        if (lane < q_copies)
+          tma_load_4d(sQ + (lane >> 1) * ATT_TILE_BYTES + (lane & 1) * ATT_HALF_BYTES, &tmQ, q_full, (lane & 1) * 64, 0, it.kvh, it.q_start + it.t0 + (lane >> 1) * TQ);
         ++n_q;
-        const int ps = p.page_size, pages_per_tile = KT / ps;
+        const int ps = p.page_size, copies = 2 * (KT / ps);                      // (8-token pages: 32)
         const int* pt = p.page_table + (size_t)p.req_slots[it.b] * p.pt_stride;
+        const int sub = lane >> 1, off = (lane & 1) * ATT_HALF_BYTES + sub * ps * 128;
+        int page = lane < copies ? pt[min(sub, p.pt_stride - 1)] : 0;
         for (int j = 0; j < it.n_tiles; ++j, ++g) {
-          const int st = g & 1;
+          const int st = g & 1, row = page * ps;
           const uint32_t ph = (g >> 1) & 1;
-          mbar_wait(&k_empty[st], ph ^ 1);
-          mbar_expect_tx(&k_full[st], ATT_TILE_BYTES);
-          for (int i = 0; i < pages_per_tile; ++i) {
-            const int page = pt[min(j * pages_per_tile + i, p.pt_stride - 1)];
-            uint8_t* dst = sK + st * ATT_TILE_BYTES + i * ps * 128;
-            tma_load_3d(dst, &tmK, &k_full[st], 0, it.kvh, page * ps);
-            tma_load_3d(dst + ATT_HALF_BYTES, &tmK, &k_full[st], 64, it.kvh, page * ps);
-          }
-          mbar_wait(&v_empty[st], ph ^ 1);
-          mbar_expect_tx(&v_full[st], ATT_TILE_BYTES);
-          for (int i = 0; i < pages_per_tile; ++i) {
-            const int page = pt[min(j * pages_per_tile + i, p.pt_stride - 1)];
-            uint8_t* dst = sV + st * ATT_TILE_BYTES + i * ps * 128;
-            tma_load_3d(dst, &tmV, &v_full[st], 0, it.kvh, page * ps);
-            tma_load_3d(dst + ATT_HALF_BYTES, &tmV, &v_full[st], 64, it.kvh, page * ps);
-          }
+          if (lane < copies && j + 1 < it.n_tiles) page = pt[min((j + 1) * (KT / ps) + sub, p.pt_stride - 1)];
+          mbar_wait_brief(&k_empty[st], ph ^ 1);
+          if (lane == 0) mbar_expect_tx(&k_full[st], ATT_TILE_BYTES);
+          __syncwarp();
+          if (lane < copies) tma_load_3d(sK + st * ATT_TILE_BYTES + off, &tmK, &k_full[st], (lane & 1) * 64, it.kvh, row);
+          mbar_wait_brief(&v_empty[st], ph ^ 1);
+          if (lane == 0) mbar_expect_tx(&v_full[st], ATT_TILE_BYTES);
+          __syncwarp();
+          if (lane < copies) tma_load_3d(sV + st * ATT_TILE_BYTES + off, &tmV, &v_full[st], (lane & 1) * 64, it.kvh, row);
         }
       }
-    } else if (warp == 1 && lane == 0) {
-      // ------------------------------------------------------------ MMA issuer
+      __syncwarp();
+    } else if (warp == 1) {
+      // ------------------------------------------------------------ MMA issuer (the warp stays together and elects a lane: descriptors in uniform registers)
       constexpr uint32_t idesc_s = make_idesc(UMMA_BF16, UMMA_BF16, 128, KT, 0, 0);
       constexpr uint32_t idesc_o = make_idesc(UMMA_BF16, UMMA_BF16, 128, ATT_D, 0, 1);
+      const uint64_t d_q = make_smem_desc_sw128(smem_u32(sQ), 0, 1024), d_k = make_smem_desc_sw128(smem_u32(sK), 0, 1024);
+      const uint64_t d_v = make_smem_desc_sw128(smem_u32(sV), ATT_HALF_BYTES, 1024);
+      const bool one = elect_one();
+      auto commit = [&](uint64_t* bar) {
+        if (one) umma_commit(bar);
+      };
       auto scores = [&](int tile, int st) {          // S_tile = Q_tile K^T
-        const uint32_t q_addr = smem_u32(sQ + tile * ATT_TILE_BYTES), k_addr = smem_u32(sK + st * ATT_TILE_BYTES);
+        const uint64_t a = d_q + tile * (ATT_TILE_BYTES / 16), b = d_k + st * (ATT_TILE_BYTES / 16);
+        if (one) {
 #pragma unroll
-        for (int k = 0; k < ATT_D / 16; ++k) {
-          const uint32_t off = (k >> 2) * ATT_HALF_BYTES + (k & 3) * 32;
-          umma_f16_ss(tmem + tile * KT, make_smem_desc_sw128(q_addr + off, 0, 1024), make_smem_desc_sw128(k_addr + off, 0, 1024), idesc_s, k != 0);
+          for (int k = 0; k < ATT_D / 16; ++k) {
+            const uint32_t off = ((k >> 2) * ATT_HALF_BYTES + (k & 3) * 32) / 16;
+            umma_f16_ss(tmem + tile * KT, a + off, b + off, idesc_s, k != 0);
+          }
+          umma_commit(&s_full[tile]);
         }
-        umma_commit(&s_full[tile]);
       };
       auto values = [&](int tile, int st, bool fresh) {      // O_tile (+)= P_tile V
-        const uint32_t v_addr = smem_u32(sV + st * ATT_TILE_BYTES);
+        const uint64_t b = d_v + st * (ATT_TILE_BYTES / 16);
+        if (one) {
 #pragma unroll
-        for (int k = 0; k < KT / 16; ++k)
-          umma_f16_ts(tmem + 2 * KT + tile * ATT_D, tmem + tile * KT + k * 8, make_smem_desc_sw128(v_addr + k * 2048, ATT_HALF_BYTES, 1024), idesc_o,
-                      !fresh || k != 0);
-        umma_commit(&o_done[tile]);
+          for (int k = 0; k < KT / 16; ++k)
+            umma_f16_ts(tmem + 2 * KT + tile * ATT_D, tmem + tile * KT + k * 8, b + k * (2048 / 16), idesc_o, !fresh || k != 0);
+          umma_commit(&o_done[tile]);
+        }
       };
       uint32_t n_it = 0, n_q = 0, n_qb = 0, g = 0, gb = 0;
       for (;;) {
         const int slot = n_it & 1;
-        mbar_wait(&item_full[slot], (n_it >> 1) & 1);
+        mbar_wait_brief(&item_full[slot], (n_it >> 1) & 1);
         const int idx = s_item[slot];
-        mbar_arrive(&item_empty[slot]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&item_empty[slot]);
         ++n_it;
         if (idx >= p.total_items) break;
         const Item it = decode_item(idx);
         const int n = it.n_tiles;
         if (n == 0) continue;
-        mbar_wait(q_full, n_q & 1);
-        mbar_wait(&k_full[g & 1], (g >> 1) & 1);
+        mbar_wait_brief(q_full, n_q & 1);
+        mbar_wait_brief(&k_full[g & 1], (g >> 1) & 1);
         tc_fence_after();
         scores(0, g & 1);
         if (it.both) scores(1, g & 1);
-        umma_commit(&k_empty[g & 1]);
-        if (n == 1) umma_commit(q_empty);
+        commit(&k_empty[g & 1]);
+        if (n == 1) commit(q_empty);
         for (int j = 0; j < n; ++j) {
           const uint32_t gt = g + j;
           const int st = gt & 1, nx = st ^ 1;
           const bool more = j + 1 < n;
-          mbar_wait(&p_full[0], gt & 1);
-          mbar_wait(&v_full[st], (gt >> 1) & 1);
-          if (j == 0) mbar_wait(&o_free[0], (n_q & 1) ^ 1);            // the epilogue of the item before has read O
+          mbar_wait_brief(&p_full[0], gt & 1);
+          mbar_wait_brief(&v_full[st], (gt >> 1) & 1);
+          if (j == 0) mbar_wait_brief(&o_free[0], (n_q & 1) ^ 1);            // the epilogue of the item before has read O
           tc_fence_after();
           values(0, st, j == 0);
-          if (!more) umma_commit(&o_final[0]);
+          if (!more) commit(&o_final[0]);
           if (more) {
-            mbar_wait(&k_full[nx], ((gt + 1) >> 1) & 1);
+            mbar_wait_brief(&k_full[nx], ((gt + 1) >> 1) & 1);
             tc_fence_after();
             scores(0, nx);
           }
           if (it.both) {
-            mbar_wait(&p_full[1], (gb + j) & 1);
-            if (j == 0) mbar_wait(&o_free[1], (n_qb & 1) ^ 1);
+            mbar_wait_brief(&p_full[1], (gb + j) & 1);
+            if (j == 0) mbar_wait_brief(&o_free[1], (n_qb & 1) ^ 1);
             tc_fence_after();
             values(1, st, j == 0);
-            if (!more) umma_commit(&o_final[1]);
+            if (!more) commit(&o_final[1]);
           }
-          umma_commit(&v_empty[st]);
+          commit(&v_empty[st]);
           if (more) {
             if (it.both) scores(1, nx);
-            umma_commit(&k_empty[nx]);
-            if (j + 2 == n) umma_commit(q_empty);
+            commit(&k_empty[nx]);
+            if (j + 2 == n) commit(q_empty);
           }
         }
         g += n;
         ++n_q;
         if (it.both) { gb += n; ++n_qb; }
       }
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ soft-max + epilogue
+    regs_up<224>();
     const int tile = (warp - 4) >> 2, q = warp & 3;
     const int r = (q << 5) + lane;
     const uint32_t lane_addr = (uint32_t)(q << 5) << 16;
@@ -1211,7 +1225,7 @@ attn_fwd_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     uint32_t n_it = 0, n_q = 0, g = 0;
     for (;;) {
       const int slot = n_it & 1;
-      mbar_wait(&item_full[slot], (n_it >> 1) & 1);
+      mbar_wait_brief(&item_full[slot], (n_it >> 1) & 1);
       const int idx = s_item[slot];
       __syncwarp();
       if (lane == 0) mbar_arrive(&item_empty[slot]);
@@ -1227,15 +1241,14 @@ attn_fwd_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       float m_i = -INFINITY, l_i = 0.f;
       for (int j = 0; j < it.n_tiles; ++j) {
         const uint32_t gt = g + j;
-        mbar_wait(&s_full[tile], gt & 1);
+        mbar_wait_brief(&s_full[tile], gt & 1);
         tc_fence_after();
         if (warp_valid) {
-          // Columns 64..127 are read twice instead of held: twelve warps share the registers.  P (64 columns) takes the place of S columns that have been
-          // turned into it
+          // a thread holds its row's 128 scores; P (64 columns) takes the place of S columns
           const int kv0 = j * KT;
           const bool need_mask = kv0 + KT > clear_to;
           const int hi = kv_last - kv0;
-          uint32_t x[32], y[32];
+          uint32_t x[4][32];
           float mxs[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // (an instruction takes two values into a running maximum)
           auto mask = [&](uint32_t (&v)[32], int c0) {
 #pragma unroll
@@ -1246,18 +1259,15 @@ attn_fwd_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 #pragma unroll
             for (int i = 0; i < 32; i += 2) mxs[(i >> 1) & 3] = max3(mxs[(i >> 1) & 3], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
           };
-          tmem_ld_32x32b_x32(s_addr + 64, x);
-          tmem_ld_32x32b_x32(s_addr + 96, y);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(s_addr + c * 32, x[c]);
           tmem_ld_wait();
-          if (need_mask) { mask(x, 64); mask(y, 96); }
-          largest(x);
-          largest(y);
-          tmem_ld_32x32b_x32(s_addr, x);
-          tmem_ld_32x32b_x32(s_addr + 32, y);
-          tmem_ld_wait();
-          if (need_mask) { mask(x, 0); mask(y, 32); }
-          largest(x);
-          largest(y);
+          if (need_mask) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) mask(x[c], c * 32);
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) largest(x[c]);
           const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])) * scale_log2;
           const float m_new = fmaxf(m_i, mx);
           const bool need = j > 0 && m_new > m_i + ATT_RESCALE_THRESHOLD;
@@ -1265,7 +1275,7 @@ attn_fwd_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             m_i = m_new;
           } else if (__any_sync(0xffffffffu, need)) {
             const float f = (m_new == -INFINITY) ? 1.f : exp2f(m_i - m_new);
-            mbar_wait(&o_done[tile], (gt - 1) & 1);
+            mbar_wait_brief(&o_done[tile], (gt - 1) & 1);
             tc_fence_after();
 #pragma unroll 1
             for (int c = 0; c < 8; ++c) {
@@ -1311,14 +1321,8 @@ attn_fwd_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             }
             tmem_st_32x32b_x16(s_addr + c * 16, pk);
           };
-          probabilities(x, 0);
-          tmem_ld_32x32b_x32(s_addr + 64, x);
-          probabilities(y, 1);
-          tmem_ld_32x32b_x32(s_addr + 96, y);
-          tmem_ld_wait();
-          if (need_mask) { mask(x, 64); mask(y, 96); }
-          probabilities(x, 2);
-          probabilities(y, 3);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) probabilities(x[c], c);
           l_i += psum;
           tmem_st_wait();
         }
@@ -1326,7 +1330,7 @@ attn_fwd_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         mbar_arrive(&p_full[tile]);
       }
       g += it.n_tiles;
-      mbar_wait(&o_final[tile], n_q & 1);
+      mbar_wait_brief(&o_final[tile], n_q & 1);
       ++n_q;
       tc_fence_after();
       if (warp_valid) {

@@ -254,39 +254,42 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
     __syncwarp();
-  } else if (warp == 1 && lane == 0) {
-    // ------------------------------------------------------------ MMA issuer
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer (the warp stays together and elects a lane: descriptors in uniform registers,
+    // 40 cycles a 16-wide product instead of 60 by a lane alone)
     constexpr uint32_t idesc_s = make_idesc(UMMA_BF16, UMMA_BF16, DA_KT, DA_NQ, 0, 0);      // A = K (K-major), B = Q (K-major)
     constexpr uint32_t idesc_o = make_idesc(UMMA_BF16, UMMA_BF16, DA_D, DA_NQ, 1, 0);       // A = V^T (MN-major: d contiguous), B = P^T
+    const uint64_t d_k = make_smem_desc_sw128(smem_u32(sK), 0, 1024), d_q = make_smem_desc_sw128(smem_u32(sQ), 0, 1024);
+    const uint64_t d_v = make_smem_desc_sw128(smem_u32(sV), DA_HALF_BYTES, 1024), d_p = make_smem_desc_sw128(smem_u32(sP), 0, 1024);
+    const bool one = elect_one();
     uint32_t n_it = 0, n_q = 0, g = 0;
     for (;;) {
       const int slot = n_it & 1;
       DA_T(0, DA_WAIT(&item_full[slot], (n_it >> 1) & 1));
       const int idx = s_item[slot];
-      mbar_arrive(&item_empty[slot]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&item_empty[slot]);
       ++n_it;
       if (idx >= p.total_items) break;
       const Item it = decode_item(idx);
       if (it.n_tiles == 0) continue;
       const int n_tiles = it.n_tiles;
       const int qs = n_q & 1;
-      const uint32_t q_addr = smem_u32(sQ + qs * DA_Q_BYTES);
-      DA_DBG(2, n_q, g);
+      if (lane == 0) DA_DBG(2, n_q, g);
       auto issue_S = [&](uint32_t gt, bool last) {
         const int st = gt % DA_STAGES;
         DA_T(1, DA_WAIT(&k_full[st], (gt / DA_STAGES) & 1));
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(sK + st * DA_TILE_BYTES);
+        if (one) {
+          const uint64_t a = d_k + st * (DA_TILE_BYTES / 16), b = d_q + qs * (DA_Q_BYTES / 16);
 #pragma unroll
-        for (int k = 0; k < DA_D / 16; ++k) {
-          const uint32_t koff = (k >> 2) * DA_HALF_BYTES + (k & 3) * 32;
-          const uint32_t qoff = (k >> 2) * (DA_NQ * 128) + (k & 3) * 32;
-          umma_f16_ss(tmem_S + (gt & 1) * DA_NQ, make_smem_desc_sw128(k_addr + koff, 0, 1024), make_smem_desc_sw128(q_addr + qoff, 0, 1024),
-                      idesc_s, k != 0);
+          for (int k = 0; k < DA_D / 16; ++k)
+            umma_f16_ss(tmem_S + (gt & 1) * DA_NQ, a + ((k >> 2) * DA_HALF_BYTES + (k & 3) * 32) / 16, b + ((k >> 2) * (DA_NQ * 128) + (k & 3) * 32) / 16,
+                        idesc_s, k != 0);
+          umma_commit(&k_empty[st]);
+          umma_commit(&s_full[gt & 1]);
+          if (last) umma_commit(&q_empty[qs]);
         }
-        umma_commit(&k_empty[st]);
-        umma_commit(&s_full[gt & 1]);
-        if (last) umma_commit(&q_empty[qs]);
       };
       DA_T(5, DA_WAIT(&q_full[qs], (n_q >> 1) & 1));
       issue_S(g, n_tiles == 1);
@@ -298,19 +301,20 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         DA_T(3, DA_WAIT(&v_full[st], (gt / DA_STAGES) & 1));
         if (j == 0) DA_T(4, DA_WAIT(o_free, (n_q & 1) ^ 1));       // the previous item's epilogue has read O^T
         tc_fence_after();
-        const uint32_t v_addr = smem_u32(sV + st * DA_TILE_BYTES);
-        const uint32_t p_addr = smem_u32(sP + (gt & 1) * DA_P_BYTES);
+        if (one) {
+          const uint64_t a = d_v + st * (DA_TILE_BYTES / 16), b = d_p + (gt & 1) * (DA_P_BYTES / 16);
 #pragma unroll
-        for (int k = 0; k < DA_KT / 16; ++k)      // 16 keys per step: A rows advance 16 x 128 B, B (P^T, K-major) advances 32 B inside a 64-key chunk
-          umma_f16_ss(tmem_O, make_smem_desc_sw128(v_addr + k * 2048, DA_HALF_BYTES, 1024),
-                      make_smem_desc_sw128(p_addr + (k >> 2) * (DA_NQ * 128) + (k & 3) * 32, 0, 1024), idesc_o, (j | k) != 0);
-        umma_commit(&v_empty[st]);
-        umma_commit(o_done);
-        if (j + 1 == n_tiles) umma_commit(o_final);
+          for (int k = 0; k < DA_KT / 16; ++k)      // 16 keys per step: A rows advance 16 x 128 B, B (P^T, K-major) advances 32 B inside a 64-key chunk
+            umma_f16_ss(tmem_O, a + k * (2048 / 16), b + ((k >> 2) * (DA_NQ * 128) + (k & 3) * 32) / 16, idesc_o, (j | k) != 0);
+          umma_commit(&v_empty[st]);
+          umma_commit(o_done);
+          if (j + 1 == n_tiles) umma_commit(o_final);
+        }
       }
       g += n_tiles;
       ++n_q;
     }
+    __syncwarp();
   } else if (warp >= 2) {
     // ------------------------------------------------------------ softmax (thread = key) + epilogue (thread = output dim)
     const int q4 = warp & 3;                              // TMEM lane quadrant of this warp

@@ -286,35 +286,37 @@ gemm_fp8_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   const uint32_t tmem_base = *tmem_ptr;
 
   if (warp == 5) {
-    if (lane == 0) {
-      int stage = 0; uint32_t phase = 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        mbar_wait(&empty[stage], phase ^ 1);
+    const bool one = elect_one();
+    int stage = 0; uint32_t phase = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      mbar_wait(&empty[stage], phase ^ 1);
+      if (one) {
         mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
         tma_load_2d(sW + stage * Cfg::W_BYTES, &tmW, &full[stage], kb * F8_BK, tile * 128);
         tma_load_2d(sX + stage * NT * F8_BK, &tmX, &full[stage], kb * F8_BK, 0);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      if (++stage == STAGES) { stage = 0; phase ^= 1; }
     }
     __syncwarp();
   } else if (warp == 4) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(UMMA_E4M3, UMMA_E4M3, 128, NT, 0, 0);
-      int stage = 0; uint32_t phase = 0;
-      int acc = 0; uint32_t acc_phase = 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        mbar_wait(&tempty[acc], acc_phase ^ 1);
-        mbar_wait(&full[stage], phase);
-        tc_fence_after();
-        const uint64_t wdesc = make_smem_desc_sw128(smem_u32(sW + stage * Cfg::W_BYTES), 0, 1024);
-        const uint64_t xdesc = make_smem_desc_sw128(smem_u32(sX + stage * NT * F8_BK), 0, 1024);
+    constexpr uint32_t idesc = make_idesc(UMMA_E4M3, UMMA_E4M3, 128, NT, 0, 0);
+    const uint64_t dw = make_smem_desc_sw128(smem_u32(sW), 0, 1024), dx = make_smem_desc_sw128(smem_u32(sX), 0, 1024);
+    const bool one = elect_one();
+    int stage = 0; uint32_t phase = 0;
+    int acc = 0; uint32_t acc_phase = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      mbar_wait(&tempty[acc], acc_phase ^ 1);
+      mbar_wait(&full[stage], phase);
+      tc_fence_after();
+      const uint64_t wdesc = dw + stage * (Cfg::W_BYTES / 16), xdesc = dx + stage * (NT * F8_BK / 16);
+      if (one) {
 #pragma unroll
         for (int k = 0; k < F8_BK / 32; ++k) umma_f8_ss(tmem_base + acc * NT, wdesc + 2 * k, xdesc + 2 * k, idesc, k != 0);
         umma_commit(&empty[stage]);
         umma_commit(&tfull[acc]);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
-        if (++acc == NACC) { acc = 0; acc_phase ^= 1; }
       }
+      if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      if (++acc == NACC) { acc = 0; acc_phase ^= 1; }
     }
     __syncwarp();
   } else {

@@ -231,6 +231,8 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_c
     const int q = warp - 4, odd = lane & 1;
     const uint32_t t_lane = tmem + ((uint32_t)(q * 32) << 16);
     int acc = 0; uint32_t acc_phase = 0;
+    int buf = 0;                                              // swap buffer of the chunk: it runs on from tile to tile, so that the barrier of one use orders the reads
+                                                              // of the last use of the other (a tile of an odd number of chunks would end and begin on the same one)
     while (work.next()) {
       const int n = work.n, f0 = work.f_block * BF;
       const int f = f0 + (SILU ? rank * 64 + (q & 1) * 32 : rank * 128 + q * 32) + lane;
@@ -243,7 +245,6 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_c
       };
       mbar_wait(&tfull[acc], acc_phase);
       tc_fence_after();
-      int buf = 0;
 #pragma unroll 1
       for (int c = 0; c < n; c += 32, buf ^= 1) {             // (n is a multiple of 16: a last half chunk holds what an earlier tile left, and is not stored)
         uint32_t r[32];

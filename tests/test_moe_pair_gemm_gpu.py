@@ -47,3 +47,29 @@ def test_block(E, K, H, I, rows, act, off):
         assert err < 4 * 2 ** -9, err
         far = (y.double() - ref).norm(dim=1) / ref.norm(dim=1).clamp(min=float(ref.norm() / T ** 0.5) * 0.05)
         assert float(far.max()) < 16 * 2 ** -9, float(far.max())
+
+
+@pytest.mark.parametrize("rows", [20, 9, 70, 90, 130])
+def test_tiles_of_odd_chunk_counts_in_a_row(rows):
+    """one K block a tile, so that the epilogue is behind the products and takes tile after tile: gate and up warps swap values through two buffers, which have to
+    alternate across tiles of one, three or five chunks (20, 9: 1, 70 and 90: 3, 130: 5) as well as inside a tile; the same bits every time, and the right ones"""
+    assert ops.load_native()
+    E, H, I = 300, 64, 1024
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    ids = torch.arange(E, device="cuda", dtype=torch.int32).repeat_interleave(rows)[torch.randperm(E * rows, generator=g, device="cuda")][:, None].contiguous()
+    x, w = rnd(E * rows, H).to(torch.bfloat16), torch.rand(E * rows, 1, generator=g, device="cuda") + 0.1
+    w13, w2 = (rnd(E, 2 * I, H) * H ** -0.5).to(torch.bfloat16), (rnd(E, H, I) * I ** -0.5).to(torch.bfloat16)
+    first = moe_ops.fused_moe(x, w13, w2, w, ids)
+    ref = torch.zeros(E * rows, H, dtype=torch.float64, device="cuda")
+    for e in range(E):
+        t = (ids[:, 0] == e).nonzero()[:, 0]
+        a, u = (x[t].double() @ w13[e].double().T).chunk(2, -1)
+        ref[t] = (torch.nn.functional.silu(a) * u) @ w2[e].double().T * w[t].double()
+    # three roundings to bf16, as above; a swapped value is as large as what it takes the place of
+    err = (first.double() - ref).norm(dim=1) / ref.norm(dim=1).clamp(min=float(ref.norm() / (E * rows) ** 0.5) * 0.05)
+    assert float(err.max()) < 16 * 2 ** -9, float(err.max())
+    differ = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(300):
+        differ += (moe_ops.fused_moe(x, w13, w2, w, ids) != first).sum()
+    assert int(differ) == 0

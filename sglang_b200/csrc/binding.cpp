@@ -6,7 +6,10 @@
 #include <torch/library.h>
 #include <torch/types.h>
 
+#include <algorithm>
 #include <atomic>
+#include <climits>
+#include <cmath>
 
 #include "kernels/api.h"
 
@@ -1193,13 +1196,53 @@ void moe_topk_softmax(const at::Tensor& logits, at::Tensor out_w, at::Tensor out
   count();
 }
 
+// Which kernel takes the products of an expert block, by the rows r that an expert gets on average (of pairs over ``all`` experts; E of them are here):
+//   0: weights streamed by small CTAs that share a tile's K, rows in tiles of 16 to 128 (gemm_grouped_decode.cu)
+//   1: pairs of SMs, rows in steps of 16 (gemm_grouped_pair.cu)          2: 128-row tiles (gemm_tc.cu)
+// The lines, us a block at r by kernels 0 / 1 / 2 (E of width x inner width, silu(gate) * up, weights not in L2):
+//  - 0 to 1 at 13 rows: 8 of 4096 x 14336: 456 / 468 / 609 at 12, 470 / 469 / 608 at 16; 8 of 4096 x 1792: 81 / 86 / 129, 86 / 87 / 129; 64 of 2048 x 352: 79 / 84 / 104,
+//    85 / 84 / 103.  Sooner where experts are many and wide, as kernel 0 is then behind its bytes: 128 of 2048 x 768: 207 / 203 at 3, 227 / 220 at 8; 32 of 2880 x 2880:
+//    288 / 279 at 6; later (36) where the first round over the SM pairs leaves a quarter of them idle, as kernel 1 does not share K: 16 of 2048 x 768 (of 128):
+//    55 / 58 at 24, 62 / 62 at 32; 2 of 4096 x 14336 (of 8): 153 / 161 at 24, 180 / 164 at 40; or K of the first product is short: 64 of 512 x 2048: 117 / 134 at 32
+//  - never 1 where its tiles fill half of the pairs at most (8 of 1024 x 512: 25 / 32 / 31 at 12, 96 / 70 by 1 / 2 at 1000) or an inner width below 256 makes a tile mostly
+//    epilogue (128 of 2048 x 192: 101 / 111 at 16, 172 / 149 by 1 / 2 at 64): then 0 to 2 at 48 and, for these narrow ones, 32 rows (163 / 142 / 145 at 40)
+//  - 1 to 2 by inner width, for the same reason: 256 (256 of 7168): 787 / 872 by 1 / 2 at 48, 1126 / 958 at 96; 384 (16 of 4096): 67 / 74 at 48, 77 / 74 at 80; 512 (32 of 4096):
+//    126 / 126 at 64, 143 / 129 at 96; 640 (128 of 2048): 784 / 795 at 400, 1258 / 1174 at 700; from 1024 on (16 of 5120) 1 throughout, 1154 / 1214 at 2000
+// fixed_order: kernel 0's shares of K follow the number of pairs; 2 adds a row's K in one order whatever they are.  kernel: -1, or the one a caller asks for
+struct MoePlan { int kernel, tile; };
+MoePlan moe_plan(long long pairs, long long E, long long all, long long H, long long I, int act, int sms, bool fixed_order, int kernel) {
+  all = std::max({all, E, 1ll});
+  const double r = (double)pairs / all;
+  // tiles that hold twice the average, so that few experts need a second one; of 16 rows up to 13 (16 / 32 rows: 456 / 465, 243 / 256, 81 / 85 us at 12 rows for 8
+  // experts of 4096 x 14336, 7168 and 1792)
+  const MoePlan streamed{0, r <= 13 ? 16 : r <= 16 ? 32 : r <= 32 ? 64 : 128}, paired{1, 16}, rows128{2, 128};
+  const bool fits = sms >= 2 && sglb::gemm_grouped_pair_fits((int)std::min(pairs + 16 * std::min(E, pairs), (long long)INT_MAX), (int)E);
+  if (kernel >= 0) {
+    TORCH_CHECK(kernel <= 2 && (kernel != 1 || fits), "expert block: kernel 0, 1 (where its tile list holds them) or 2");
+    return kernel == 0 ? streamed : kernel == 1 ? paired : rows128;
+  }
+  if (fixed_order) return rows128;
+  const long long units = sms / 2, tiles = E * std::max(1ll, (long long)std::ceil(r / 256)), n1 = act == 0 ? I : act == 1 ? 2 * I : I, bf1 = act == 0 ? 128 : 256;
+  const long long i1 = tiles * ((n1 + bf1 - 1) / bf1), i2 = tiles * ((H + 255) / 256);
+  // share of the SM pairs that is busy over the rounds of both products
+  const double busy = units ? (double)(i1 * H + i2 * I) / (units * ((i1 + units - 1) / units * H + (i2 + units - 1) / units * I)) : 0.;
+  const double from = H < 1024 ? 48 : busy < 0.75 ? 36 : E >= 64 && I >= 640 ? 3 : E >= 32 && I >= 640 && busy > 0.9 ? 6 : 13;
+  const double upto = busy < 0.55 || I < 256 ? 0 : I < 512 ? 48 : I < 640 ? 64 : H < 2048 || I < 1024 ? 400 : 1e30;
+  if (r > from && r <= upto && fits) return paired;
+  return r > (I < 256 ? 32 : 48) || (upto > 0 && r > from) ? rows128 : streamed;
+}
+std::vector<int64_t> moe_block_plan(int64_t pairs, int64_t E, int64_t all, int64_t H, int64_t I, int64_t act, int64_t sms, bool fixed_order) {
+  const MoePlan p = moe_plan(pairs, E, all, H, I, (int)act, (int)sms, fixed_order, -1);
+  return {p.kernel, p.tile};
+}
+
 // Whole expert MLP block on expert-sorted rows: align -> gather -> grouped GEMM (silu(gate)*up fused) -> grouped GEMM (routing
 // weight fused) -> combine.  act: 0 = silu(gate) * up, 1 = clamped GLU, 2 = ungated max(up, 0)^2 (w13 = [E, I, H]).  ``weight_input``: the routing weight
 // multiplies an expert's input (in the gather) instead of its output.  With peer pointers the combine pushes its result into every peer's NVLink arena instead of `out`.
 void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, const at::Tensor& topk_w,
                           const at::Tensor& topk_ids, c10::optional<at::Tensor> out, int64_t expert_offset,
                           const int64_t* peer_slots, const int64_t* peer_flags, int rank, int world, const uint32_t* epoch,
-                          uint32_t* done, bool fixed_order, int act = 0, float act_limit = 0.f, float act_alpha = 0.f, bool weight_input = false) {
+                          uint32_t* done, bool fixed_order, int64_t all_experts, int64_t kernel = -1, int act = 0, float act_limit = 0.f, float act_alpha = 0.f, bool weight_input = false) {
   CHECK_CUDA(x); CHECK_BF16(x); CHECK_BF16(w13); CHECK_BF16(w2); CHECK_I32(topk_ids); CHECK_LAST_CONTIG(x);
   TORCH_CHECK(x.dim() == 2 && w13.dim() == 3 && w2.dim() == 3 && w13.is_contiguous() && w2.is_contiguous());
   TORCH_CHECK(topk_w.scalar_type() == at::kFloat && topk_w.is_contiguous() && topk_ids.is_contiguous());
@@ -1209,14 +1252,10 @@ void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::
   c10::cuda::CUDAGuard g(x.device());
   auto stream = cur_stream();
   const int pairs = T * K;
-  // Few rows an expert: small CTAs that share a tile's K stream the weights best (gemm_grouped_decode.cu).  From 6 rows on, pairs of SMs with the rows as the
-  // narrow operand (gemm_grouped_pair.cu), and from 3 where experts are many and their tiles fill the pairs evenly.  us a block here / there, 8 experts of
-  // 4096 x 14336, 2 chosen: 460 / 472 at 5 rows, 475 / 475 at 8, 483 / 473 at 12, 533 / 485 at 38; 128 experts of 2048 x 768, 8 chosen: 162 / 161 at 2.6,
-  // 187 / 178 at 5, 251 / 218 at 21, 342 / 268 at 48.  Under expert parallelism the pairs are those of all ranks, so the line is met sooner by their number.
-  // fixed_order: the first kernel's shares of K follow the number of pairs; 128-row tiles (gemm_tc.cu) add a row's K in one order whatever they are.
-  const bool decode = !fixed_order && pairs <= (E >= 64 ? 3ll : 6ll) * E;
-  const bool two_sm = !decode && !fixed_order && num_sms() >= 2 && sglb::gemm_grouped_pair_fits(pairs + 16 * std::min(E, pairs), E);
-  const int tile = decode || two_sm ? 16 : 128;
+  // (under expert parallelism the pairs are those of all ranks: their experts say how many rows one gets)
+  const MoePlan plan = moe_plan(pairs, E, all_experts, H, I, act, num_sms(), fixed_order, (int)kernel);
+  const bool decode = plan.kernel == 0, two_sm = plan.kernel == 1;
+  const int tile = plan.tile;
   const int max_tiles = pairs / tile + std::min(E, pairs);
   const int live_tiles = std::max(1, std::min(max_tiles, std::min(E, pairs)));
   const int cap = max_tiles * tile;
@@ -1236,7 +1275,7 @@ void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::
   enum { NONE = 0, SILU = 1, ROWSCALE = 2, RELU2 = 3 };
   auto product = [&](const at::Tensor& a, const at::Tensor& w, at::Tensor& c, int n_out, int k, int epi) {
     if (decode)
-      sglb::gemm_grouped_decode(a.data_ptr(), w.data_ptr(), c.data_ptr(), row_w.data_ptr<float>(), sorted_row, n_out, k, k, n_out, E, tile_expert,
+      sglb::gemm_grouped_decode(a.data_ptr(), w.data_ptr(), c.data_ptr(), row_w.data_ptr<float>(), sorted_row, tile, n_out, k, k, n_out, E, tile_expert,
                                 num_tiles, max_tiles, live_tiles, epi, num_sms(), stream);
     else if (two_sm)
       sglb::gemm_grouped_pair(a.data_ptr(), w.data_ptr(), c.data_ptr(), row_w.data_ptr<float>(), cap, n_out, k, k, n_out, E, expert_start, epi, num_sms(), stream);
@@ -1268,32 +1307,34 @@ void moe_grouped_mlp_impl(const at::Tensor& x, const at::Tensor& w13, const at::
 }
 
 void moe_grouped_mlp(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, const at::Tensor& topk_w,
-                     const at::Tensor& topk_ids, at::Tensor out, int64_t expert_offset, bool fixed_order) {
+                     const at::Tensor& topk_ids, at::Tensor out, int64_t expert_offset, bool fixed_order, int64_t all_experts, int64_t kernel) {
   CHECK_BF16(out);
-  moe_grouped_mlp_impl(x, w13, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, fixed_order);
+  moe_grouped_mlp_impl(x, w13, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, fixed_order, all_experts, kernel);
 }
 
 void moe_grouped_mlp_glu(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, const at::Tensor& topk_w,
                          const at::Tensor& topk_ids, at::Tensor out, int64_t expert_offset, double limit, double alpha,
-                         bool fixed_order) {
+                         bool fixed_order, int64_t all_experts, int64_t kernel) {
   CHECK_BF16(out);
-  moe_grouped_mlp_impl(x, w13, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, fixed_order, 1, (float)limit,
+  moe_grouped_mlp_impl(x, w13, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, fixed_order, all_experts, kernel, 1, (float)limit,
                        (float)alpha);
 }
 
 void moe_grouped_mlp_relu2(const at::Tensor& x, const at::Tensor& w1, const at::Tensor& w2, const at::Tensor& topk_w, const at::Tensor& topk_ids,
-                           at::Tensor out, int64_t expert_offset, bool weight_input, bool fixed_order) {
+                           at::Tensor out, int64_t expert_offset, bool weight_input, bool fixed_order, int64_t all_experts,
+                           int64_t kernel) {
   CHECK_BF16(out);
-  moe_grouped_mlp_impl(x, w1, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, fixed_order, 2, 0.f, 0.f, weight_input);
+  moe_grouped_mlp_impl(x, w1, w2, topk_w, topk_ids, out, expert_offset, nullptr, nullptr, 0, 1, nullptr, nullptr, fixed_order, all_experts, kernel, 2, 0.f, 0.f, weight_input);
 }
 
 void moe_grouped_mlp_push(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, const at::Tensor& topk_w,
                           const at::Tensor& topk_ids, int64_t expert_offset, const at::Tensor& peer_slot_ptrs,
-                          const at::Tensor& peer_flag_ptrs, int64_t rank, int64_t world, at::Tensor epoch, at::Tensor done, bool fixed_order) {
+                          const at::Tensor& peer_flag_ptrs, int64_t rank, int64_t world, at::Tensor epoch, at::Tensor done, bool fixed_order,
+                          int64_t all_experts) {
   TORCH_CHECK(!peer_slot_ptrs.is_cuda() && !peer_flag_ptrs.is_cuda());
   moe_grouped_mlp_impl(x, w13, w2, topk_w, topk_ids, c10::nullopt, expert_offset, peer_slot_ptrs.data_ptr<int64_t>(),
                        peer_flag_ptrs.data_ptr<int64_t>(), (int)rank, (int)world, reinterpret_cast<const uint32_t*>(epoch.data_ptr<int>()),
-                       reinterpret_cast<uint32_t*>(done.data_ptr<int>()), fixed_order);
+                       reinterpret_cast<uint32_t*>(done.data_ptr<int>()), fixed_order, all_experts);
 }
 
 }  // namespace
@@ -1315,12 +1356,13 @@ TORCH_LIBRARY(sglb, m) {
   m.def("fp8_block_linear(Tensor x, Tensor wq, Tensor ws, bool ue8m0, bool fixed_order=False) -> Tensor", &fp8_block_linear);
   m.def("gemm_fp8_block(Tensor xq, Tensor xs, Tensor wq, Tensor ws, Tensor(a!) out, bool fixed_order=False) -> ()", &gemm_fp8_block);
   m.def("moe_topk_softmax(Tensor logits, Tensor(a!) out_w, Tensor(b!) out_ids, bool renorm) -> ()", &moe_topk_softmax);
-  m.def("moe_grouped_mlp(Tensor x, Tensor w13, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset, bool fixed_order=False) -> ()",
+  m.def("moe_block_plan(int pairs, int experts, int all_experts, int hidden, int inter, int act, int sms, bool fixed_order) -> int[]", &moe_block_plan);
+  m.def("moe_grouped_mlp(Tensor x, Tensor w13, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset, bool fixed_order=False, int all_experts=0, int kernel=-1) -> ()",
         &moe_grouped_mlp);
   m.def("moe_grouped_mlp_glu(Tensor x, Tensor w13, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset, float limit, "
-        "float alpha, bool fixed_order=False) -> ()", &moe_grouped_mlp_glu);
+        "float alpha, bool fixed_order=False, int all_experts=0, int kernel=-1) -> ()", &moe_grouped_mlp_glu);
   m.def("moe_grouped_mlp_push(Tensor x, Tensor w13, Tensor w2, Tensor topk_w, Tensor topk_ids, int expert_offset, Tensor peer_slot_ptrs, "
-        "Tensor peer_flag_ptrs, int rank, int world, Tensor(a!) epoch, Tensor(b!) done, bool fixed_order=False) -> ()", &moe_grouped_mlp_push);
+        "Tensor peer_flag_ptrs, int rank, int world, Tensor(a!) epoch, Tensor(b!) done, bool fixed_order=False, int all_experts=0) -> ()", &moe_grouped_mlp_push);
   m.def("gemm_push(Tensor a, Tensor w, Tensor peer_slot_ptrs, Tensor peer_flag_ptrs, int rank, int world, Tensor(a!) epoch, "
         "Tensor(b!) done, int bn) -> ()", &gemm_push);
   m.def("nvl_local_reduce_add_rmsnorm(Tensor slot, int flags_ptr, Tensor(a!)? residual, Tensor w, Tensor(b!) out, int world, int nslabs, float eps, "
@@ -1388,7 +1430,7 @@ TORCH_LIBRARY(sglb, m) {
         "Tensor(c!) v_cache, Tensor loc, Tensor(d!) q_out, int pad=0) -> ()", &conv_attention_prepare);
   m.def("norm_add_f32(Tensor(a!) x, Tensor src, Tensor? ids, Tensor w, Tensor(b!)? out, float eps, bool zero_centred=True) -> ()", &norm_add_f32);
   m.def("moe_sigmoid_route(Tensor logits, bool renorm, float scale, Tensor(a!) w, Tensor(b!) ids) -> ()", &moe_sigmoid_route);
-  m.def("moe_grouped_mlp_relu2(Tensor x, Tensor w1, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset, bool weight_input, bool fixed_order=False) -> ()",
+  m.def("moe_grouped_mlp_relu2(Tensor x, Tensor w1, Tensor w2, Tensor topk_w, Tensor topk_ids, Tensor(a!) out, int expert_offset, bool weight_input, bool fixed_order=False, int all_experts=0, int kernel=-1) -> ()",
         &moe_grouped_mlp_relu2);
   m.def("attention_sink_gate(Tensor o, Tensor lse, Tensor sinks, int Dv, Tensor(a!) out) -> ()", &attention_sink_gate);
   m.def("moe_softmax_bias_route(Tensor logits, Tensor? corr, int n_real, Tensor(a!) w, Tensor(b!) ids, Tensor(c!) ident) -> ()", &moe_softmax_bias_route);

@@ -57,7 +57,7 @@ void gemm_bf16_tc_grouped(const void* A, const void* W, void* C, const float* ro
 bool gemm_grouped_pair_fits(int cap_rows, int E);
 void gemm_grouped_pair(const void* X, const void* W, void* C, const float* row_scale, int cap_rows, int n_out, int K, int lda, int ldc, int E,
                        const int* expert_start, int epi, int num_sms, cudaStream_t stream);
-void gemm_grouped_decode(const void* X, const void* W, void* C, const float* row_scale, const int* sorted_row, int n_out, int K, int lda, int ldc,
+void gemm_grouped_decode(const void* X, const void* W, void* C, const float* row_scale, const int* sorted_row, int tile, int n_out, int K, int lda, int ldc,
                          int E, const int* tile_expert, const int* num_tiles, int max_tiles, int live_tiles, int epi, int num_sms, cudaStream_t stream);
 
 // kvio.cu: device pool <-> pinned host pool page movers (HiCache L1 <-> L2), zero-copy over UVA, layer_first / page_first host layouts

@@ -194,9 +194,9 @@ class FusedMoE(nn.Module):
 
             if envs.SGLB_FUSED_AR.get() == "push" and get_pp_group().world_size == 1:
                 # combine kernel pushes the partial sums to every peer; the next RMSNorm reduces them locally
-                off = tp.nvl.moe_push(x, self.w13, self.w2, w, ids.to(torch.int32), self.expert_offset)
+                off = tp.nvl.moe_push(x, self.w13, self.w2, w, ids.to(torch.int32), self.expert_offset, self.ep_size * self.local_experts)
                 return PendingAllReduce(tp.nvl, off, x.shape[0], x.shape[1], "push")
-        y = moe_ops.fused_moe(x, self.w13, self.w2, w, ids, self.expert_offset, self.act, self.weight_input)
+        y = moe_ops.fused_moe(x, self.w13, self.w2, w, ids, self.expert_offset, self.act, self.weight_input, self.ep_size * self.local_experts)
         if tp.world_size > 1:
             y = tp.all_reduce(y)
         return y

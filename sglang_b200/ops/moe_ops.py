@@ -30,10 +30,11 @@ def topk_softmax(router_logits: torch.Tensor, top_k: int, renormalize: bool = Tr
 
 
 def fused_moe(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_w: torch.Tensor, topk_ids: torch.Tensor,
-              expert_offset: int = 0, act=None, weight_input: bool = False) -> torch.Tensor:
+              expert_offset: int = 0, act=None, weight_input: bool = False, num_experts: int = 0) -> torch.Tensor:
     """``act``: None = silu(gate) * up; ``("clamped_glu", limit, alpha)`` = min(g, limit) * sigmoid(alpha g) * (clamp(u, +-limit) + 1);
     ``("relu2",)`` = ungated experts, max(up, 0)^2 with ``w13`` [E, I, H].  ``weight_input``: a routing weight multiplies its expert's input
-    instead of its output (ungated experts)"""
+    instead of its output (ungated experts).  ``num_experts``: how many experts ``topk_ids`` are spread over, where that is more than are here
+    (expert parallelism); the kernels are chosen by the rows an expert gets"""
     fn = None
     assert not weight_input or (act is not None and act[0] == "relu2"), "input weights: ungated experts only"
     if act is not None and act[0] == "relu2":
@@ -42,7 +43,7 @@ def fused_moe(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_w: torc
         if (x.is_cuda and x.dtype == torch.bfloat16 and _has("moe_grouped_mlp_relu2") and H % 32 == 0 and I % 32 == 0 and w13.shape[0] <= 512
                 and x.stride(1) == 1 and x.stride(0) % 8 == 0):
             out = torch.empty_like(x)
-            torch.ops.sglb.moe_grouped_mlp_relu2(x, w13, w2, topk_w, topk_ids, out, expert_offset, weight_input, envs.SGLB_FIXED_ORDER.get())
+            torch.ops.sglb.moe_grouped_mlp_relu2(x, w13, w2, topk_w, topk_ids, out, expert_offset, weight_input, envs.SGLB_FIXED_ORDER.get(), num_experts)
             return out
         if not x.is_cuda:
             return torch_ref.fused_moe(x, w13, w2, topk_w, topk_ids, expert_offset, fn, weight_input)
@@ -60,11 +61,11 @@ def fused_moe(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_w: torc
             and x.stride(0) % 8 == 0):
         # expert-sorted rows through the tcgen05 grouped GEMMs, no host sync: align -> gather -> gate|up GEMM -> clamped GLU -> down GEMM -> combine
         out = torch.empty_like(x)
-        torch.ops.sglb.moe_grouped_mlp_glu(x, w13, w2, topk_w, topk_ids, out, expert_offset, float(limit), float(alpha), envs.SGLB_FIXED_ORDER.get())
+        torch.ops.sglb.moe_grouped_mlp_glu(x, w13, w2, topk_w, topk_ids, out, expert_offset, float(limit), float(alpha), envs.SGLB_FIXED_ORDER.get(), num_experts)
         return out
     if act is None and x.dtype == torch.bfloat16 and _has("moe_grouped_mlp") and H % 32 == 0 and I % 32 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0:
         out = torch.empty_like(x)
-        torch.ops.sglb.moe_grouped_mlp(x, w13, w2, topk_w, topk_ids, out, expert_offset, envs.SGLB_FIXED_ORDER.get())
+        torch.ops.sglb.moe_grouped_mlp(x, w13, w2, topk_w, topk_ids, out, expert_offset, envs.SGLB_FIXED_ORDER.get(), num_experts)
         return out
     return _fused_moe_sorted(x, w13, w2, topk_w, topk_ids, expert_offset, fn)
 

@@ -191,7 +191,7 @@ class NvlComm:
         return off
 
     def moe_push(self, x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_w: torch.Tensor, topk_ids: torch.Tensor,
-                 expert_offset: int) -> int:
+                 expert_offset: int, num_experts: int = 0) -> int:
         """expert MLP block (align -> gather -> grouped GEMMs -> combine) whose combine kernel stores this rank's partial
         [T,H] straight into slot [rank] of every peer's arena: the expert-parallel reduction costs no kernel of its own."""
         T, H = x.shape
@@ -200,7 +200,7 @@ class NvlComm:
         off = self._slot(ch)
         torch.ops.sglb.moe_grouped_mlp_push(x, w13, w2, topk_w, topk_ids, expert_offset, self.buf_ptrs + off,
                                             self.flag_ptrs + ch * MAX_RANKS * 4, self.rank, self.world, self.epochs[ch:ch + 1],
-                                            self.done[ch, 1:], envs.SGLB_FIXED_ORDER.get())
+                                            self.done[ch, 1:], envs.SGLB_FIXED_ORDER.get(), num_experts)
         self.calls += 1
         return off
 

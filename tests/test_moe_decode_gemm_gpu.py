@@ -1,5 +1,6 @@
-"""Expert blocks on both sides of the line between the weight-streaming kernel (csrc/kernels/gemm_grouped_decode.cu) and 128-row tiles, against float64:
-row tiles of every size with remainders, output widths that end inside a tile, shared K, one overfull expert, experts of another rank, every epilogue."""
+"""Expert blocks of few rows, against float64: the weight-streaming kernel (csrc/kernels/gemm_grouped_decode.cu) with row tiles of every size and their remainders,
+output widths that end inside a tile, shared K, overfull experts, experts of another rank, every epilogue, and both sides of its lines (the blocks here are small or
+narrow, which is where it stays ahead of pairs of SMs up to 32 and 48 rows an expert)."""
 import pytest
 import torch
 
@@ -31,7 +32,7 @@ def _ref(x, w13, w2, w, ids, off, act, weight_input):
     return out
 
 
-@pytest.mark.parametrize("T,E,K,H,I,off,skew", [(1, 8, 2, 512, 256, 0, 0), (9, 8, 2, 160, 96, 0, 0), (20, 8, 2, 4096, 1024, 0, 0), (40, 16, 4, 256, 160, 0, 0),
+@pytest.mark.parametrize("T,E,K,H,I,off,skew", [(1, 8, 2, 512, 256, 0, 0), (9, 8, 2, 160, 96, 0, 0), (20, 8, 2, 4096, 1024, 0, 0), (20, 8, 2, 512, 256, 0, 4), (22, 8, 2, 512, 256, 3, 2), (40, 16, 4, 256, 160, 0, 0),
                                                 (64, 8, 2, 512, 416, 0, 3), (130, 8, 2, 512, 256, 4, 0), (190, 8, 2, 256, 128, 0, 0), (194, 8, 2, 256, 128, 0, 0), (250, 8, 2, 256, 128, 0, 0),
                                                 (260, 8, 2, 256, 128, 0, 0),
                                                 (333, 128, 8, 256, 96, 0, 0), (3, 300, 1, 128, 64, 0, 0), (700, 8, 2, 256, 128, 0, 2), (2100, 128, 8, 128, 64, 0, 0)])
@@ -57,7 +58,7 @@ def test_block(T, E, K, H, I, off, skew, act):
 
 
 def test_rows_beyond_the_line_are_alike():
-    """from 48 rows an expert on one kernel sums K in sequence: a token's bits do not follow how many others there are"""
+    """from 48 rows an expert on 128-row tiles sum K in sequence: a token's bits do not follow how many others there are"""
     E, K, H, I, T = 8, 2, 4096, 512, 400
     g = torch.Generator(device="cuda").manual_seed(5)
     x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)

@@ -91,10 +91,11 @@ __device__ __forceinline__ size_t mc_stride(size_t v) {
   return v;
 }
 // z / (1 + exp(-z)) without a branch: quotient by the reciprocal's approximation, and one Newton step by what it leaves (Newton-Raphson on d q = z).
-// 1 + exp(-z) is at least 1, and where it would overflow z over the largest number is as good as zero
+// 1 + exp(-z) is at least 1, and where it would overflow z over the largest number is as good as zero.  From 20 on it is 1: z itself, infinity too (the step would
+// take it from itself)
 __device__ __forceinline__ float mc_silu(float z) {
   const float d = fminf(1.f + expf(-z), 3e38f), r = rcp_approx(d), q = z * r;
-  return fmaf(fmaf(-d, q, z), r, q);
+  return z > 20.f ? z : fmaf(fmaf(-d, q, z), r, q);
 }
 // Chunk c of request b has slot cu_q[b] / 64 + b + c: no two share one, and none lies beyond T / 64 + B.
 __device__ __forceinline__ int mc_slot(int q0, int b) { return q0 / MC_L + b; }

@@ -85,6 +85,24 @@ def test_values_that_are_not_finite_stay_behind(bad):
     assert float((y[~hit].double() - want[~hit]).norm() / want[~hit].norm()) < 6e-7
 
 
+@pytest.mark.parametrize("bf16", [True, False])
+def test_infinite_and_large_gates(bf16):
+    """z / (1 + exp(-z)) over the whole range: infinity stays infinite with the sign of what it scales, large negative gates close"""
+    H, P, N, G, lens = 4, 64, 128, 1, [100, 90]
+    u, z, D, dt, da, state, old, cu, rows, call = _inputs(H, P, N, G, lens, "step", torch.bfloat16 if bf16 else torch.float32, 9)
+    z[7], z[8], z[9], z[70], z[71], z[72] = float("inf"), 1e30, -1e30, 20.0, 19.9, 80.0
+    z[10, 3], z[120, 5] = float("inf"), float("nan")
+    want, _ = _oracle(H, P, N, G, lens, u, z, D, dt, da, state, old, cu, rows)
+    y = call(state)
+    assert torch.isinf(y[7]).all() and torch.isinf(y[10, 3]) and torch.equal(y[7] > 0, want[7] > 0) and (y[10, 3] > 0) == (want[10, 3] > 0)
+    assert torch.equal(torch.isfinite(y), torch.isfinite(want)) and float(y[9].abs().max()) < 1e-30
+    for rows_ in (y[8].double() / want[8], y[70:73].double() / want[70:73]):
+        assert float((rows_ - 1).abs().median()) < 3e-7              # (a factor of an ulp at most on fp32 sums)
+    ok = torch.isfinite(want)
+    ok[8] = False
+    assert float((y[ok].double() - want[ok]).norm() / want[ok].norm()) < 6e-7
+
+
 def test_groups_in_slices_and_under_capture(monkeypatch):
     """more chunks of B, C and their products than the workspace holds at once; replayed from a graph, against the token-by-token order"""
     H, P, N, G, lens = 16, 128, 128, 16, [9700, 300]

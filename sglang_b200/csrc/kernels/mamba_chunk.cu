@@ -25,6 +25,11 @@
 // Measured, 64 heads of 64 x 128, 3001 tokens in 5 requests: 588 us eight tokens a step, 143 us here; one request of 1000: 333 and 111; 16 heads of
 // 128 x 128, one request of 3000: 982 and 300.  Error of y and of the state against 64 bits, 500 tokens in 12 requests: 1.18e-7 and 5.9e-8 eight tokens
 // a step, 9.3e-8 and 1.6e-8 here (the decays' products are formed in 64 bits); one of 1000: 8.9e-8 and 6.9e-9, 8.2e-8 and 3.4e-9.
+// Other values, 500 + 130 tokens, mean error against the sum of the terms' magnitudes over that of eight tokens a step: normal 0.5, one sign or alternating signs 0.5, over
+// six decades 0.6, cancelling pairs 0.3, one term alone 0.6 (constant decay 0.3 to 0.9).  Only where decay and step are exactly 1, and eight tokens a step round nothing
+// but sums, it is larger: 1.3 (N = 64: 1.8) for one sign, 1.8 for equal values, 2.5 for a single moving term, at most 1.3e-7.  Without MC_BIAS all but equal values
+// are worse (one sign at a decay of 1: 2.5).
+// Not finite: an infinite x, or one above 3.38e38, makes its column NaN from that token to the end (an infinite x is one of both signs in S^T C as soon as C changes sign).
 #include "common.cuh"
 #include "mamba2.h"
 #include "tma_host.h"

@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("H,P,N,G", [(4, 64, 128, 2), (2, 128, 64, 1), (6, 192, 128, 3)])
-@pytest.mark.parametrize("lens", [[2], [7, 1, 8], [9, 16, 17, 3], [40, 1, 65]])
+# (the 64-token form takes 24 tokens a request and 24 more of the first two widths: [40, 1, 65] there, while [40, 1, 29, 1, 65, 1] stays below its line)
+@pytest.mark.parametrize("lens", [[2], [7, 1, 8], [9, 16, 17, 3], [40, 1, 65], [40, 1, 29, 1, 65, 1], [47]])
 @pytest.mark.parametrize("mode", ["step", "decay", "gates"])
 @pytest.mark.parametrize("bf16", [True, False])
 def test_against_float64(H, P, N, G, lens, mode, bf16):

@@ -133,3 +133,77 @@ def test_groups_in_slices_and_under_capture(monkeypatch):
     assert float((got.double() - want.double()).norm() / want.double().norm()) < 3e-6
     assert float((keep.double() - s1.double()).norm() / s1.double().norm()) < 3e-6
     assert torch.equal(s2, keep)
+
+
+def _values(dist, T, H, P, N, G, g):
+    """rows of [x | B | C] whose products add up in every way: independent, of one sign, all alike, alternating, over six decades, one term alone, pairs that cancel"""
+    r = torch.randn(T, H * P + 2 * G * N, generator=g, device="cuda")
+    b, c = r[:, H * P:H * P + G * N].view(T, G, N), r[:, H * P + G * N:].view(T, G, N)
+    if dist == "positive":
+        r.abs_()
+    elif dist == "ones":
+        r.fill_(1.0)
+    elif dist == "alternating":
+        r.abs_()[:, H * P:].mul_(1.0 - 2.0 * (torch.arange(2 * G * N, device="cuda") % 2))
+    elif dist == "mixed":
+        r.mul_(10 ** (torch.rand(r.shape, generator=g, device="cuda") * 6 - 3))
+    elif dist in ("one term", "one moving term"):
+        keep = torch.full((T, G, 1), 3, device="cuda") if dist == "one term" else torch.randint(0, N, (T, G, 1), generator=g, device="cuda")
+        hot = torch.zeros(T, G, N, device="cuda").scatter_(2, keep, 1.0)
+        b.mul_(hot), c.mul_(hot)
+    elif dist == "cancelling":
+        b[..., 1::2] = b[..., ::2] * 1.001
+        c[..., 1::2] = -c[..., ::2]
+    return r
+
+
+@pytest.mark.parametrize("H,P,N,G", [(8, 64, 128, 2), (4, 128, 128, 2), (4, 64, 64, 2)])
+@pytest.mark.parametrize("lens", [[500, 130], [65, 129, 193, 65, 1]])        # (with chunks of a single token)
+@pytest.mark.parametrize("mode", ["step", "decay", "one"])
+@pytest.mark.parametrize("dist", ["normal", "positive", "ones", "alternating", "mixed", "one term", "one moving term", "cancelling"])
+def test_error_against_the_sum_of_magnitudes(H, P, N, G, lens, mode, dist):
+    """The constants that carry the accumulator's truncation back were measured on independent values: whatever the sums look like, down to one term and a decay and step
+    of exactly 1, an error stays one of fp32 sums.  Scale: the same recurrence over magnitudes, which no cancellation shrinks."""
+    g = torch.Generator(device="cuda").manual_seed(len(lens) + N + P)
+    T, B = sum(lens), len(lens)
+    u, state = _values(dist, T, H, P, N, G, g), torch.randn(B, H, N, P, generator=g, device="cuda")
+    args, kw = (None, None, None), {}
+    if mode == "step":
+        raw, bias, A_log = torch.randn(T, H, generator=g, device="cuda"), torch.randn(H, generator=g, device="cuda") - 3, torch.randn(H, generator=g, device="cuda").abs()
+        args = (raw, bias, A_log)
+        dt = torch.log1p(torch.exp(raw.double() + bias.double()))
+        da = torch.exp(-A_log.double().exp() * dt)
+    else:
+        kw["decay"] = torch.ones(H, device="cuda") if mode == "one" else torch.rand(H, generator=g, device="cuda") * 0.2 + 0.8
+        dt, da = torch.ones(T, H, device="cuda", dtype=torch.float64), kw["decay"].double().expand(T, H)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    rows, past = list(range(B)), [9] * B
+    want, s_want = _oracle(H, P, N, G, lens, u, None, None, dt, da, state, past, cu, rows)
+    size, s_size = _oracle(H, P, N, G, lens, u.abs(), None, None, dt, da, state.abs(), past, cu, rows)
+    y = ops.mamba2_scan(u, None, *args, None, state, _i32(rows), _i32([n + 9 for n in lens]), _i32(cu), _i32(lens), H, P, N, G, **kw)
+    for got, ref, scale in ((y, want, size), (state, s_want, s_size)):
+        # magnitudes that decayed below 1e-24 meet the end of the bf16 parts' range (2^-126, 24 bits further down): they count as that
+        e = (got.double() - ref).abs() / scale.clamp(min=1e-24)
+        # at worst: one accumulator takes up to eight products of the largest part (N / 16) and as many truncations of 2^-24, M and the decays a few more: 2^-20.  In the
+        # mean: half an ulp each for the sums of Y1, Y2 and of the state that Y1 reads, and for the factors on them, 2^-22 if all of them lean one way (eight tokens a
+        # step come to 1.4e-7 on one term with constant decay; measured here 1.3e-7)
+        assert float(e.max()) < 2 ** -20 and float(e.square().mean().sqrt()) < 2 ** -22, (float(e.max()), float(e.square().mean().sqrt()))
+
+
+def test_more_requests_than_are_ordered():
+    """beyond 256 requests none is taken by length, and the split kernel's threads look through several requests each; some are empty"""
+    H, P, N, G = 2, 64, 128, 1
+    g = torch.Generator().manual_seed(4)
+    lens = [0 if i % 7 == 3 else int(n) for i, n in enumerate(torch.randint(1, 90, (300,), generator=g))]
+    assert sum(lens) >= 24 * (len(lens) + 1)
+    u, z, D, dt, da, state, old, cu, rows, call = _inputs(H, P, N, G, lens, "step", torch.bfloat16, 21)
+    ref, s0 = _oracle(H, P, N, G, lens, u, z, D, dt, da, state, old, cu, rows)
+    empty = [rows[i] for i, n in enumerate(lens) if n == 0]
+    before = state[empty].clone()
+    y = call(state)
+    assert torch.equal(state[empty], before)
+    live = [rows[i] for i, n in enumerate(lens) if n]
+    assert float((y.double() - ref).norm() / ref.norm()) < 6e-7
+    assert float((state[live].double() - s0[live]).norm() / s0[live].norm()) < 6e-7

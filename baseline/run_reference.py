@@ -16,7 +16,7 @@ Modes (tried in order by bench.py until one produces a line; the one that ran is
   stock      the reference's own defaults on sm_100: trtllm_mha attention (FlashInfer trtllm-gen cubins), FlashInfer sampling, CUDA graphs
              (+ --bf16-gemm-backend torch in every mode, see MODES)
   fi         --attention-backend flashinfer
-  degraded   --attention-backend triton --sampling-backend pytorch          
+  degraded   --attention-backend triton --sampling-backend pytorch
 """
 from __future__ import annotations
 
@@ -44,7 +44,7 @@ sys.path.append(ROOT)
 # every mode carries the reference's own --bf16-gemm-backend torch: its sm_100 default ("cutedsl") imports cutlass.cute.experimental, which the
 # image's nvidia-cutlass-dsl refuses below CUDA toolkit 13.1 (this image: 12.9) — F.linear / cuBLAS is the reference's documented alternative
 # --mem-fraction-static 0.8: with its own default (0.854 on this part) the reference runs out of memory while capturing its prefill CUDA graphs
-# on this image (run D: "Tried to allocate 420 MiB ... 178.2 GiB in use"); lowering the fraction is the reference's documented remedy.
+# on this image ("Tried to allocate 420 MiB ... 178.2 GiB in use"); lowering the fraction is the reference's documented remedy.
 # --cuda-graph-max-bs-prefill 2048: at its default (16384 tokens x 74 shapes) every captured prefill shape took 10-15 GB on this torch build and the
 # capture ran the 178 GB card out of memory at ANY mem fraction (runs D / E); 2048 is the value the reference's own OOM message recommends.  The
 # `*_nopg` modes (--disable-prefill-cuda-graph) are the second fallback.

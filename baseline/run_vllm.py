@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""External sanity arm (BASELINE.md §4.3b): vLLM 0.22 (as installed in the image, LIBRARY code) on the same synthetic trace, through its
+"""External sanity arm: vLLM 0.22 (as installed in the image, LIBRARY code) on the same synthetic trace, through its
 public offline API ``vllm.LLM.generate``.  Not the headline baseline — a second same-box point next to the reference arm."""
 from __future__ import annotations
 

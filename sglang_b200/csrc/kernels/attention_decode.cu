@@ -1,7 +1,7 @@
 // Decode attention for sm_100a with the MMA operands SWAPPED: the 128 KEYS of a tile are the UMMA M dimension, the (few) query heads that
 // share a KV head are the UMMA N dimension.
 //
-// Why (profiles/attention_persist_r1.md): in the query-major kernel (attention_tc.cu) a decode item uses G = 4
+// Why: in the query-major kernel (attention_tc.cu) a decode item uses G = 4
 // of the 128 rows of every S / O tile, one softmax warp of four does all the exponentials (64 per thread per 64-key tile), the Q box drags
 // 32 KB through TMA to use 1 KB, and the tensor pipe spends 512 cycles per 16 KB of KV on rows that carry nothing.  Transposed:
 //
@@ -21,7 +21,7 @@
 // split-KV decode kernel (kernels/ops/attention/decode_attention.py:472).
 #include <math.h>
 
-// Round-2 experiments that did NOT pay and were removed again (numbers: profiles/attn_decode_r2.md, profiles/tma_gather_r2.md):
+// Tried without gain:
 //   * two softmax groups on alternating tiles (the consumer was not the limiter);
 //   * separate K / V producer warps + one 5-D TMA box per V page (fewer issues per thread; same speed, slower on ragged batches);
 //   * an L2 prefetcher warp running ahead of the work queue (extra TMA traffic cost more than the added bytes in flight gave).

@@ -1012,8 +1012,9 @@ __global__ void attn_merge_splits_diff_kernel(const float* __restrict__ part_o, 
 //   shared : Q 64 KB, two stages of K and V
 // Plain scores only (no cap, bias, window, chunk, tree or splits).  Same arithmetic in the same order per row as the kernel above.
 // A soft-max thread holds its row's 128 scores: the first warpgroup gives it the registers (with an equal share it spilled, and read half of S twice).
-// Measured: 4096 queries, 32 + 8 heads, at the end of 15011 keys: 1119 us in the kernel above, 942 here with one thread each for copies and products and
-// equal registers, 787 now; 2000 at the end of 9000: 321 -> 266; 17 prompts of 68 to 886 tokens (5003): 121 -> 79 us.
+// Measured, 4096 queries, 32 + 8 heads, at the end of 15011 keys, calls one behind the other on the same inputs: 1119 us in the kernel above, 956 here with one
+// thread each for copies and products and equal registers, 784 now (inputs that change from call to call: 989 and 868); 2000 at the end of 9000: 330 -> 276;
+// 17 prompts of 68 to 886 tokens (5003): 121 -> 79 us.
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));

@@ -38,8 +38,9 @@ __device__ __forceinline__ void fma_pair(float2& sum, float s, uint32_t a, uint3
 // Bound by the hand-off of an accumulator to the promotion (TMEM loads, 32 packed multiply-adds a warp, and the waits on both sides take about three times
 // the 256 cycles that 128 columns cost the tensor core), so a 256-wide tile has two halves with two accumulators each: one half is drained while the other is
 // formed.  The promotion warps take the registers of the other warpgroup, so that sixteen columns are on their way while sixteen are multiplied.
-// Measured, us a block (quantiser, [2I x H], SiLU, quantiser, [H x I]), before (whole 256-wide accumulators, one thread each for copies and products) and
-// now: 3001 tokens of 4096 / 14336: 715 / 691, 188: 111 / 98; 624 tokens of 8192 / 3584: 105 / 95, 147: 60 / 51, 65: 56 / 46.
+// Measured, us a block (quantiser, [2I x H], SiLU, quantiser, [H x I]), blocks one behind the other on the same inputs, before (whole 256-wide accumulators, one
+// thread each for copies and products) and now: 3001 tokens of 4096 / 14336: 723 / 696 (inputs that change: 823 / 793), 188: 126 / 109; 624 tokens of 8192 / 3584:
+// 112 / 104, 147: 66 / 55, 65: 59 / 49.
 template <int BN>
 struct F8Cfg {
   static constexpr int A_BYTES = F8_BM * F8_BK;

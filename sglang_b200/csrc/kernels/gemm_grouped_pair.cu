@@ -88,7 +88,7 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_c
   uint8_t* sA = smem;
   uint8_t* sB = smem + GP_STAGES * GP_A_BYTES;
   float* s_swap = reinterpret_cast<float*>(smem + GP_STAGES * GP_STAGE_BYTES);
-  uint2* s_tile = reinterpret_cast<uint2*>(smem + GP_STAGES * GP_STAGE_BYTES + GP_SWAP);      // first row; tokens / 16 (5 bits), expert (11), row tiles of the expert
+  uint2* s_tile = reinterpret_cast<uint2*>(smem + GP_STAGES * GP_STAGE_BYTES + GP_SWAP);      // first row; tokens / 16 (5 bits), expert (10; one unused), row tiles of the expert
   uint64_t* full = reinterpret_cast<uint64_t*>(s_tile + GP_LIST);
   uint64_t* empty = full + GP_STAGES;
   uint64_t* tfull = empty + GP_STAGES;
@@ -115,13 +115,11 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_c
   if (tid < 5) s_count[tid] = 0;
   __syncthreads();
   int steps[GP_MAX_E / GP_THREADS], row0[GP_MAX_E / GP_THREADS];
-  int rows = 0;
 #pragma unroll
   for (int i = 0; i < GP_MAX_E / GP_THREADS; ++i) {
     const int e = tid * (GP_MAX_E / GP_THREADS) + i;
     row0[i] = e < E ? __ldg(expert_start + e) : 0;
     steps[i] = e < E ? __ldg(expert_start + e + 1) - row0[i] : 0;
-    rows += steps[i];
   }
 #pragma unroll
   for (int k = 0; k < 5; ++k) {

@@ -2,7 +2,7 @@
 //
 // For M this small the classic orientation wastes the machine twice: the 128-row A box is mostly zero padding (smem and
 // tcgen05 rows that carry no data) and every CTA re-reads all of A, so a weight-streaming GEMM ends up latency-bound at a
-// fraction of HBM bandwidth (profiles/microbench_r1.md: cuBLAS and our wide kernel both sit at 25-30 us for 33-50 MB of
+// fraction of HBM bandwidth (cuBLAS and our wide kernel both sit at 25-30 us for 33-50 MB of
 // weights).  This kernel swaps the operands and splits K:
 //
 //   * W is the UMMA *M* operand: each CTA owns 128 output features and streams ONLY useful bytes (16 KB of W per 64-wide K

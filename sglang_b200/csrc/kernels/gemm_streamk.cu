@@ -1,6 +1,6 @@
 // Persistent stream-K weight-streaming GEMM for sm_100a decode shapes:   C[M,N] = A[M,K] * W[N,K]^T   (M <= 256 tokens)
 //
-// Why this kernel exists (profiles/gemm_decode_r1.md): at decode the four projections of a layer are pure weight streaming, and both the
+// Why this kernel exists: at decode the four projections of a layer are pure weight streaming, and both the
 // library and the first swap-AB kernel sit at 0.5-0.7 of the HBM roofline in-graph because their work decomposition is tile x wave:
 //   * gate_up = 224 tiles on 148 SMs = 1.51 waves, o/down = 32 tiles (21 % of the machine unless K is split by hand),
 //   * every CTA pays prologue + pipeline fill + epilogue drain once per tile on a 10-40 us kernel.

@@ -78,7 +78,7 @@ def EnvStr(name: str, default: Optional[str], doc: str = "") -> EnvVar[Optional[
 
 class _Envs:
     # --- build / kernels
-    SGLB_REQUIRE_NATIVE = EnvBool("SGLB_REQUIRE_NATIVE", True, "fail loudly if the CUDA extension is missing on a GPU box")
+    SGLB_REQUIRE_NATIVE = EnvBool("SGLB_REQUIRE_NATIVE", True, "fail loudly if the CUDA extension is missing where there is a GPU")
     SGLB_FORCE_TORCH_OPS = EnvBool("SGLB_FORCE_TORCH_OPS", False, "debug: route every op through the fp32 torch reference")
     SGLB_ATTN_IMPL = EnvStr("SGLB_ATTN_IMPL", "auto", "auto|tc (tcgen05)|simt (reference-grade CUDA)")
     SGLB_GEMM_IMPL = EnvStr("SGLB_GEMM_IMPL", "auto", "auto|tc (own tcgen05 GEMM)|lib (cuBLASLt)")
@@ -86,13 +86,12 @@ class _Envs:
     SGLB_SKINNY = EnvStr("SGLB_SKINNY", "tp", "tp|on|off: decode-shape (<=256 tokens) swap-AB split-K tcgen05 GEMM — tp: only as the fused "
                          "GEMM+all-reduce producer; on: every decode GEMM with fused consumers")
     SGLB_STREAMK_MAX_M = EnvInt("SGLB_STREAMK_MAX_M", 0, "bf16 GEMMs with <= this many tokens run on the persistent stream-K tcgen05 kernel "
-                                "(gemm_streamk.cu); 0 = never (cuBLAS).  Default 0: measured in-graph it does not beat the library yet "
-                                "(profiles/gemm_streamk_r2.md)")
+                                "(gemm_streamk.cu); 0 = never (cuBLAS).  Default 0: measured in-graph it does not beat the library yet")
     SGLB_FIXED_ORDER = EnvBool("SGLB_FIXED_ORDER", False, "the sums of a token's row in one order whatever shares its batch: one form of the own kernels "
                                "that have several (set by --enable-deterministic-inference)")
     SGLB_NVTX = EnvBool("SGLB_NVTX", False, "bracket every model forward with an NVTX range (mode, batch size)")
-    SGLB_TP_LIBRARY_AR_MIN_BYTES = EnvInt("SGLB_TP_LIBRARY_AR_MIN_BYTES", 3 << 19, "TP > 2: row-parallel outputs of at least this many bytes (default 1.5 MB) are all-reduced by NCCL (NVLS) + a local add+norm kernel; smaller ones by the own fused one-shot kernel (measured crossover, profiles/mgpu_tp4_r2.md); 0 = never")
-    SGLB_RS_AG_MIN_BYTES = EnvInt("SGLB_RS_AG_MIN_BYTES", 0, "TP > 2: row-parallel outputs of at least this many bytes use reduce-scatter + norm + all-gather with a row-sharded residual (0 bytes per rank growth with world) instead of the one-shot fused all-reduce + norm; 0 = never (default: measured no faster than the one-shot kernel at 4 ranks, profiles/mgpu_tp4_r2.md)")
+    SGLB_TP_LIBRARY_AR_MIN_BYTES = EnvInt("SGLB_TP_LIBRARY_AR_MIN_BYTES", 3 << 19, "TP > 2: row-parallel outputs of at least this many bytes (default 1.5 MB) are all-reduced by NCCL (NVLS) + a local add+norm kernel; smaller ones by the own fused one-shot kernel (measured crossover); 0 = never")
+    SGLB_RS_AG_MIN_BYTES = EnvInt("SGLB_RS_AG_MIN_BYTES", 0, "TP > 2: row-parallel outputs of at least this many bytes use reduce-scatter + norm + all-gather with a row-sharded residual (0 bytes per rank growth with world) instead of the one-shot fused all-reduce + norm; 0 = never (default: measured no faster than the one-shot kernel at 4 ranks)")
     SGLB_TP_GREEDY_SHARD = EnvBool("SGLB_TP_GREEDY_SHARD", True, "TP > 1: all-greedy decode batches take a vocab-parallel argmax (8 bytes per rank and row through the arena) instead of the [B, V] logits all-gather")
     SGLB_ATTN_DECODE = EnvStr("SGLB_ATTN_DECODE", "v3", "v3 = keys-as-M decode kernel (attention_decode.cu) | v2 = query-major kernel")
     SGLB_DISABLE_CUDA_GRAPH = EnvBool("SGLB_DISABLE_CUDA_GRAPH", False)
@@ -107,7 +106,7 @@ class _Envs:
     SGLB_COMM_IMPL = EnvStr("SGLB_COMM_IMPL", "auto", "auto|nvl (own P2P/multicast kernels)|nccl")
     SGLB_FUSED_AR = EnvStr("SGLB_FUSED_AR", "pull", "pull (GEMM writes its partial into the local arena slot, the next norm kernel reduces across "
                            "ranks via peer loads / NVLS) | push (GEMM epilogue stores into every peer, norm reduces locally) | off.  Measured: "
-                           "pull wins at 2 and 8 GPUs (push issues O(world) remote stores per rank; profiles/mgpu_tp8_r1.md)")
+                           "pull wins at 2 and 8 GPUs (push issues O(world) remote stores per rank)")
     SGLB_SP_MIN_TOKENS = EnvInt("SGLB_SP_MIN_TOKENS", 512, "sequence parallelism: prefills with fewer new tokens keep the fused all-reduce + norm path")
     SGLB_CP_MIN_TOKENS = EnvInt("SGLB_CP_MIN_TOKENS", 1024, "prefill CP: batches with fewer new tokens run the plain TP path (KV all-gather would dominate)")
     SGLB_MOE_A2A = EnvBool("SGLB_MOE_A2A", True, "DP-attention + expert parallel: all-to-all token dispatch/combine instead of gather-all-tokens")

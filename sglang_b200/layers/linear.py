@@ -49,7 +49,7 @@ class PendingAllReduce:
 
 class PendingLibraryAllReduce:
     """Partial sums of a LARGE row-parallel output whose all-reduce goes to NCCL (NVLS algorithm inside the library): measured on 4 x B200
-    (profiles/mgpu_tp4_r2.md) the library beats both own kernels from ~2 MB up (8 MB: NCCL + local norm 57 us, own one-shot fused 75 us, own
+    the library beats both own kernels from ~2 MB up (8 MB: NCCL + local norm 57 us, own one-shot fused 75 us, own
     reduce-scatter + norm + all-gather 77 us), while the own fused kernels win below ~1 MB.  Size-based dispatch, as the reference does
     (custom all-reduce for small messages, NCCL for large ones: distributed/parallel_state.py:648-757)."""
     __slots__ = ("y", "group", "T", "H")
@@ -93,7 +93,7 @@ class PendingSlabs:
 def _skinny_allowed(layer, x: torch.Tensor, push: bool = False) -> bool:
     """decode-shape tcgen05 GEMM policy.  ``SGLB_SKINNY=tp`` (default): only where it buys a fusion cuBLAS cannot give — the
     tensor-parallel GEMM + all-reduce producer (``push``); measured in-graph on B200, cuBLAS + our elementwise kernels is on par
-    or faster for the purely local GEMMs (profiles/gemm_decode_r1.md).  ``on``: every decode GEMM; ``off``: never."""
+    or faster for the purely local GEMMs.  ``on``: every decode GEMM; ``off``: never."""
     from ..environ import envs
 
     mode = envs.SGLB_SKINNY.get()

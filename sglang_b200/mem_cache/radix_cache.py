@@ -1,6 +1,6 @@
 """RadixAttention prefix cache (page-granular radix tree over token ids).
 
-Semantics follow the reference protocol (SURVEY §3.5, Appendix A.6;
+Semantics follow the reference protocol (
 ``python/sglang/srt/mem_cache/radix_cache.py``: ``match_prefix:377``, ``cache_finished_req:459``,
 ``cache_unfinished_req:516``, ``evict:593``, ``inc_lock_ref:623``, node split ``:705``; eviction
 strategies ``evict_policy.py:16-53``).  Design differences (B200-first):

@@ -1,7 +1,7 @@
 """ForwardBatch: the device-side view of one scheduler step.
 
 Parity: reference ``python/sglang/srt/model_executor/forward_batch_info.py`` (``ForwardMode``, ``init_new:705``,
-``compute_position:1771``) and SURVEY Appendix A.5.
+``compute_position:1771``).
 
 B200-first: ``ForwardBatch.build`` packs every per-step integer (input ids, positions, KV slot ids, request
 slots, sequence lengths, query offsets, page-table deltas, last-token indices) into ONE pinned int32 buffer and

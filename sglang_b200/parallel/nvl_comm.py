@@ -46,7 +46,7 @@ class NvlComm:
         self.graph_epoch = [0] * NUM_CHANNELS
         self.capturing = False
         # one-shot -> two-shot crossover: 512 KB on 8 GPUs (reference k3_ar_fusion.py:36-38); with two ranks a reduce-scatter +
-        # all-gather moves exactly the same bytes as the one-shot exchange, so two-shot never wins (measured: profiles/mgpu_tp2_r1.md)
+        # all-gather moves exactly the same bytes as the one-shot exchange, so two-shot never wins (measured)
         self.max_oneshot_bytes = (1 << 40) if self.world == 2 else 512 * 1024
         self.calls = 0
         self.use_nvls = bool(self.mc_ptr) and envs.SGLB_NVLS.get()      # NVSwitch in-network reduction when a multicast alias exists
@@ -54,7 +54,7 @@ class NvlComm:
         # nvl_rs_add_rmsnorm_ag_kernel).  The model runner switches it on per forward (``rs_active``) for model families whose every residual
         # update goes through a fused consume_norm; with two ranks the one-shot exchange moves the same bytes, so it stays off there.
         _rs = envs.SGLB_RS_AG_MIN_BYTES.get()
-        # validated at 4 ranks only: the 8-rank run of tools/mgpu_test.py died in this kernel (launch failure, run N) -> refused above 4 ranks
+        # validated at 4 ranks only: at 8 this kernel ended in a launch failure -> refused above 4 ranks
         self.rs_min_bytes = _rs if (2 < self.world <= 4 and _rs > 0) else (1 << 60)
         self.rs_active = False
         _lib = envs.SGLB_TP_LIBRARY_AR_MIN_BYTES.get()

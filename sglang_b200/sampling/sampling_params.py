@@ -1,6 +1,6 @@
 """Per-request sampling parameters.
 
-Field list and defaults follow the reference contract (SURVEY Appendix A.2;
+Field list and defaults follow the reference contract (
 ``python/sglang/srt/sampling/sampling_params.py``): ``max_new_tokens=128, temperature=1.0,
 top_p=1.0, top_k=-1, min_p=0.0, penalties, stop / stop_token_ids / stop_regex,
 json_schema | regex | ebnf | structural_tag (mutually exclusive), n, ignore_eos, ...``.

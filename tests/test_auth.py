@@ -1,5 +1,5 @@
 """Authorisation policy: deny by default once a key is configured (reference: srt/utils/auth.py decide_request_auth + test/registered/
-openai_server auth cases).  Regression for ADVICE r1: /invocations, /flush_cache, /get_weights_by_name, /pause_generation answered 200
+openai_server auth cases).  Regression: /invocations, /flush_cache, /get_weights_by_name, /pause_generation answered 200
 without a key when only --api-key was set."""
 import types
 

@@ -1,4 +1,4 @@
-"""Auxiliary / debugging subsystems (SURVEY §5): tensor invariants, rank consensus + slow-rank detection, tensor dumper/comparator, weights
+"""Auxiliary / debugging subsystems: tensor invariants, rank consensus + slow-rank detection, tensor dumper/comparator, weights
 checker, /slow_down, /set_trace_level, YAML config merge, crash dump, plugins, device timer."""
 import json
 import os

@@ -60,7 +60,7 @@ def test_pd_transfer_failure_is_reported():
 
 
 def test_tcp_transport_rejects_pickles_and_wrong_secret(monkeypatch):
-    """ADVICE r1: the listener used to pickle.loads() the header of any inbound connection (RCE).  The wire format is now magic + JSON + HMAC:
+    """the listener used to pickle.loads() the header of any inbound connection (RCE).  The wire format is now magic + JSON + HMAC:
     a pickle blob, a wrong secret and a non-allow-listed dtype are all dropped without touching the inbox."""
     import pickle
     import socket

@@ -1,6 +1,6 @@
 """BASELINE config #1: radix prefix cache + continuous batching correctness on a 2-layer transformer, CPU, world=1.
 Batched/chunked/retracted/cached generation must reproduce one-request-at-a-time greedy outputs token for token
-(reference strategy: mock-model e2e + scheduler kits, SURVEY §4.2)."""
+(reference strategy: mock-model e2e + scheduler kits)."""
 import numpy as np
 import pytest
 
@@ -123,7 +123,7 @@ def test_abort_and_priority():
 
 
 def test_flush_and_abort_see_the_unmerged_prefill_batch():
-    """ADVICE r1: between a prefill step and the next iteration the batch lives only in scheduler.last_batch.  flush_cache() used to succeed
+    """between a prefill step and the next iteration the batch lives only in scheduler.last_batch.  flush_cache() used to succeed
     there (tree / allocator reset under live requests -> 'dec_lock_ref underflow' kills the scheduler) and abort_request() missed it."""
     from sglang_b200.managers import io_struct as ios
 
@@ -156,7 +156,7 @@ def test_flush_and_abort_see_the_unmerged_prefill_batch():
 
 
 def test_seeded_sampling_is_scheduling_independent_and_min_new_tokens_holds_under_overlap():
-    """ADVICE r1: a per-request seed must give the same text whatever the batch composition / step the scheduler picks (the RNG counter is the
+    """a per-request seed must give the same text whatever the batch composition / step the scheduler picks (the RNG counter is the
     request's own output position), and min_new_tokens must suppress EOS exactly that long in overlap mode too."""
     eng = sgl.Engine(model_path="dummy:tiny-llama", page_size=4)
     assert eng.scheduler.enable_overlap

@@ -34,7 +34,7 @@ def test_native_extension_is_loaded():
 
     from sglang_b200 import ops
 
-    assert ops.load_native(), "the CUDA extension must load on a GPU box (no silent torch fallback)"
+    assert ops.load_native(), "the CUDA extension must load where there is a GPU (no silent torch fallback)"
     x = torch.randn(4, 1024, device="cuda", dtype=torch.bfloat16)
     c0 = ops.launch_count()
     ops.rmsnorm(x, torch.ones(1024, device="cuda", dtype=torch.bfloat16), 1e-5)

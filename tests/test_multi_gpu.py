@@ -1,10 +1,10 @@
 """Multi-GPU gate (``pytest -m gpu`` on a box with >= 2 GPUs; skipped otherwise).
 
-Round 1 shipped with a manual multi-GPU script only, which is how the TP>=4 mbarrier deadlock went unseen until the driver's scaling run.  This
-gate launches exactly what the driver launches — ``python -m torch.distributed.run ... bench.py --gpus N`` for several full traces — plus the NVL
+A deadlock at TP >= 4 once went unseen by a manual script.  This
+gate launches what a user launches — ``python -m torch.distributed.run ... bench.py --gpus N`` for several full traces — plus the NVL
 collective / fused-kernel numerics and the TP-vs-TP=1 prompt-logprob parity of ``tools/mgpu_test.py``.
 
-Reference strategy: test/registered/ (2/4/8-GPU suites, ``run_bench_serving`` floors) — SURVEY.md §4.
+Reference strategy: test/registered/ (2/4/8-GPU suites, ``run_bench_serving`` floors).
 """
 import json
 import os

@@ -16,7 +16,7 @@ DEV = "cuda"
 def _need():
     if not torch.cuda.is_available():
         pytest.skip("needs a GPU")
-    assert ops.load_native(), "the CUDA extension must be built on a GPU box"
+    assert ops.load_native(), "the CUDA extension must be built where there is a GPU"
 
 
 def _i32(x, dev=DEV):

@@ -1,4 +1,4 @@
-"""Microbenchmarks for the two non-bf16-dense configs BASELINE.json names: block-scaled fp8 linears (Llama-3-70B TP=8 shard shapes and
+"""Microbenchmarks for block-scaled fp8 linears (Llama-3-70B TP=8 shard shapes and
 Llama-3-8B shapes) and the Mixtral-8x7B expert block.  CUDA events, L2 flushed (256 MB write) between iterations, median of 7.
 fp8: our tcgen05 kind::f8f6f4 block-scaled GEMM (+ activation quant kernel) vs cuBLAS bf16 on the same logical GEMM and vs
 torch._scaled_mm (per-tensor fp8, library) where available.  MoE: native grouped path (align + gather + 2 grouped tcgen05 GEMMs +

@@ -1,4 +1,4 @@
-"""One-shot GPU check of the late round-2 model families: tiny random Hugging Face checkpoints (bf16, head_dim 128 so the tcgen05 attention
+"""One-shot GPU check of the model families: tiny random Hugging Face checkpoints (bf16, head_dim 128 so the tcgen05 attention
 kernels are the ones that run) served by the engine on cuda:0 and compared with the Hugging Face forward (fp32 math on the same bf16 weights).
 Usage: python tools/gpu_families_check.py [device] [out.json]"""
 import json

@@ -181,7 +181,7 @@ else:
         against an fp32 reference; timed against the one-shot fused kernel and NCCL + local norm at decode batches of 128..1024 tokens"""
         from sglang_b200.parallel.nvl_comm import CH_RS_AG
         if world > 4:
-            log("  rs+norm+ag: skipped above 4 ranks (the kernel faulted at 8 ranks in run N and is refused there by NvlComm; off by default)")
+            log("  rs+norm+ag: skipped above 4 ranks (the kernel faulted at 8 ranks and is refused there by NvlComm; off by default)")
             return
         for T, H in ((3, 4096), (130, 4096), (256, 4096), (512, 4096), (1024, 4096), (1024, 8192)):
             torch.manual_seed(300 + rank)
